@@ -42,6 +42,51 @@ SV_API int sv_last_error(char* buf, size_t len) {
 void sv_ctx_check(sv_context* ctx) {
   if (!ctx) sv_throw(SV_ERR_ARG, "null context");
   SV_CUDA(cudaSetDevice(ctx->device));
+  if (sv_pool != ctx->pool) sv_pool = ctx->pool;
+}
+
+thread_local std::shared_ptr<SvPool> sv_pool;
+
+void* SvPool::alloc(size_t bytes) {
+  void* p = nullptr;
+  cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, pool, stream);
+  if (e == cudaErrorMemoryAllocation) {
+    // let the stream's frees take effect and give back what the pool keeps, then
+    // try once more
+    cudaGetLastError();
+    cudaStreamSynchronize(stream);
+    cudaMemPoolTrimTo(pool, 0);
+    e = cudaMallocFromPoolAsync(&p, bytes, pool, stream);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    sv_throw(e == cudaErrorMemoryAllocation ? SV_ERR_OOM : SV_ERR_CUDA,
+             "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
+  }
+  return p;
+}
+
+void SvPool::free(void* p) {
+  std::lock_guard<std::mutex> lk(mu);
+  cudaSetDevice(device);
+  if (alive) {
+    cudaFreeAsync(p, stream);
+  } else {
+    cudaFree(p);
+    cudaMemPoolTrimTo(pool, 0);
+  }
+}
+
+void SvPool::close() {
+  std::lock_guard<std::mutex> lk(mu);
+  alive = false;
+  uint64_t none = 0;
+  cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &none);
+  cudaMemPoolTrimTo(pool, 0);
+}
+
+SvPool::~SvPool() {
+  if (pool) cudaMemPoolDestroy(pool);
 }
 
 cudaEvent_t sv_ctx_event(sv_context* ctx) {
@@ -79,6 +124,17 @@ void* sv_ctx_stage(sv_context* ctx, size_t bytes) {
     ctx->h_stage_bytes = b;
   }
   return ctx->h_stage;
+}
+
+void* sv_ctx_run_stage(sv_context* ctx, size_t bytes) {
+  if (bytes > ctx->h_run_bytes) {
+    if (ctx->h_run) cudaFreeHost(ctx->h_run);
+    ctx->h_run = nullptr;
+    ctx->h_run_bytes = 0;
+    SV_CUDA(cudaMallocHost(&ctx->h_run, bytes));
+    ctx->h_run_bytes = bytes;
+  }
+  return ctx->h_run;
 }
 
 void sv_sync(sv_context* ctx) { SV_CUDA(cudaStreamSynchronize(ctx->stream)); }
@@ -254,6 +310,21 @@ SV_API int sv_context_create(int device, sv_context** out) {
     delete ctx;
     sv_throw(SV_ERR_CUDA, "cudaStreamCreate: %s", cudaGetErrorString(e));
   }
+  ctx->pool = std::make_shared<SvPool>();
+  ctx->pool->device = device;
+  ctx->pool->stream = ctx->stream;
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = device;
+  uint64_t keep = (uint64_t)(prop.totalGlobalMem / SV_POOL_KEEP);
+  e = cudaMemPoolCreate(&ctx->pool->pool, &props);
+  if (e == cudaSuccess) e = cudaMemPoolSetAttribute(ctx->pool->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  if (e != cudaSuccess) {
+    cudaStreamDestroy(ctx->stream);
+    delete ctx;
+    sv_throw(SV_ERR_CUDA, "memory pool: %s", cudaGetErrorString(e));
+  }
   for (int i = 0; i < 16; ++i) SV_CUDA(cudaEventCreate(&ctx->marks[i]));
   SV_CUDA(cudaMalloc((void**)&ctx->d_status, 256));
   SV_CUDA(cudaMemsetAsync(ctx->d_status, 0, 256, ctx->stream));
@@ -275,11 +346,14 @@ SV_API int sv_context_destroy(sv_context* ctx) {
     if (ctx->marks[i]) cudaEventDestroy(ctx->marks[i]);
   if (ctx->d_status) cudaFree(ctx->d_status);
   if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
+  if (ctx->h_run) cudaFreeHost(ctx->h_run);
   for (void* p : ctx->h_io)
     if (p) cudaFreeHost(p);
   for (cudaEvent_t e : ctx->h_io_ev)
     if (e) cudaEventDestroy(e);
+  ctx->pool->close();
   cudaStreamDestroy(ctx->stream);
+  if (sv_pool == ctx->pool) sv_pool.reset();
   delete ctx;
   return SV_OK;
 }

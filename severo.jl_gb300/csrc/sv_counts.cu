@@ -829,7 +829,6 @@ SV_API int sv_counts_download_csr(sv_context* ctx, const sv_counts* c, int64_t* 
 
 SV_API int sv_counts_free(sv_counts* c) {
   if (c) {
-    if (c->ctx) cudaSetDevice(c->ctx->device);
     delete c;
   }
   return SV_OK;

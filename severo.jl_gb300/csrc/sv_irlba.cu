@@ -1808,8 +1808,8 @@ struct Lanczos {
     sv_memset(ctx, counter.get(), 0, 16);
     sv_memset(ctx, flag.get(), 0, nseg * 4);
     sv_memset(ctx, B.get(), 0, (size_t)nseg * work * work * 8);
-    SV_CUDA(cudaMallocHost((void**)&hsum, (size_t)nseg * (2 * work + 2) * 8));
-    SV_CUDA(cudaMallocHost((void**)&hflags, (size_t)nseg * 4));
+    hsum = (double*)sv_ctx_run_stage(ctx, (size_t)nseg * (2 * work + 2) * 8 + (size_t)nseg * 4);
+    hflags = (int*)(hsum + (size_t)nseg * (2 * work + 2));
     op->bind_active(active.get());
     SV_CUDA(cudaFuncSetAttribute(k_jacobi_svd, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  4 * MAX_WORK * MAX_WORK * 4));
@@ -1820,8 +1820,6 @@ struct Lanczos {
   ~Lanczos() {
     for (auto& g : graphs)
       if (g.exec) cudaGraphExecDestroy(g.exec);
-    if (hsum) cudaFreeHost(hsum);
-    if (hflags) cudaFreeHost(hflags);
   }
   Lanczos(const Lanczos&) = delete;
   Lanczos& operator=(const Lanczos&) = delete;
@@ -2378,7 +2376,6 @@ SV_API int sv_embed_info(const sv_embed* e, int64_t* n_cells, int64_t* npcs) {
 
 SV_API int sv_embed_free(sv_embed* e) {
   if (e) {
-    if (e->ctx) cudaSetDevice(e->ctx->device);
     delete e;
   }
   return SV_OK;

@@ -445,7 +445,6 @@ SV_API int sv_knn_info(const sv_knn* h, int64_t* n, int64_t* k) {
 
 SV_API int sv_knn_free(sv_knn* h) {
   if (h) {
-    if (h->ctx) cudaSetDevice(h->ctx->device);
     delete h;
   }
   return SV_OK;

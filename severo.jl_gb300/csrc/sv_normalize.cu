@@ -250,7 +250,6 @@ SV_API int sv_data_cell_totals(sv_context* ctx, const sv_data* d, int64_t* total
 
 SV_API int sv_data_free(sv_data* d) {
   if (d) {
-    if (d->ctx) cudaSetDevice(d->ctx->device);
     delete d;
   }
   return SV_OK;

@@ -2078,7 +2078,6 @@ SV_API int sv_batch_stats(sv_context* ctx, const sv_batch* b, double* mu, double
 
 SV_API int sv_batch_free(sv_batch* b) {
   if (b) {
-    if (b->ctx) cudaSetDevice(b->ctx->device);
     sv_centered_free(b->base);
     delete b;
   }
@@ -2284,7 +2283,6 @@ SV_API int sv_centered_mul(sv_context* ctx, const sv_centered* s, char trans, in
 
 SV_API int sv_centered_free(sv_centered* s) {
   if (s) {
-    if (s->ctx) cudaSetDevice(s->ctx->device);
     sv_data* d = s->own_data;
     sv_counts* c = s->own_counts;
     delete s;

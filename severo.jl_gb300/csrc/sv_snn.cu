@@ -675,7 +675,6 @@ SV_API int sv_graph_network(sv_context* ctx, const sv_graph* g, int64_t* nedges,
 
 SV_API int sv_graph_free(sv_graph* g) {
   if (g) {
-    if (g->ctx) cudaSetDevice(g->ctx->device);
     delete g;
   }
   return SV_OK;
