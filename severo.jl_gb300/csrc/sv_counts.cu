@@ -76,6 +76,11 @@ __global__ void k_seg_unsorted(const int64_t* __restrict__ ptr, const int32_t* _
 // the same output segment by source segment, so every output segment comes out
 // sorted without a sort and without global atomics.  tile_off[t * n_major + m] is
 // where source segment m's entries for tile t begin, relative to its start.
+//
+// The walk waits on its loads (a batch took ~4 us with 375 warps on the device),
+// so with few tiles the source segments are cut into `parts` groups as well, one
+// warp per (tile, group): the count pass leaves each output segment's entries
+// per group, their running sums give every group its place.
 
 constexpr int TR_WARPS = 8;     // tiles (warps) per block
 constexpr int TR_MAXT = 256;    // largest tile
@@ -156,24 +161,28 @@ __global__ void k_tr_swap(const int32_t* __restrict__ in, int64_t rows, int64_t 
   }
 }
 
-// Entries per output segment.  Warp per tile, shared-memory counters; lane l
+// Entries per output segment and group of source segments (seg_cnt[group *
+// n_minor + segment]).  Warp per (tile, group), shared-memory counters; lane l
 // walks source segment g0 + l of each batch of 32 (spreading a batch's entries
 // evenly over the lanes measured slower: the walk waits on loads, not lanes).
 __global__ void __launch_bounds__(TR_WARPS * 32) k_tr_count(
     const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx, int64_t n_major, int64_t n_minor,
-    int tshift, int64_t n_tiles, const int32_t* __restrict__ toff, int64_t* __restrict__ seg_cnt) {
+    int tshift, int64_t n_tiles, const int32_t* __restrict__ toff, int64_t per_part,
+    int32_t* __restrict__ seg_cnt) {
   __shared__ int cnt[TR_WARPS][TR_MAXT];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, T = 1 << tshift;
   const int64_t t = (int64_t)blockIdx.x * TR_WARPS + w;
   if (t >= n_tiles) return;
+  const int64_t m0 = blockIdx.y * per_part, m1 = min(n_major, m0 + per_part);
+  seg_cnt += blockIdx.y * n_minor;
   for (int k = lane; k < T; k += 32) cnt[w][k] = 0;
   __syncwarp();
   const int64_t c0 = t << tshift;
   const int32_t* lo = toff + t * n_major;
   const int32_t* hi = lo + n_major;
-  for (int64_t g0 = 0; g0 < n_major; g0 += 32) {
+  for (int64_t g0 = m0; g0 < m1; g0 += 32) {
     int64_t g = g0 + lane;
-    if (g < n_major) {
+    if (g < m1) {
       const int64_t base = ptr[g], a = base + lo[g], b = base + hi[g];
 #pragma unroll 4
       for (int64_t j = a; j < b; ++j) atomicAdd(&cnt[w][idx[j] - c0], 1);
@@ -183,18 +192,34 @@ __global__ void __launch_bounds__(TR_WARPS * 32) k_tr_count(
   for (int k = lane; k < T && c0 + k < n_minor; k += 32) seg_cnt[c0 + k] = cnt[w][k];
 }
 
-// Places every entry.  Warp per tile; per batch of 32·H source segments (H per
+// Per output segment: the groups' counts -> running sums, and the total.
+__global__ void k_tr_prefix(int32_t* __restrict__ seg_cnt, int64_t n_minor, int parts,
+                            int64_t* __restrict__ total) {
+  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n_minor;
+       k += (int64_t)gridDim.x * blockDim.x) {
+    int32_t sum = 0;
+    for (int p = 0; p < parts; ++p) {
+      const int32_t c = seg_cnt[p * n_minor + k];
+      seg_cnt[p * n_minor + k] = sum;
+      sum += c;
+    }
+    total[k] = sum;
+  }
+}
+
+// Places every entry.  Warp per (tile, group); per batch of 32·H source segments (H per
 // lane) an H-word mask per output segment gives each entry its rank among the
 // batch's entries of the same output segment.  Wider batches halve the batch
 // count each time and lengthen each output row's run per batch, so fewer of its
-// stores reach DRAM as partial sectors; with few tiles H = 1 keeps a lane's
-// load chain short.  Shared memory (dynamic): per warp T masks of H words and
+// stores reach DRAM as partial sectors; narrower ones keep a lane's load chain
+// short.  Shared memory (dynamic): per warp T masks of H words and
 // T cursors.
 template <int H>
 __global__ void __launch_bounds__(TR_WARPS * 32) k_tr_write(
     const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx, const int32_t* __restrict__ val,
     int64_t n_major, int64_t n_minor, int tshift, int64_t n_tiles, const int32_t* __restrict__ toff,
-    const int64_t* __restrict__ optr, int32_t* __restrict__ oidx, int32_t* __restrict__ oval) {
+    int64_t per_part, const int32_t* __restrict__ before, const int64_t* __restrict__ optr,
+    int32_t* __restrict__ oidx, int32_t* __restrict__ oval) {
   extern __shared__ __align__(16) unsigned char tr_smem[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, T = 1 << tshift;
   int64_t* pos = (int64_t*)tr_smem + (size_t)w * T;
@@ -202,22 +227,24 @@ __global__ void __launch_bounds__(TR_WARPS * 32) k_tr_write(
   const int64_t t = (int64_t)blockIdx.x * TR_WARPS + w;
   if (t >= n_tiles) return;
   const int64_t c0 = t << tshift;
+  const int64_t m0 = blockIdx.y * per_part, m1 = min(n_major, m0 + per_part);
+  before += blockIdx.y * n_minor;
   for (int k = lane; k < T; k += 32) {
 #pragma unroll
     for (int h = 0; h < H; ++h) mask[k * H + h] = 0u;
-    pos[k] = c0 + k < n_minor ? optr[c0 + k] : 0;
+    pos[k] = c0 + k < n_minor ? optr[c0 + k] + before[c0 + k] : 0;
   }
   __syncwarp();
   const int32_t* lo = toff + t * n_major;
   const int32_t* hi = lo + n_major;
   const unsigned bit = 1u << lane, below = bit - 1u;
-  for (int64_t g0 = 0; g0 < n_major; g0 += 32 * H) {
+  for (int64_t g0 = m0; g0 < m1; g0 += 32 * H) {
     int64_t a[H], b[H];
 #pragma unroll
     for (int h = 0; h < H; ++h) {
       int64_t g = g0 + 32 * h + lane;
       a[h] = b[h] = 0;
-      if (g < n_major) {
+      if (g < m1) {
         int64_t base = ptr[g];
         a[h] = base + lo[g];
         b[h] = base + hi[g];
@@ -555,29 +582,36 @@ void sv_transpose_counts(sv_context* ctx, int64_t n_major, int64_t n_minor, int6
               (unsigned)(ty < 65535 ? ty : 65535)), dim3(32, 8), 0, (const int32_t*)toffm.get(), n_major,
               n_tiles + 1, toff.get());
   }
-  const dim3 gt((unsigned)((n_tiles + TR_WARPS - 1) / TR_WARPS)), bt(TR_WARPS * 32);
+  // groups of source segments: ~48 warps per SM in all, 64 segments or more per
+  // group (24 and 96 warps per SM: count 161 and 98 us against 96 us, placement
+  // within 5%, at 12,000 x 27,998 with 24 M entries)
+  const int64_t want = ((int64_t)ctx->num_sms * 48 + n_tiles - 1) / n_tiles;
+  const int64_t per_part = std::max<int64_t>((n_major + want - 1) / want, 64);
+  const int parts = (int)std::max<int64_t>(1, (n_major + per_part - 1) / per_part);
+  const dim3 gt((unsigned)((n_tiles + TR_WARPS - 1) / TR_WARPS), (unsigned)parts), bt(TR_WARPS * 32);
+  DevBuf<int32_t> part_cnt((size_t)parts * n_minor);
   DevBuf<int64_t> seg(n_minor + 1);
   sv_launch(ctx, "counts_transpose_count", k_tr_count, gt, bt, 0, ptr, idx, n_major, n_minor, tshift,
-            n_tiles, (const int32_t*)toff.get(), seg.get());
+            n_tiles, (const int32_t*)toff.get(), per_part, part_cnt.get());
+  sv_launch(ctx, "counts_transpose_prefix", k_tr_prefix, dim3(sv_grid_for(ctx, n_minor, 256)), dim3(256), 0,
+            part_cnt.get(), n_minor, parts, seg.get());
   optr.alloc(n_minor + 1);
   sv_scan_i64(ctx, seg.get(), optr.get(), n_minor);
   oidx.alloc(nnz);
   ocnt.alloc(nnz);
-  // batch width: 256 source segments with many tiles, 32 with few
   const int T = 1 << tshift;
+  // batch width: 256 source segments with many tiles (77 against 108 ms for 64 at
+  // 1.3 M cells), 128 with few, where groups keep the device busy (30,000 x
+  // 33,538, 60 M entries: 1.19 ms, 1.83 and 1.55 ms for 32 and 256; one group:
+  // 3.53 ms)
   const bool wide = n_tiles >= (int64_t)ctx->num_sms * 32;
-  const int H = wide ? 8 : 1;
+  const int H = wide ? 8 : 4;
+  auto kern = wide ? k_tr_write<8> : k_tr_write<4>;
   const size_t smem = (size_t)TR_WARPS * T * (8 + 4 * H);
-  if (wide) {
-    SV_CUDA(cudaFuncSetAttribute(k_tr_write<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    sv_launch(ctx, "counts_transpose_write", k_tr_write<8>, gt, bt, smem, ptr, idx, cnt, n_major, n_minor,
-              tshift, n_tiles, (const int32_t*)toff.get(), (const int64_t*)optr.get(), oidx.get(),
-              ocnt.get());
-  } else {
-    sv_launch(ctx, "counts_transpose_write", k_tr_write<1>, gt, bt, smem, ptr, idx, cnt, n_major, n_minor,
-              tshift, n_tiles, (const int32_t*)toff.get(), (const int64_t*)optr.get(), oidx.get(),
-              ocnt.get());
-  }
+  SV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  sv_launch(ctx, "counts_transpose_write", kern, gt, bt, smem, ptr, idx, cnt, n_major, n_minor, tshift,
+            n_tiles, (const int32_t*)toff.get(), per_part, (const int32_t*)part_cnt.get(),
+            (const int64_t*)optr.get(), oidx.get(), ocnt.get());
   sv_sync(ctx);
 }
 
