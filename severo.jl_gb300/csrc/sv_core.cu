@@ -47,8 +47,23 @@ void sv_ctx_check(sv_context* ctx) {
 
 thread_local std::shared_ptr<SvPool> sv_pool;
 
+// the pool releases what it holds above its threshold, live blocks included
+void SvPool::account(int64_t delta) {
+  live += delta;
+  const int64_t want = (int64_t)live + (int64_t)keep;
+  const int64_t off = want - (int64_t)threshold;
+  if (off < (int64_t)(keep / 8) && -off < (int64_t)(keep / 8)) return;
+  uint64_t t = (uint64_t)want;
+  cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &t);
+  threshold = (size_t)want;
+}
+
 void* SvPool::alloc(size_t bytes) {
   void* p = nullptr;
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    account((int64_t)bytes);
+  }
   cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, pool, stream);
   if (e == cudaErrorMemoryAllocation) {
     // let the stream's frees take effect and give back what the pool keeps, then
@@ -60,16 +75,19 @@ void* SvPool::alloc(size_t bytes) {
   }
   if (e != cudaSuccess) {
     cudaGetLastError();
+    std::lock_guard<std::mutex> lk(mu);
+    account(-(int64_t)bytes);
     sv_throw(e == cudaErrorMemoryAllocation ? SV_ERR_OOM : SV_ERR_CUDA,
              "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
   }
   return p;
 }
 
-void SvPool::free(void* p) {
+void SvPool::free(void* p, size_t bytes) {
   std::lock_guard<std::mutex> lk(mu);
   cudaSetDevice(device);
   if (alive) {
+    account(-(int64_t)bytes);
     cudaFreeAsync(p, stream);
   } else {
     cudaFree(p);
@@ -317,9 +335,9 @@ SV_API int sv_context_create(int device, sv_context** out) {
   props.allocType = cudaMemAllocationTypePinned;
   props.location.type = cudaMemLocationTypeDevice;
   props.location.id = device;
-  uint64_t keep = (uint64_t)(prop.totalGlobalMem / SV_POOL_KEEP);
+  ctx->pool->keep = prop.totalGlobalMem / SV_POOL_KEEP;
   e = cudaMemPoolCreate(&ctx->pool->pool, &props);
-  if (e == cudaSuccess) e = cudaMemPoolSetAttribute(ctx->pool->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  if (e == cudaSuccess) ctx->pool->account(0);
   if (e != cudaSuccess) {
     cudaStreamDestroy(ctx->stream);
     delete ctx;

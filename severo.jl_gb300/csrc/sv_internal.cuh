@@ -85,8 +85,12 @@ struct SvPool {
   cudaMemPool_t pool = nullptr;
   std::mutex mu;        // blocks may be freed by other threads than the context's
   bool alive = true;    // the context's stream exists
+  size_t live = 0;      // bytes of blocks in use
+  size_t keep = 0;      // most bytes kept besides
+  size_t threshold = 0;
+  void account(int64_t delta);
   void* alloc(size_t bytes);
-  void free(void* p);
+  void free(void* p, size_t bytes);
   void close();         // the context goes away
   ~SvPool();
 };
@@ -179,13 +183,13 @@ struct DevBuf {
     release();
     if (!sv_pool) sv_throw(SV_ERR_STATE, "allocation outside a context's call");
     // pad so that 16-byte vector loads past the logical end stay inside the allocation
-    size_t bytes = (count * sizeof(T) + 64 + 255) & ~size_t(255);
-    p = (T*)sv_pool->alloc(bytes);
+    p = (T*)sv_pool->alloc(bytes(count));
     pool = sv_pool;
     n = count;
   }
+  static size_t bytes(size_t count) { return (count * sizeof(T) + 64 + 255) & ~size_t(255); }
   void release() {
-    if (p) pool->free(p);
+    if (p) pool->free(p, bytes(n));
     p = nullptr;
     n = 0;
     pool.reset();
