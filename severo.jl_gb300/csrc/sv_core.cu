@@ -369,6 +369,9 @@ SV_API int sv_context_destroy(sv_context* ctx) {
     if (p) cudaFreeHost(p);
   for (cudaEvent_t e : ctx->h_io_ev)
     if (e) cudaEventDestroy(e);
+  for (cudaEvent_t e : ctx->fork_ev)
+    if (e) cudaEventDestroy(e);
+  if (ctx->side) cudaStreamDestroy(ctx->side);
   ctx->pool->close();
   cudaStreamDestroy(ctx->stream);
   if (sv_pool == ctx->pool) sv_pool.reset();

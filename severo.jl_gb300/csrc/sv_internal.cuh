@@ -117,6 +117,9 @@ struct sv_context {
   void* h_io[2] = {nullptr, nullptr};
   size_t h_io_bytes = 0;
   cudaEvent_t h_io_ev[2] = {nullptr, nullptr};   // last transfer from / into each buffer
+  // a second stream that captured work forks to and joins from
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork_ev[2] = {nullptr, nullptr};
   // pinned read-back area of a Lanczos run (sv_ctx_run_stage)
   void* h_run = nullptr;
   size_t h_run_bytes = 0;
@@ -147,6 +150,40 @@ inline void sv_launch(sv_context* ctx, const char* name, Kern kernel, dim3 grid,
   kernel<<<grid, block, smem, ctx->stream>>>(args...);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) sv_throw(SV_ERR_CUDA, "launch of %s failed: %s", name, cudaGetErrorString(e));
+  ctx->launches++;
+  if (ctx->profiling) {
+    SV_CUDA(cudaEventRecord(b, ctx->stream));
+    ctx->pending.push_back({name, a, b});
+  }
+}
+
+// The same with thread-block clusters of `cluster` blocks along x.
+template <typename... KArgs, typename... Args>
+inline void sv_launch_cluster(sv_context* ctx, const char* name, void (*kernel)(KArgs...), dim3 grid,
+                              dim3 block, size_t smem, unsigned cluster, Args... args) {
+  cudaEvent_t a = nullptr, b = nullptr;
+  if (ctx->profiling) {
+    a = sv_ctx_event(ctx);
+    b = sv_ctx_event(ctx);
+    SV_CUDA(cudaEventRecord(a, ctx->stream));
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = cluster;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    sv_throw(SV_ERR_CUDA, "launch of %s failed: %s", name, cudaGetErrorString(e));
+  }
   ctx->launches++;
   if (ctx->profiling) {
     SV_CUDA(cudaEventRecord(b, ctx->stream));
@@ -304,6 +341,18 @@ struct sv_batch {
   DevBuf<double> upart;               // n_rb sums of u
 };
 
+// X^T u of one sample before its finish: per-feature partial sums of B^T u,
+// either per row block (FP32, rb[b * nf + f]) or per CSC chunk (FP64, chunks
+// foff[f] .. foff[f + 1] - 1), and mu.
+struct SvTPart {
+  const float* rb = nullptr;
+  int64_t n_rb = 0;
+  const double* chunk = nullptr;
+  const int64_t* foff = nullptr;
+  const double* mu = nullptr;
+  int64_t nf = 0;
+};
+
 struct sv_embed {
   sv_context* ctx = nullptr;
   int64_t n_cells = 0, npcs = 0, nf = 0;
@@ -390,6 +439,10 @@ void sv_h2d(sv_context* ctx, void* dst, const void* src, size_t bytes);
 void sv_d2h(sv_context* ctx, void* dst, const void* src, size_t bytes);
 // the context's two pinned staging buffers (SV_IO_CHUNK bytes each) and the
 // events of their last transfers (wait on them before refilling)
+// blocks and threads of the pass that sums u for X^T u (its partial sums are
+// grid-stride sums of this shape)
+constexpr int SV_UPREP_BLOCKS = 304;
+constexpr int SV_UPREP_THREADS = 256;
 constexpr size_t SV_IO_CHUNK = (size_t)64 << 20;
 void sv_ctx_io(sv_context* ctx, void* buf[2], cudaEvent_t ev[2]);
 // memcpy split over up to 8 host threads

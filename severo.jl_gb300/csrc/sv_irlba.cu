@@ -47,6 +47,9 @@ void sv_batch_apply_N_df(sv_context* ctx, const sv_batch* b, const float* xh, co
 void sv_batch_apply_T(sv_context* ctx, const sv_batch* b, const double* u, double* y,
                       const double* csub, const double* z, const int* active);
 
+void sv_centered_apply_t_part(sv_context* ctx, const sv_centered* S, const double* ud, const float* uf,
+                              SvTPart* o);
+
 namespace {
 
 constexpr int RED_BLOCKS = 608;    // blocks of the tall reductions (4 per SM)
@@ -954,73 +957,28 @@ __device__ __forceinline__ unsigned long long breakdown_tag(const double* ctl, u
 }
 
 // Basis column := x / nrm[s] (double-float) and cur := the same in FP64; the B
-// entry of sample s (B + s*bstride + boff, when B is given) := nrm[s].  When
-// nrm[s] < the sample's threshold the Krylov space is (numerically) invariant:
-// cur := a random vector, B entry := 0, flag[s] set for k_fix_df, which
-// orthonormalises cur against the basis and writes the column.  Rows of sample
-// s are indexed from its offset for the random vector (i - off).
-__global__ void k_scal_df(const float* __restrict__ xh, const float* __restrict__ xl,
-                          const BlkRange* __restrict__ blk, const int* __restrict__ seg_blk,
-                          const int64_t* __restrict__ off, const int* __restrict__ active,
-                          const double* __restrict__ nrm, const double* __restrict__ ctl,
-                          float* __restrict__ colh, float* __restrict__ coll, double* __restrict__ cur,
-                          double* __restrict__ B, int64_t boff, int64_t bstride, int* __restrict__ flag,
-                          unsigned long long seed, unsigned step) {
-  const BlkRange br = blk[blockIdx.x];
-  const int sg = br.seg;
-  if (active && !active[sg]) return;
-  const double* c = ctl + sg * CTL_N;
-  double s = nrm[sg];
-  bool brk = !(s >= c[CTL_THRESH]);
-  unsigned long long tag = breakdown_tag(c, step);
-  double inv = brk ? 0.0 : 1.0 / s;
-  for (int64_t i = br.r0 + threadIdx.x; i < br.r1; i += blockDim.x) {
-    if (brk) {
-      cur[i] = normal_at(seed, tag, i - off[sg]);
-    } else {
-      double v = df_val(xh[i], xl[i]) * inv;
-      cur[i] = v;
-      df_split(v, colh[i], coll[i]);
-    }
-  }
-  if ((int)blockIdx.x == seg_blk[sg] && threadIdx.x == 0) {
-    if (B) B[sg * bstride + boff] = brk ? 0.0 : s;
-    if (brk) flag[sg] = 1;
-  }
-}
-
-// zero the norm slot (the sub-diagonal scalar the next product uses) of every
-// sample whose breakdown was flagged, and its pending correction (cp, cell
-// side); separate launch so every k_scal_df block has read it
-__global__ void k_scal_post(double* nrm, const int* flag, int nseg, double* cp) {
-  for (int s = threadIdx.x; s < nseg; s += blockDim.x)
-    if (flag[s]) {
-      nrm[s] = 0.0;
-      // the replacement vector is orthonormalised in full: nothing pending
-      if (cp)
-        for (int j = 0; j < MAX_WORK; ++j) cp[s * MAX_WORK + j] = 0.0;
-    }
-}
-
-// One block per sample: if flag[s], cur <- CGS2(cur, Q[:, :ncols]) normalised
-// (FP64 arithmetic on the double-float basis) over the sample's rows, written to
-// the basis column as well; clears the flag.  Runs only on a breakdown.
-__global__ void k_fix_df(double* __restrict__ cur0, const int64_t* __restrict__ off,
-                         const float* __restrict__ Qh0, const float* __restrict__ Ql0, int64_t ld,
-                         int ncols, float* __restrict__ colh0, float* __restrict__ coll0,
-                         int* __restrict__ flags) {
+// entry of sample s (B + s*bstride + boff, when B is given) := nrm[s].  Rows by
+// the block schedule blk, or (blk null, one sample) grid-stride; then, on the
+// cell side, also uf := the column in FP32 and upart[block] := the FP64 sum of
+// the block's rows: the input of the X^T u product and its centring term, in
+// the order k_u_prep sums them (a pass of its own took ~7 us).
+// When nrm[s] is below the sample's threshold the Krylov space is (numerically)
+// invariant: the column becomes a random vector (rows indexed from the sample's
+// offset) orthonormalised against the basis by CGS2 (FP64 arithmetic on the
+// double-float basis), done by the last of the sample's blocks to arrive; the B
+// entry, the norm slot (the sub-diagonal scalar the next product uses) and the
+// pending correction cp become 0.  (The breakdown used to be two more launches
+// in every step, ~5 us each.)
+__device__ void scal_breakdown(int64_t o0, int64_t len, const float* __restrict__ Qh0,
+                               const float* __restrict__ Ql0, int64_t ld, int ncols,
+                               float* __restrict__ colh0, float* __restrict__ coll0, double* __restrict__ cur0,
+                               float* __restrict__ uf0, double* __restrict__ upart, int nupart) {
   __shared__ double sh[32];
   __shared__ double cs[MAX_WORK];
   __shared__ double tot;
-  const int sg = blockIdx.x;
-  int* flag = flags + sg;
-  if (*flag == 0) return;
-  const int64_t o0 = off[sg], len = off[sg + 1] - o0;
-  double* cur = cur0 + o0;
+  volatile double* cur = cur0 + o0;   // written by other blocks before the counter
   const float* Qh = Qh0 + o0;
   const float* Ql = Ql0 + o0;
-  float* colh = colh0 + o0;
-  float* coll = coll0 + o0;
   for (int pass = 0; pass < 2; ++pass) {
     for (int j = 0; j < ncols; ++j) {
       double acc = 0;
@@ -1047,14 +1005,443 @@ __global__ void k_fix_df(double* __restrict__ cur0, const int64_t* __restrict__ 
   acc = block_sum(acc, sh);
   if (threadIdx.x == 0) tot = sqrt(acc);
   __syncthreads();
-  double s = tot;
+  const double s = tot;
+  double us = 0;
   for (int64_t i = threadIdx.x; i < len; i += blockDim.x) {
     double v = cur[i] / s;
     cur[i] = v;
-    df_split(v, colh[i], coll[i]);
+    df_split(v, colh0[o0 + i], coll0[o0 + i]);
+    if (uf0) uf0[o0 + i] = (float)v;
+    us += v;
   }
+  us = block_sum(us, sh);
+  if (upart) {
+    if (threadIdx.x == 0) tot = us;
+    __syncthreads();
+    for (int b = threadIdx.x; b < nupart; b += blockDim.x) upart[b] = b == 0 ? tot : 0.0;
+  }
+}
+
+__global__ void __launch_bounds__(SV_UPREP_THREADS) k_scal(
+    const float* __restrict__ xh, const float* __restrict__ xl, const BlkRange* __restrict__ blk,
+    const int* __restrict__ seg_blk, const int64_t* __restrict__ off, const int* __restrict__ active,
+    double* __restrict__ nrm, const double* __restrict__ ctl, const float* __restrict__ Qh,
+    const float* __restrict__ Ql, int64_t ld, int ncols, float* __restrict__ colh, float* __restrict__ coll,
+    double* __restrict__ cur, float* __restrict__ uf, double* __restrict__ upart, double* __restrict__ cp,
+    double* __restrict__ B, int64_t boff, int64_t bstride, unsigned int* __restrict__ counter,
+    unsigned long long seed, unsigned step) {
+  __shared__ double red[32];
+  __shared__ bool last;
+  int sg = 0, b0 = 0, b1 = gridDim.x;
+  int64_t r0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, r1 = off[1];
+  int64_t st = (int64_t)gridDim.x * blockDim.x;
+  if (blk) {
+    const BlkRange br = blk[blockIdx.x];
+    sg = br.seg;
+    r0 = br.r0 + threadIdx.x;
+    r1 = br.r1;
+    st = blockDim.x;
+    b0 = seg_blk[sg];
+    b1 = seg_blk[sg + 1];
+  }
+  if (active && !active[sg]) return;
+  const double* c = ctl + sg * CTL_N;
+  const double s = nrm[sg];
+  if (s >= c[CTL_THRESH]) {
+    const double inv = 1.0 / s;
+    double us = 0;
+    for (int64_t i = r0; i < r1; i += st) {
+      const double v = df_val(xh[i], xl[i]) * inv;
+      cur[i] = v;
+      float h, l;
+      df_split(v, h, l);
+      colh[i] = h;
+      coll[i] = l;
+      if (uf) uf[i] = h;
+      us = __dadd_rn(us, v);   // the rounded v, as a reader of cur would sum it
+    }
+    if (upart) {
+      us = sv_warp_sum(us);
+      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = us;
+      __syncthreads();
+      if (threadIdx.x < 32) {
+        double v = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
+        v = sv_warp_sum(v);
+        if (threadIdx.x == 0) upart[blockIdx.x] = v;
+      }
+    }
+    if ((int)blockIdx.x == b0 && threadIdx.x == 0 && B) B[sg * bstride + boff] = s;
+    return;
+  }
+  const unsigned long long tag = breakdown_tag(c, step);
+  const int64_t o0 = off[sg];
+  for (int64_t i = r0; i < r1; i += st) cur[i] = normal_at(seed, tag, i - o0);
+  __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) *flag = 0;
+  if (threadIdx.x == 0) last = atomicAdd(counter + sg, 1u) == (unsigned)(b1 - b0 - 1);
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  scal_breakdown(o0, off[sg + 1] - o0, Qh, Ql, ld, ncols, colh, coll, cur, uf, upart, b1 - b0);
+  if (threadIdx.x == 0) {
+    counter[sg] = 0;
+    nrm[sg] = 0.0;
+    if (B) B[sg * bstride + boff] = 0.0;
+    if (cp)
+      for (int j = 0; j < MAX_WORK; ++j) cp[sg * MAX_WORK + j] = 0.0;
+  }
+}
+
+// ---- the feature-side step of one sample in two launches ------------------------
+// The finish of the X^T u product and the G column of cell-side column jn in one
+// pass over the features, a warp per 32 of them (the FP64 terms of a row are a
+// chain; a warp alone on its SM does not share the FP64 pipe): the arithmetic
+// and order of k_rb_finish / k_spmv_csc_finish and k_gcol.
+//   F = (sum of the partial sums - mu sum(u)) - alpha v;  F -= G[:, :jn] cp;
+//   G[:, jn] = F + alpha v
+__global__ void __launch_bounds__(32) k_gstep(const SvTPart t, const double* __restrict__ upart,
+                                              double* __restrict__ F, float* __restrict__ Gh,
+                                              float* __restrict__ Gl, int64_t ld, int jn,
+                                              const double* __restrict__ cp, const double* __restrict__ alpha,
+                                              const double* __restrict__ v) {
+  constexpr int NU = (SV_UPREP_BLOCKS + 31) / 32;
+  __shared__ double cs[MAX_WORK];
+  const int lane = threadIdx.x;
+  double up[NU];
+#pragma unroll
+  for (int k = 0; k < NU; ++k) up[k] = 32 * k + lane < SV_UPREP_BLOCKS ? upart[32 * k + lane] : 0.0;
+  for (int j = lane; j < jn; j += 32) cs[j] = cp[j];
+  const double a = *alpha;
+  const int64_t i = blockIdx.x * (int64_t)32 + lane;
+  double acc = 0, mu = 0, vi = 0;
+  if (i < t.nf) {
+    mu = t.mu[i];
+    vi = v[i];
+    if (t.rb) {
+#pragma unroll 8
+      for (int64_t b = 0; b < t.n_rb; ++b) acc += (double)t.rb[b * t.nf + i];
+    } else {
+      for (int64_t c = t.foff[i]; c < t.foff[i + 1]; ++c) acc += t.chunk[c];
+    }
+  }
+  double su = 0;
+#pragma unroll
+  for (int k = 0; k < NU; ++k)
+    if (32 * k + lane < SV_UPREP_BLOCKS) su += up[k];
+  su = sv_warp_sum(su);
+  __syncwarp();
+  if (i >= t.nf) return;
+  double out = __fma_rn(-mu, su, acc);
+  out = __dsub_rn(out, __dmul_rn(a, vi));
+  double corr = 0;
+  const float* gh = Gh + i;
+  const float* gl = Gl + i;
+  int j = 0;
+  for (; j + 8 <= jn; j += 8) {
+    float h[8], l[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      h[u] = gh[(int64_t)(j + u) * ld];
+      l[u] = gl[(int64_t)(j + u) * ld];
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) corr += df_val(h[u], l[u]) * cs[j + u];
+  }
+  for (; j < jn; ++j) corr += df_val(gh[(int64_t)j * ld], gl[(int64_t)j * ld]) * cs[j];
+  const double f = out - corr;
+  F[i] = f;
+  df_split(f + a * vi, Gh[(int64_t)jn * ld + i], Gl[(int64_t)jn * ld + i]);
+}
+
+// CGS2 of x = F against V[:, :ncols], nrm = |x| and, when write_col >= 0, the new
+// column x / |x| (double-float, FP64 copy in cur) with the B entry, or on a
+// breakdown (|x| < threshold) a random vector orthonormalised against
+// V[:, :ncols] with B entry = nrm = 0.  write_col < 0 (last step of a cycle)
+// leaves the residual in xh / xl and F.
+// One thread-block cluster instead of the four launches of orth_norm and
+// k_scal, in their arithmetic and order, bit for bit: the blocks of the
+// schedule (at most 64 rows each) are shared out over the cluster's CTAs, a
+// (block, column) dot product is one warp's, its double-float partial sums are
+// added over the blocks in FP64 by the CTA that the column belongs to, and a
+// row's update is eight chains (columns mod 8) joined in order.  What bounds it
+// is latency, so the CTA's rows of V are staged in shared memory at the start
+// (an acquire of the cluster barrier empties L1: reading them again from global
+// memory in every pass took 52 instead of 33 us at 3,000 features and ~37
+// columns) and sums cross the cluster through distributed shared memory.
+// df_fma with every rounding spelled out, the same in every context
+__device__ __forceinline__ void dfr_fma(float& sh, float& sl, float ah, float al, float bh, float bl) {
+  const float p = __fmul_rn(ah, bh);
+  float e = __fmaf_rn(ah, bh, -p);
+  e = __fmaf_rn(ah, bl, e);
+  e = __fmaf_rn(al, bh, e);
+  const float t = __fadd_rn(sh, p);
+  const float v = __fsub_rn(t, sh);
+  const float err = __fadd_rn(__fsub_rn(sh, __fsub_rn(t, v)), __fsub_rn(p, v));
+  sh = t;
+  sl = __fadd_rn(sl, __fadd_rn(err, e));
+}
+constexpr int VC_THREADS = 512;
+constexpr int VC_WARPS = VC_THREADS / 32;
+constexpr int VC_BLOCK = 64;                // most rows of a schedule block
+constexpr size_t VC_SMEM = 200 * 1024;      // most dynamic shared memory
+
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.aligned;\n barrier.cluster.wait.aligned;" ::: "memory");
+}
+// the address of the same shared-memory place in CTA q of the cluster
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, unsigned q) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(q));
+  return r;
+}
+__device__ __forceinline__ double cluster_load(const double* p, unsigned q) {
+  double v;
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(cluster_addr(p, q)) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cluster_store(float2* p, unsigned q, float2 v) {
+  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(cluster_addr(p, q)), "f"(v.x), "f"(v.y)
+               : "memory");
+}
+
+struct VCgs {
+  double* F;
+  int n, per, nblk, bpc;     // rows, rows per schedule block, blocks, blocks per CTA
+  const int* active;
+  float *Vh, *Vl;
+  int64_t ld;
+  int ncols, write_col;
+  double* nrm;
+  const double* ctl;
+  double* B;
+  int64_t boff;
+  double* cur;
+  float *xh, *xl;
+  unsigned long long seed;
+  unsigned step;
+};
+
+// the row sums of one update, K = 8 / P column classes per thread: thread (i, p)
+// takes classes K p .. K p + K - 1; complete in p == 0
+template <int K>
+__device__ __forceinline__ void vc_row_sum(const float* __restrict__ sv, int tile, int R, int ncols,
+                                           const float2* __restrict__ cs, int i, int p, bool on, float* redh,
+                                           float* redl, int rows, float& oh, float& ol) {
+  float sh[K], sl[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) sh[k] = sl[k] = 0.f;
+  if (on) {
+    for (int j0 = 0; j0 < ncols; j0 += 8) {
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const int j = j0 + K * p + k;
+        if (j < ncols) dfr_fma(sh[k], sl[k], sv[j * R + i], sv[tile + j * R + i], cs[j].x, cs[j].y);
+      }
+    }
+  }
+  if (K < 8) {
+    if (on && p > 0) {
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        redh[(K * p + k - K) * rows + i] = sh[k];
+        redl[(K * p + k - K) * rows + i] = sl[k];
+      }
+    }
+    __syncthreads();
+  }
+  oh = ol = 0.f;
+  if (on && p == 0) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) df_acc(oh, ol, sh[k], sl[k]);
+#pragma unroll
+    for (int k = K; k < 8; ++k) df_acc(oh, ol, redh[(k - K) * rows + i], redl[(k - K) * rows + i]);
+  }
+  if (K < 8) __syncthreads();
+}
+
+__global__ void __launch_bounds__(VC_THREADS) k_vcgs(const VCgs a) {
+  extern __shared__ __align__(16) float vc_dyn[];
+  __shared__ float2 csm[MAX_WORK];           // the current coefficients (hi, lo)
+  __shared__ float redh[1024], redl[1024];
+  __shared__ double bc[2];                   // |x|, 1 / |x|
+  if (a.active && !a.active[0]) return;
+  unsigned C, rank;
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(C));
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int rows = a.bpc * a.per, R = (rows + 3) & ~3;
+  const int f0 = min(rows * (int)rank, a.n);   // the CTA's first row
+  const int nr = min(rows, a.n - f0);
+  const int nb = (nr + a.per - 1) / a.per;     // its schedule blocks
+  const int ncols = a.ncols;
+  const int tile = ncols * R;
+  float* sv = vc_dyn;                          // V hi, V lo
+  float* sxh = sv + 2 * tile;
+  float* sxl = sxh + R;
+  double* part = (double*)(sxl + R);           // [block][column]
+  double* npart = part + a.bpc * ncols;        // [block]
+  double* hsum = npart + a.bpc;                // [block][half]
+  for (int col = w; col < 2 * ncols; col += VC_WARPS) {
+    const int c = col >= ncols ? col - ncols : col;
+    const float* src = (col >= ncols ? a.Vl : a.Vh) + (int64_t)c * a.ld + f0;
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(sv + col * R);
+    if ((rows & 3) == 0) {
+      // 16-byte copies may read up to 3 rows past the CTA's, inside the padded
+      // leading dimension; nothing uses them
+      for (int k = lane; 4 * k < nr; k += 32)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * k), "l"(src + 4 * k) : "memory");
+    } else {
+      for (int k = lane; k < nr; k += 32)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 4 * k), "l"(src + k) : "memory");
+    }
+  }
+  for (int i = tid; i < nr; i += VC_THREADS) df_split(a.F[f0 + i], sxh[i], sxl[i]);
+  asm volatile("cp.async.commit_group;\n cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  const int rpad = (nr + 31) & ~31;
+  const int P = rpad <= 128 ? 4 : rpad <= 256 ? 2 : 1;   // threads per row
+  const double thresh = a.ctl[CTL_THRESH];
+  bool brk = false;
+  double s = 0;
+  for (int phase = 0;;) {
+    if (ncols > 0) {
+      // the blocks' dot products V[:, c] . x, four (block, column) pairs per warp at a time
+      const int ntask = nb * ncols;
+      for (int t0 = w; t0 < ntask; t0 += 4 * VC_WARPS) {
+        float h[4], l[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          h[u] = l[u] = 0.f;
+          const int tk = t0 + u * VC_WARPS;
+          if (tk < ntask) {
+            const int lb = tk / ncols, c = tk - lb * ncols;
+            const int i = lb * a.per + lane, e = min(nr, (lb + 1) * a.per);
+            const float* qh = sv + c * R;
+            const float* ql = qh + tile;
+            const bool va = i < e, vb = i + 32 < e;
+            dfr_fma(h[u], l[u], va ? qh[i] : 0.f, va ? ql[i] : 0.f, va ? sxh[i] : 0.f, va ? sxl[i] : 0.f);
+            dfr_fma(h[u], l[u], vb ? qh[i + 32] : 0.f, vb ? ql[i + 32] : 0.f, vb ? sxh[i + 32] : 0.f,
+                   vb ? sxl[i + 32] : 0.f);
+          }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            float h2 = __shfl_xor_sync(0xffffffffu, h[u], o);
+            float l2 = __shfl_xor_sync(0xffffffffu, l[u], o);
+            float sm = h[u] + h2;
+            float v = sm - h[u];
+            float err = (h[u] - (sm - v)) + (h2 - v);
+            float lo = err + l[u] + l2;
+            h[u] = sm + lo;
+            l[u] = lo - (h[u] - sm);
+          }
+        }
+        if (lane == 0) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (t0 + u * VC_WARPS < ntask) part[t0 + u * VC_WARPS] = df_val(h[u], l[u]);
+        }
+      }
+      __syncthreads();
+      cluster_sync();
+      // column c belongs to CTA c mod C: the blocks' sums in order, then to every CTA
+      for (int c = (int)rank + (int)C * w; c < ncols; c += (int)C * VC_WARPS) {
+        double t = 0;
+        for (int b = lane; b < a.nblk; b += 32) {
+          const int q = b / a.bpc;
+          t += cluster_load(part + (b - q * a.bpc) * ncols + c, q);
+        }
+        t = sv_warp_sum(t);
+        if (lane < (int)C) {
+          float2 v;
+          df_split(t, v.x, v.y);
+          cluster_store(csm + c, lane, v);
+        }
+      }
+      cluster_sync();
+      // x -= V c
+      if (P == 1) {
+        for (int i = tid; i < nr; i += VC_THREADS) {
+          float sh, sl;
+          vc_row_sum<8>(sv, tile, R, ncols, csm, i, 0, true, redh, redl, 0, sh, sl);
+          float h = sxh[i], l = sxl[i];
+          df_sub(h, l, sh, sl);
+          sxh[i] = h;
+          sxl[i] = l;
+        }
+      } else {
+        const int rw = VC_THREADS / P, p = tid / rw, i = tid - p * rw;
+        float sh, sl;
+        if (P == 2) vc_row_sum<4>(sv, tile, R, ncols, csm, i, p, i < nr, redh, redl, rw, sh, sl);
+        else vc_row_sum<2>(sv, tile, R, ncols, csm, i, p, i < nr, redh, redl, rw, sh, sl);
+        if (p == 0 && i < nr) {
+          float h = sxh[i], l = sxl[i];
+          df_sub(h, l, sh, sl);
+          sxh[i] = h;
+          sxl[i] = l;
+        }
+      }
+      __syncthreads();
+    }
+    if (++phase < 2) continue;
+    // |x|: per block two half sums, then the blocks in order
+    for (int t = w; t < 2 * nb; t += VC_WARPS) {
+      const int lb = t >> 1, r = 32 * (t & 1) + lane, i = lb * a.per + r;
+      double v = 0;
+      if (r < a.per && i < nr) {
+        const double x = df_val(sxh[i], sxl[i]);
+        v = x * x;
+      }
+      v = sv_warp_sum(v);
+      if (lane == 0) hsum[t] = v;
+    }
+    __syncthreads();
+    for (int lb = tid; lb < nb; lb += VC_THREADS) npart[lb] = hsum[2 * lb] + hsum[2 * lb + 1];
+    __syncthreads();
+    cluster_sync();
+    if (w == 0) {
+      double t = 0;
+      for (int b0 = 0; b0 < a.nblk; b0 += 32) {
+        const int b = b0 + lane, q = b / a.bpc;
+        const double v = b < a.nblk ? cluster_load(npart + (b - q * a.bpc), q) : 0.0;
+        const int m = min(32, a.nblk - b0);
+        for (int k = 0; k < m; ++k) t += __shfl_sync(0xffffffffu, v, k);
+      }
+      if (lane == 0) {
+        const double r = sqrt(t);
+        bc[0] = r;
+        bc[1] = 1.0 / r;
+      }
+    }
+    __syncthreads();
+    if (!brk) s = bc[0];
+    if (a.write_col < 0 || brk || s >= thresh) break;
+    brk = true;
+    s = 0.0;
+    phase = 0;
+    const unsigned long long tag = breakdown_tag(a.ctl, a.step);
+    for (int i = tid; i < nr; i += VC_THREADS) df_split(normal_at(a.seed, tag, f0 + i), sxh[i], sxl[i]);
+    __syncthreads();
+  }
+  const double inv = bc[1];
+  for (int i = tid; i < nr; i += VC_THREADS) {
+    if (a.write_col < 0) {
+      a.xh[f0 + i] = sxh[i];
+      a.xl[f0 + i] = sxl[i];
+      a.F[f0 + i] = df_val(sxh[i], sxl[i]);
+    } else {
+      const double v = df_val(sxh[i], sxl[i]) * inv;
+      a.cur[f0 + i] = v;
+      df_split(v, a.Vh[(int64_t)a.write_col * a.ld + f0 + i], a.Vl[(int64_t)a.write_col * a.ld + f0 + i]);
+    }
+  }
+  if (rank == 0 && tid == 0) {
+    a.nrm[0] = s;
+    if (a.B) a.B[a.boff] = s;
+  }
+  cluster_sync();                            // no CTA leaves while its sums are read
 }
 
 // The whole feature-side step of a sample in one block (the feature side is
@@ -1523,6 +1910,10 @@ struct Op {
   virtual void N(const double* x, double* y, const double* csub, const double* z) = 0;
   // y = A^T x - (csub ? *csub : 0) * z      (x in R^m, y in R^n)
   virtual void T(const double* x, double* y, const double* csub, const double* z) = 0;
+  // A^T x up to its partial sums (x as FP64 and FP32), which k_gstep finishes,
+  // where the operator has that form
+  virtual bool has_part() const { return false; }
+  virtual void T_part(const double* x, const float* xf, SvTPart* o) { (void)x, (void)xf, (void)o; }
   // true when N and T only enqueue device work (no host round trip), so that a
   // Lanczos cycle over them can be captured as a CUDA graph
   virtual bool device_only() const { return false; }
@@ -1545,6 +1936,10 @@ struct CenteredOp : Op {
   }
   void T(const double* x, double* y, const double* csub, const double* z) override {
     sv_centered_apply(ctx, S, 'T', x, y, 1.0, 0.0, csub, z);
+  }
+  bool has_part() const override { return S->n_rb > 0 || S->t_blocks == 0; }
+  void T_part(const double* x, const float* xf, SvTPart* o) override {
+    sv_centered_apply_t_part(ctx, S, x, xf, o);
   }
   bool device_only() const override { return true; }
   bool N_df(const float* xh, const float* xl, float* yh, float* yl, const double* csub,
@@ -1725,13 +2120,19 @@ struct Lanczos {
   DevBuf<unsigned char> rot_b;
   DevBuf<int> rot_f;
   DevBuf<unsigned int> counter;
-  DevBuf<int> flag, active, finsel;
+  DevBuf<int> active, finsel;
+  DevBuf<float> uf;             // the current cell-side vector in FP32 (X^T u's input)
+  DevBuf<double> upart;         // and its partial sums
   double* hsum = nullptr;       // pinned copy of the cycle summaries
   int* hflags = nullptr;        // pinned staging of the active / finish masks
   double eps_b = 0;
   int cgs_blocks = RED_BLOCKS;  // resident blocks of the CGS kernels (one wave)
   bool vside_multi = false;     // feature side through the multi-block kernels
   bool lag_tma = false;         // the cell-side pass with TMA-fed basis tiles
+  bool vfused = false;          // feature side of one sample as k_gstep + k_vcgs
+  int vcluster = 16, vper = 0, vbpc = 0;   // its cluster, rows per block, blocks per CTA
+  size_t vsmem = 0;
+  bool capturing = false;
   // graphs of the first cycle and of restart cycles from basis set 0 / set 1
   CycleGraph graphs[3];
 
@@ -1781,6 +2182,11 @@ struct Lanczos {
       vside_multi = Vs.max_seg > 32768 || (nseg == 1 && Vs.len >= 1024);
       if (mode && strcmp(mode, "multi") == 0) vside_multi = true;
       if (mode && strcmp(mode, "block") == 0 && Vs.max_seg <= 32768) vside_multi = false;
+      // over a device matrix with partial sums the multi-block kernels of one
+      // sample are joined in k_gstep and k_vcgs while the schedule's blocks have
+      // at most 64 rows and a CTA's rows of V fit its shared memory (409,000
+      // basis entries over 16 CTAs: 7,000 features at 57 columns)
+      if (vside_multi && nseg == 1 && !mode && op->device_only() && op->has_part()) vfused_setup();
     }
     ytmp.alloc(std::max(m, n));
     F.alloc(n);
@@ -1799,14 +2205,14 @@ struct Lanczos {
     }
     rot_b.alloc(6 * 64 * 64 * 2);
     rot_f.alloc(64);
-    counter.alloc(4);
-    flag.alloc(nseg);
+    counter.alloc(4 + nseg);   // [0] the CGS passes; [4 + s] breakdowns of sample s
+    uf.alloc(vfused ? m : 1);
+    upart.alloc(SV_UPREP_BLOCKS);
     active.alloc(nseg);
     finsel.alloc(nseg);
     Ufin.alloc(m * nu);
     Vfin.alloc(n * nu);
-    sv_memset(ctx, counter.get(), 0, 16);
-    sv_memset(ctx, flag.get(), 0, nseg * 4);
+    sv_memset(ctx, counter.get(), 0, (4 + nseg) * 4);
     sv_memset(ctx, B.get(), 0, (size_t)nseg * work * work * 8);
     hsum = (double*)sv_ctx_run_stage(ctx, (size_t)nseg * (2 * work + 2) * 8 + (size_t)nseg * 4);
     hflags = (int*)(hsum + (size_t)nseg * (2 * work + 2));
@@ -1870,20 +2276,104 @@ struct Lanczos {
     else orth_norm_nj<12>(s, y, ncols, nrm);
   }
 
+  void vfused_setup() {
+    vper = (int)((n + Vs.red.nblk - 1) / Vs.red.nblk);
+    const int nblk = (int)((n + vper - 1) / vper);
+    if (vper > VC_BLOCK || nblk != Vs.red.nblk) return;
+    SV_CUDA(cudaFuncSetAttribute(k_vcgs, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    SV_CUDA(cudaFuncSetAttribute(k_vcgs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)VC_SMEM));
+    for (vcluster = 16; vcluster >= 8; vcluster /= 2) {
+      vbpc = (nblk + vcluster - 1) / vcluster;
+      const size_t R = ((size_t)vbpc * vper + 3) & ~(size_t)3;
+      vsmem = (size_t)vbpc * (work + 3) * 8 + R * 8 * (1 + (size_t)work);
+      if (vsmem > VC_SMEM) return;
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute at[1];
+      cfg.gridDim = dim3(vcluster);
+      cfg.blockDim = dim3(VC_THREADS);
+      cfg.dynamicSmemBytes = vsmem;
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = vcluster;
+      at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      int fit = 0;
+      if (cudaOccupancyMaxActiveClusters(&fit, k_vcgs, &cfg) == cudaSuccess && fit > 0) {
+        vfused = true;
+        break;
+      }
+      cudaGetLastError();
+    }
+    if (vfused && !ctx->side) {
+      SV_CUDA(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
+      for (cudaEvent_t& e : ctx->fork_ev) SV_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    }
+  }
+
   // basis column j := working vector / nrm[s] (FP64 copy in cur), breakdown
-  // handling; the B entry at offset boff of each sample's B (boff < 0: none)
-  void scal_fix(Side& s, int j, double* nrm, const double* c, int64_t boff, uint64_t seed,
-                unsigned step) {
-    sv_launch(ctx, "irlba_scal", k_scal_df, dim3(s.red.nblk), dim3(256), 0, (const float*)s.xh.get(),
-              (const float*)s.xl.get(), (const BlkRange*)s.red.blk.get(), (const int*)s.red.seg_blk.get(),
-              (const int64_t*)s.off.get(), (const int*)active.get(), (const double*)nrm, c, s.ch(j),
-              s.cl(j), s.cur.get(), boff >= 0 ? B.get() : (double*)nullptr, boff,
-              (int64_t)work * work, flag.get(), (unsigned long long)seed, step);
-    sv_launch(ctx, "irlba_scal_post", k_scal_post, dim3(1), dim3(64), 0, nrm, (const int*)flag.get(),
-              nseg, &s == &Ws ? cpv() : (double*)nullptr);
-    sv_launch(ctx, "irlba_fix", k_fix_df, dim3(nseg), dim3(1024), 0, s.cur.get(),
-              (const int64_t*)s.off.get(), (const float*)s.bh(), (const float*)s.bl(), s.ld, j, s.ch(j),
-              s.cl(j), flag.get());
+  // handling; the B entry at offset boff of each sample's B (boff < 0: none).  On
+  // the cell side of a fused run also the input of the X^T u product.
+  void scale_col(Side& s, int j, double* nrm, const double* c, int64_t boff, uint64_t seed, unsigned step) {
+    const bool W = &s == &Ws, u = W && vfused;
+    sv_launch(ctx, "irlba_scal", k_scal, dim3(u ? SV_UPREP_BLOCKS : s.red.nblk), dim3(SV_UPREP_THREADS), 0,
+              (const float*)s.xh.get(), (const float*)s.xl.get(),
+              u ? (const BlkRange*)nullptr : (const BlkRange*)s.red.blk.get(), (const int*)s.red.seg_blk.get(),
+              (const int64_t*)s.off.get(), (const int*)active.get(), nrm, c, (const float*)s.bh(),
+              (const float*)s.bl(), s.ld, j, s.ch(j), s.cl(j), s.cur.get(), u ? uf.get() : (float*)nullptr,
+              u ? upart.get() : (double*)nullptr, W ? cpv() : (double*)nullptr,
+              boff >= 0 ? B.get() : (double*)nullptr, boff, (int64_t)work * work, counter.get() + 4,
+              (unsigned long long)seed, step);
+  }
+
+  // the feature-side step of a fused run after the product of cell-side column
+  // jc (its partial sums in tp): k_gstep, k_vcgs
+  void vside_fused(const SvTPart& tp, int jc, int write_col, double* nrm, const double* c, int64_t boff,
+                   uint64_t seed, unsigned step) {
+    sv_launch(ctx, "irlba_gstep", k_gstep, dim3((unsigned)((n + 31) / 32)), dim3(32), 0, tp,
+              (const double*)upart.get(), F.get(), Gh(), Gl(), n, jc, (const double*)cpv(), (const double*)sS(),
+              (const double*)Vs.cur.get());
+    VCgs a;
+    a.F = F.get();
+    a.n = (int)n;
+    a.per = vper;
+    a.nblk = Vs.red.nblk;
+    a.bpc = vbpc;
+    a.active = active.get();
+    a.Vh = Vs.bh();
+    a.Vl = Vs.bl();
+    a.ld = Vs.ld;
+    a.ncols = jc + 1;
+    a.write_col = write_col;
+    a.nrm = nrm;
+    a.ctl = c;
+    a.B = boff >= 0 ? B.get() : (double*)nullptr;
+    a.boff = boff;
+    a.cur = Vs.cur.get();
+    a.xh = Vs.xh.get();
+    a.xl = Vs.xl.get();
+    a.seed = seed;
+    a.step = step;
+    sv_launch_cluster(ctx, "irlba_vcgs", k_vcgs, dim3((unsigned)vcluster), dim3(VC_THREADS), vsmem,
+                      (unsigned)vcluster, a);
+  }
+
+  // Work between fork() and join() runs beside what is launched between split()
+  // and join(): captured on a second stream (direct launches stay in line).
+  cudaStream_t main_stream = nullptr;
+  void fork() {
+    if (!capturing) return;
+    main_stream = ctx->stream;
+    SV_CUDA(cudaEventRecord(ctx->fork_ev[0], main_stream));
+    SV_CUDA(cudaStreamWaitEvent(ctx->side, ctx->fork_ev[0], 0));
+    ctx->stream = ctx->side;
+  }
+  void split() {
+    if (!capturing) return;
+    SV_CUDA(cudaEventRecord(ctx->fork_ev[1], ctx->side));
+    ctx->stream = main_stream;
+  }
+  void join() {
+    if (capturing) SV_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->fork_ev[1], 0));
   }
 
   // the feature-side step: one block per sample (k_vside), or the multi-block
@@ -1892,7 +2382,7 @@ struct Lanczos {
              unsigned step) {
     if (vside_multi) {
       orth_norm(Vs, F.get(), ncols, nrm);
-      if (write_col >= 0) scal_fix(Vs, write_col, nrm, c, boff, seed, step);
+      if (write_col >= 0) scale_col(Vs, write_col, nrm, c, boff, seed, step);
       return;
     }
     sv_launch(ctx, "irlba_vside", k_vside, dim3(nseg), dim3(1024), 0, (const double*)F.get(),
@@ -1936,17 +2426,20 @@ struct Lanczos {
               work, M, (int64_t)work * work, nout, outh, outl, outd, ld_out);
   }
 
+  void gdots(int jn, int pend) {
+    sv_launch(ctx, "irlba_gdots", k_gdots, dim3(jn, nseg), dim3(256), 0, (const float*)Gh(),
+              (const float*)Gl(), n, (const int64_t*)Vs.off.get(), (const double*)Vs.cur.get(), pend,
+              (const double*)sR(), (const double*)cpv(), (const int*)active.get(), c0v());
+  }
+
   // The cell-side CGS2 step of column jn in one pass over the basis (k_cgs_lag):
-  // first-projection coefficients from G (k_gdots), the pending column pend
+  // first-projection coefficients from G (gdots, launched before), the pending column pend
   // (the previous step's, or -1) corrected on the way; y: the FP64 product, or
   // null when the product is in the working vector.  s0 = the norm per sample,
   // cp = the new column's pending correction.
   template <int NJ>
   void w_step_nj(int jn, int pend, const double* y) {
     const int g = Ws.lag.nblk;
-    sv_launch(ctx, "irlba_gdots", k_gdots, dim3(jn, nseg), dim3(256), 0, (const float*)Gh(),
-              (const float*)Gl(), n, (const int64_t*)Vs.off.get(), (const double*)Vs.cur.get(), pend,
-              (const double*)sR(), (const double*)cpv(), (const int*)active.get(), c0v());
     if (NJ == 8 && lag_tma) {
       // the basis columns 0..jn-1 as two 2D tensors (rows x jn columns, 16-byte
       // column stride), boxes of 64 rows x 8 columns
@@ -2024,7 +2517,7 @@ struct Lanczos {
                  act);
       Vs.flip();
       Ws.flip();
-      df_residual_to_fp64();
+      if (!vfused) df_residual_to_fp64();
       dim3 grid((unsigned)std::max(1, std::min(sv_grid_for(ctx, Vs.max_seg, 256, 4), 64)), (unsigned)nseg);
       sv_launch(ctx, "irlba_restart", k_restart_tail, grid, dim3(256), 0, Vs.ch(k), Vs.cl(k),
                 Vs.cur.get(), (const double*)F.get(), (const int64_t*)Vs.off.get(),
@@ -2033,39 +2526,58 @@ struct Lanczos {
     unsigned step = 1;
     int j = k;
     // W[:, j] = A V[:, j]; CGS2 against W[:, :j] (the first column of a run:
-    // its norm only)
+    // its norm only); the first projection's coefficients beside the product
     bool pending = false;
-    if (op->N_df(Vs.ch(j), Vs.cl(j), Ws.xh.get(), Ws.xl.get(), nullptr, nullptr, nullptr)) {
-      if (j == 0) orth_norm(Ws, nullptr, 0, s0);
-      else w_step(j, -1, nullptr);
-    } else {
+    if (j > 0) {
+      fork();
+      gdots(j, -1);
+      split();
+    }
+    const double* y = nullptr;
+    if (!op->N_df(Vs.ch(j), Vs.cl(j), Ws.xh.get(), Ws.xl.get(), nullptr, nullptr, nullptr)) {
       op->N(Vs.cur.get(), ytmp.get(), nullptr, nullptr);
-      if (j == 0) orth_norm(Ws, ytmp.get(), 0, s0);
-      else w_step(j, -1, ytmp.get());
+      y = ytmp.get();
+    }
+    if (j == 0) {
+      orth_norm(Ws, y, 0, s0);
+    } else {
+      join();
+      w_step(j, -1, y);
     }
     pending = j > 0;
     nmv++;
-    scal_fix(Ws, j, s0, c, (int64_t)j * work + j, seed, step++);
+    scale_col(Ws, j, s0, c, (int64_t)j * work + j, seed, step++);
     while (true) {
       // F = A^T W[:, j] - S V[:, j]; CGS2 against V[:, :j+1]
-      op->T(Ws.cur.get(), F.get(), s0, Vs.cur.get());
+      SvTPart tp;
+      if (vfused) {
+        op->T_part(Ws.cur.get(), uf.get(), &tp);
+      } else {
+        op->T(Ws.cur.get(), F.get(), s0, Vs.cur.get());
+        g_col(j);
+      }
       nmv++;
-      g_col(j);
       if (j + 1 < work) {
-        vside(j + 1, j + 1, s1, c, (int64_t)j * work + j + 1, seed, step++);
+        if (vfused) vside_fused(tp, j, j + 1, s1, c, (int64_t)j * work + j + 1, seed, step++);
+        else vside(j + 1, j + 1, s1, c, (int64_t)j * work + j + 1, seed, step++);
         // W[:, j+1] = A V[:, j+1] - R W[:, j]
-        if (op->N_df(Vs.ch(j + 1), Vs.cl(j + 1), Ws.xh.get(), Ws.xl.get(), s1, Ws.ch(j), Ws.cl(j))) {
-          w_step(j + 1, j, nullptr);
-        } else {
+        fork();
+        gdots(j + 1, j);
+        split();
+        y = nullptr;
+        if (!op->N_df(Vs.ch(j + 1), Vs.cl(j + 1), Ws.xh.get(), Ws.xl.get(), s1, Ws.ch(j), Ws.cl(j))) {
           op->N(Vs.cur.get(), ytmp.get(), s1, Ws.cur.get());
-          w_step(j + 1, j, ytmp.get());
+          y = ytmp.get();
         }
+        join();
+        w_step(j + 1, j, y);
         pending = true;
         nmv++;
-        scal_fix(Ws, j + 1, s0, c, (int64_t)(j + 1) * work + j + 1, seed, step++);
+        scale_col(Ws, j + 1, s0, c, (int64_t)(j + 1) * work + j + 1, seed, step++);
         ++j;
       } else {
-        vside(j + 1, -1, s1, c, -1, seed, step++);   // residual f and |f|
+        if (vfused) vside_fused(tp, j, -1, s1, c, -1, seed, step++);   // residual f and |f|
+        else vside(j + 1, -1, s1, c, -1, seed, step++);
         break;
       }
     }
@@ -2093,8 +2605,12 @@ struct Lanczos {
       cudaGraph_t graph = nullptr;
       SV_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
       try {
+        capturing = ctx->side != nullptr;
         g.matvecs = cycle(restart, k, seed);
+        capturing = false;
       } catch (...) {
+        if (capturing && main_stream) ctx->stream = main_stream;
+        capturing = false;
         cudaStreamEndCapture(ctx->stream, &graph);
         if (graph) cudaGraphDestroy(graph);
         cudaGetLastError();

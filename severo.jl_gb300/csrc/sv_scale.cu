@@ -1396,13 +1396,73 @@ __global__ void k_spmv_csc_finish(const double* __restrict__ partial,
   }
 }
 
-constexpr int UPREP_BLOCKS = 304;
+constexpr int UPREP_BLOCKS = SV_UPREP_BLOCKS;
 
 }  // namespace
 
 // ---------------------------------------------------------------------------
 // internal product entry points (device vectors), used by irlba too
 // ---------------------------------------------------------------------------
+// row-blocked CSC: u (FP32) staged per row block in shared memory
+static void launch_rb(sv_context* ctx, const sv_centered* S, const float* uf) {
+  sv_centered* Sm = const_cast<sv_centered*>(S);
+  // one wave of resident blocks, ~6 tasks (row block, feature group) each,
+  // at least 32 features per task
+  const int resident = ctx->num_sms * S->rb_per_sm;
+  const int fg = (int)std::max<int64_t>(
+      1, std::min<int64_t>(std::max<int64_t>(1, S->nf / 32), (6 * resident + S->n_rb - 1) / S->n_rb));
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(resident, S->n_rb * fg));
+  size_t smem = RB_ROWS * sizeof(float);
+  if (S->dtype == SV_F32)
+    sv_launch(ctx, "spmv_rb", k_spmv_rb_waves<float>, dim3(grid), dim3(RB_THREADS), smem,
+              (const int64_t*)S->rb_ptr.get(), (const unsigned long long*)S->rb_idx.get(),
+              (const float*)S->rb_val.get(), S->nf, S->n_cells, S->n_rb, fg,
+              (const float*)S->inv_std_f.get(), (const float*)S->clip_f.get(), uf, Sm->rb_partial.get());
+  else
+    sv_launch(ctx, "spmv_rb", k_spmv_rb_waves<__nv_bfloat16>, dim3(grid), dim3(RB_THREADS), smem,
+              (const int64_t*)S->rb_ptr.get(), (const unsigned long long*)S->rb_idx.get(),
+              (const __nv_bfloat16*)S->rb_val.get(), S->nf, S->n_cells, S->n_rb, fg,
+              (const float*)S->inv_std_f.get(), (const float*)S->clip_f.get(), uf, Sm->rb_partial.get());
+}
+
+// CSC chunks over the feature ranges: u FP32 (uf) or, for FP64 data, FP64 (ud)
+static void launch_chunks(sv_context* ctx, const sv_centered* S, const double* ud, const float* uf) {
+  sv_centered* Sm = const_cast<sv_centered*>(S);
+  int grid = sv_grid_for(ctx, S->n_chunks * 32, 256, 8);
+  const sv_data* D = S->data;
+  const int32_t* rowidx = D->counts->csc_rowidx.get();
+#define LAUNCH_CSC(VT)                                                                            \
+  sv_launch(ctx, "spmv_csc_chunks", k_spmv_csc_chunks<VT>, dim3(grid), dim3(256), 0, rowidx,      \
+            (const VT*)D->csc_val.get(), (const int32_t*)S->chunk_feat.get(),                     \
+            (const int64_t*)S->chunk_start.get(), (const int64_t*)S->chunk_end.get(), S->n_chunks, \
+            (const float*)S->inv_std_f.get(), (const float*)S->clip_f.get(),                      \
+            (const double*)S->inv_std_d.get(), (const double*)S->clip_d.get(), uf, ud,            \
+            Sm->chunk_partial.get())
+  switch (S->dtype) {
+    case SV_F64: LAUNCH_CSC(double); break;
+    case SV_F32: LAUNCH_CSC(float); break;
+    default: LAUNCH_CSC(__nv_bfloat16); break;
+  }
+#undef LAUNCH_CSC
+}
+
+// The partial sums of X^T u alone, for a caller that finishes them itself (the
+// Lanczos feature side): u as FP64 and as FP32.  Not for the form over CSR_h.
+void sv_centered_apply_t_part(sv_context* ctx, const sv_centered* S, const double* ud, const float* uf,
+                              SvTPart* o) {
+  o->mu = S->mu.get();
+  o->nf = S->nf;
+  if (S->n_rb > 0) {
+    launch_rb(ctx, S, uf);
+    o->rb = S->rb_partial.get();
+    o->n_rb = S->n_rb;
+  } else {
+    launch_chunks(ctx, S, ud, uf);
+    o->chunk = S->chunk_partial.get();
+    o->foff = S->feat_chunk_off.get();
+  }
+}
+
 void sv_centered_apply(sv_context* ctx, const sv_centered* S, char trans, const double* x, double* y,
                        double alpha, double beta, const double* csub, const double* z) {
   if (trans == 'N') {
@@ -1432,29 +1492,10 @@ void sv_centered_apply(sv_context* ctx, const sv_centered* S, char trans, const 
     }
 #undef LAUNCH_CSR
   } else if (S->n_rb > 0) {
-    // row-blocked CSC: u staged per row block in shared memory
     sv_centered* Sm = const_cast<sv_centered*>(S);
-    sv_launch(ctx, "spmv_csc_uprep", k_u_prep, dim3(UPREP_BLOCKS), dim3(256), 0, x, S->n_cells,
+    sv_launch(ctx, "spmv_csc_uprep", k_u_prep, dim3(UPREP_BLOCKS), dim3(SV_UPREP_THREADS), 0, x, S->n_cells,
               Sm->u_f32.get(), Sm->red_partial.get());
-    // one wave of resident blocks, ~6 tasks (row block, feature group) each,
-    // at least 32 features per task
-    const int resident = ctx->num_sms * S->rb_per_sm;
-    const int fg = (int)std::max<int64_t>(
-        1, std::min<int64_t>(std::max<int64_t>(1, S->nf / 32), (6 * resident + S->n_rb - 1) / S->n_rb));
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(resident, S->n_rb * fg));
-    size_t smem = RB_ROWS * sizeof(float);
-    if (S->dtype == SV_F32)
-      sv_launch(ctx, "spmv_rb", k_spmv_rb_waves<float>, dim3(grid), dim3(RB_THREADS), smem,
-                (const int64_t*)S->rb_ptr.get(), (const unsigned long long*)S->rb_idx.get(),
-                (const float*)S->rb_val.get(), S->nf, S->n_cells, S->n_rb, fg,
-                (const float*)S->inv_std_f.get(), (const float*)S->clip_f.get(),
-                (const float*)Sm->u_f32.get(), Sm->rb_partial.get());
-    else
-      sv_launch(ctx, "spmv_rb", k_spmv_rb_waves<__nv_bfloat16>, dim3(grid), dim3(RB_THREADS), smem,
-                (const int64_t*)S->rb_ptr.get(), (const unsigned long long*)S->rb_idx.get(),
-                (const __nv_bfloat16*)S->rb_val.get(), S->nf, S->n_cells, S->n_rb, fg,
-                (const float*)S->inv_std_f.get(), (const float*)S->clip_f.get(),
-                (const float*)Sm->u_f32.get(), Sm->rb_partial.get());
+    launch_rb(ctx, S, S->u_f32.get());
     sv_launch(ctx, "spmv_rb_finish", k_rb_finish, dim3(sv_grid_for(ctx, S->nf, 256, 4)), dim3(256), 0,
               (const float*)Sm->rb_partial.get(), S->n_rb, S->nf, (const double*)S->mu.get(),
               (const double*)Sm->red_partial.get(), UPREP_BLOCKS, alpha, beta, y, csub, z);
@@ -1500,22 +1541,7 @@ void sv_centered_apply(sv_context* ctx, const sv_centered* S, char trans, const 
     bool f64 = S->dtype == SV_F64;
     sv_launch(ctx, "spmv_csc_uprep", k_u_prep, dim3(UPREP_BLOCKS), dim3(256), 0, x, S->n_cells,
               f64 ? (float*)nullptr : Sm->u_f32.get(), Sm->red_partial.get());
-    int grid = sv_grid_for(ctx, S->n_chunks * 32, 256, 8);
-    const sv_data* D = S->data;
-    const int32_t* rowidx = D->counts->csc_rowidx.get();
-#define LAUNCH_CSC(VT)                                                                            \
-  sv_launch(ctx, "spmv_csc_chunks", k_spmv_csc_chunks<VT>, dim3(grid), dim3(256), 0, rowidx,      \
-            (const VT*)D->csc_val.get(), (const int32_t*)S->chunk_feat.get(),                     \
-            (const int64_t*)S->chunk_start.get(), (const int64_t*)S->chunk_end.get(), S->n_chunks, \
-            (const float*)S->inv_std_f.get(), (const float*)S->clip_f.get(),                      \
-            (const double*)S->inv_std_d.get(), (const double*)S->clip_d.get(),                    \
-            (const float*)Sm->u_f32.get(), x, Sm->chunk_partial.get())
-    switch (S->dtype) {
-      case SV_F64: LAUNCH_CSC(double); break;
-      case SV_F32: LAUNCH_CSC(float); break;
-      default: LAUNCH_CSC(__nv_bfloat16); break;
-    }
-#undef LAUNCH_CSC
+    launch_chunks(ctx, S, x, S->u_f32.get());
     sv_launch(ctx, "spmv_csc_finish", k_spmv_csc_finish, dim3(sv_grid_for(ctx, S->nf, 256, 4)),
               dim3(256), 0, (const double*)S->chunk_partial.get(),
               (const int64_t*)S->feat_chunk_off.get(), S->nf, (const double*)S->mu.get(),
