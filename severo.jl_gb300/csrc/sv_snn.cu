@@ -14,11 +14,13 @@
 // or one block over a global scratch buffer (larger hubs).  The warp and block
 // forms count the candidates in a shared-memory hash table (row and count
 // packed in one 32-bit word, open addressing, at least 1.5 times as many slots
-// as candidates), keep the entries whose weight passes the prune threshold, and
-// sort only those by row; the hub form (and rows or k too large for the
-// packing) sorts all candidates and reads the counts as run lengths.  Two
-// passes: count the kept entries, scan, write.  All integer work; the one
-// division is IEEE-correctly rounded.
+// as candidates), keep the entries whose weight passes the prune threshold, sort
+// only those by row and leave them as packed words in an arena; once the kept
+// counts are scanned, a second kernel writes rows and weights from there.  The
+// hub form (and rows or k too large for the packing, or an arena above 1/16 of
+// the device's memory) sorts all candidates, reads the counts as run lengths and
+// runs twice: count the kept entries, scan, write.  All integer work; a weight
+// is one IEEE-correctly rounded division, made once per possible count.
 #include "sv_internal.cuh"
 #include <limits.h>
 
@@ -77,7 +79,8 @@ __global__ void k_snn_reverse(const int32_t* __restrict__ G, const int32_t* __re
   }
 }
 
-// candidate totals per column and classification into the three work lists
+// candidate totals per column and classification into the three work lists;
+// lcnt: the lists' lengths, the largest hub, the warp and block columns' candidates
 __global__ void k_snn_classify(const int32_t* __restrict__ G, const int32_t* __restrict__ gcnt,
                                const int64_t* __restrict__ rptr, int64_t n, int k,
                                int32_t* __restrict__ lists, unsigned long long* __restrict__ lcnt,
@@ -90,10 +93,17 @@ __global__ void k_snn_classify(const int32_t* __restrict__ G, const int32_t* __r
       int32_t r = G[j * k + t];
       tot += rptr[r + 1] - rptr[r];
     }
-    int cls = tot <= CAP_WARP ? 0 : (tot <= CAP_BLOCK ? 1 : 2);
-    unsigned long long pos = atomicAdd(&lcnt[cls], 1ull);
+    const int cls = tot <= CAP_WARP ? 0 : (tot <= CAP_BLOCK ? 1 : 2);
+    // one atomic per warp and list
+    const unsigned act = __activemask();
+    const unsigned same = __match_any_sync(act, cls);
+    const int lane = threadIdx.x & 31, lead = __ffs(same) - 1;
+    unsigned long long pos = 0;
+    if (lane == lead) pos = atomicAdd(&lcnt[cls], (unsigned long long)__popc(same));
+    pos = __shfl_sync(same, pos, lead) + __popc(same & ((1u << lane) - 1u));
     lists[(int64_t)cls * n + pos] = (int32_t)j;
     if (cls == 2) atomicMax(maxtot, (unsigned long long)tot);
+    else atomicAdd(&lcnt[4 + (blockIdx.x & 31)], (unsigned long long)tot);
   }
 }
 
@@ -245,48 +255,111 @@ __device__ __forceinline__ void group_prefix(bool flag, int* wsum, const Grp& g,
   __syncthreads();
 }
 
-// Column j counted in a hash table `tab` of 1.5 * (candidates) slots or more:
-// word = (row + 1) << cb | count (cb bits hold any count <= k; 0 = empty).
-// WRITE=false: the kept count; WRITE=true: the kept entries written at `base`
-// in row order.  Same weights and threshold as snn_column.
-template <typename T, bool WRITE, typename Grp>
-__device__ int64_t snn_column_hash(int64_t j, const int32_t* __restrict__ G, const int32_t* __restrict__ gcnt,
-                                   const int64_t* __restrict__ rptr, const int32_t* __restrict__ rlist, int k,
-                                   int kparam, T prune, int cb, uint32_t* tab, int* wsum, const Grp& g,
-                                   int64_t base, int32_t* __restrict__ orow, T* __restrict__ oval,
-                                   int* status) {
-  const int m = gcnt[j];
-  int tot = 0;
-  for (int t = 0; t < m; ++t) {
-    const int32_t r = G[j * k + t];
-    tot += (int)(rptr[r + 1] - rptr[r]);
+// The weights of the counts 0 .. k for column size kk, and whether they are kept
+// (droptol!: |w| > prune): one division per count and block (in FP64 a division
+// per table slot held the FP64 pipe longer than the counting took).
+template <typename T>
+struct WTab {
+  T* w;
+  unsigned char* keep;
+  int kk;
+  T prune;
+  __device__ void build(unsigned char* smem, int k, int kk_, T prune_) {
+    w = (T*)smem;
+    keep = smem + (size_t)(k + 1) * sizeof(T);
+    kk = kk_;
+    prune = prune_;
+    for (int c = threadIdx.x; c <= k; c += blockDim.x) {
+      w[c] = Wt<T>::w(c, kk);
+      keep[c] = w[c] > prune;
+    }
   }
+};
+
+// Column j counted in a hash table `tab` of 1.5 * (candidates) slots or more:
+// word = (row + 1) << cb | count (cb bits hold any count <= k; 0 = empty).  The
+// kept words end up sorted at the front of tab; returns how many.  The reverse
+// lists of 32 neighbours at a time are taken as one sequence, so that every
+// lane has a candidate and its loads do not wait for the previous list's
+// (off: the group's 33 offsets, rp: the lists' starts).
+template <typename T, typename Grp>
+__device__ int snn_column_hash(int64_t j, const int32_t* __restrict__ G, const int32_t* __restrict__ gcnt,
+                               const int64_t* __restrict__ rptr, const int32_t* __restrict__ rlist, int k,
+                               int kparam, const WTab<T>& wt, int cb, uint32_t* tab, int* off, int64_t* rp,
+                               int* wsum, const Grp& g, int* status) {
+  const int m = gcnt[j];
+  const int lane = threadIdx.x & 31;
+  const bool first = g.size() == 32 || threadIdx.x < 32;   // the warp that reads the lists' bounds
+  int tot = 0;
+  if (first) {
+    for (int t = lane; t < m; t += 32) {
+      const int32_t r = G[j * k + t];
+      tot += (int)(rptr[r + 1] - rptr[r]);
+    }
+    tot = sv_warp_sum(tot);
+    if (lane == 0) off[0] = tot;
+  }
+  g.sync();
+  tot = off[0];
   // a multiple of 32, load at most 2/3; never above the table (tot <= CAP)
   const int S = max(32, (3 * tot / 2 + 31) / 32 * 32);
   const uint32_t cmask = (1u << cb) - 1u;
-  for (int i = g.rank(); i < S; i += g.size()) tab[i] = 0u;
-  g.sync();
-  for (int t = 0; t < m; ++t) {
-    const int32_t r = G[j * k + t];
-    const int64_t s0 = rptr[r], e0 = rptr[r + 1];
-    for (int64_t q = s0 + g.rank(); q < e0; q += g.size()) {
-      const uint32_t key = (uint32_t)rlist[q] + 1u;
-      uint32_t h = __umulhi(key * 2654435761u, (uint32_t)S);
-      int probes = 0;
-      while (true) {
-        uint32_t cur = tab[h];
-        if (cur == 0u) {
-          cur = atomicCAS(&tab[h], 0u, (key << cb) | 1u);
-          if (cur == 0u) break;
+  for (int i = g.rank(); i < S / 4; i += g.size()) ((uint4*)tab)[i] = make_uint4(0u, 0u, 0u, 0u);
+  for (int t0 = 0; t0 < m; t0 += 32) {
+    g.sync();
+    if (first) {
+      int len = 0;
+      if (t0 + lane < m) {
+        const int32_t r = G[j * k + t0 + lane];
+        const int64_t s0 = rptr[r];
+        len = (int)(rptr[r + 1] - s0);
+        rp[lane] = s0;
+      }
+      int incl = len;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      off[lane + 1] = incl;
+      if (lane == 0) off[0] = 0;
+    }
+    g.sync();
+    const int nc = off[32];
+    for (int i0 = g.rank(); i0 < nc; i0 += 4 * g.size()) {
+      uint32_t key[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i = i0 + u * g.size();
+        key[u] = 0;
+        if (i < nc) {
+          int lo = 0;
+#pragma unroll
+          for (int b = 16; b > 0; b >>= 1)
+            if (off[lo + b] <= i) lo += b;
+          key[u] = (uint32_t)rlist[rp[lo] + (i - off[lo])] + 1u;
         }
-        if ((cur >> cb) == key) {
-          atomicAdd(&tab[h], 1u);
-          break;
-        }
-        h = h + 1 == (uint32_t)S ? 0u : h + 1;
-        if (++probes >= S) {   // cannot happen with S > candidates
-          sv_flag(status, SV_STATUS_LIMIT);
-          break;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (key[u] == 0) continue;
+        uint32_t h = __umulhi(key[u] * 2654435761u, (uint32_t)S);
+        int probes = 0;
+        while (true) {
+          uint32_t cur = tab[h];
+          if (cur == 0u) {
+            cur = atomicCAS(&tab[h], 0u, (key[u] << cb) | 1u);
+            if (cur == 0u) break;
+          }
+          if ((cur >> cb) == key[u]) {
+            atomicAdd(&tab[h], 1u);
+            break;
+          }
+          h = h + 1 == (uint32_t)S ? 0u : h + 1;
+          if (++probes >= S) {   // cannot happen with S > candidates
+            sv_flag(status, SV_STATUS_LIMIT);
+            break;
+          }
         }
       }
     }
@@ -300,31 +373,112 @@ __device__ int64_t snn_column_hash(int64_t j, const int32_t* __restrict__ G, con
     const int i = c0 + g.rank();
     const uint32_t v = i < S ? tab[i] : 0u;
     bool keep = false;
-    if (v != 0u) keep = Wt<T>::w((int)(v & cmask), kk) > prune;   // droptol!: |w| > prune kept
+    if (v != 0u) {
+      const int c = (int)(v & cmask);
+      keep = kk == wt.kk ? wt.keep[c] != 0 : Wt<T>::w(c, kk) > wt.prune;
+    }
     int before, chunk;
     group_prefix(keep, wsum, g, before, chunk);
-    if (WRITE) {
-      g.sync();   // every read of this chunk before any write
-      if (keep) tab[nk + before] = v;
-    }
+    g.sync();   // every read of this chunk before any write
+    if (keep) tab[nk + before] = v;
     nk += chunk;
-  }
-  if (!WRITE) {
-    g.sync();
-    return nk;
   }
   int n2 = 1;
   while (n2 < nk) n2 <<= 1;
+  g.sync();
   for (int i = nk + g.rank(); i < n2; i += g.size()) tab[i] = 0xFFFFFFFFu;
   g.sync();
   group_bitonic_u32(tab, n2, g);
-  for (int p = g.rank(); p < nk; p += g.size()) {
-    const uint32_t v = tab[p];
-    orow[base + p] = (int32_t)((v >> cb) - 1u);
-    oval[base + p] = Wt<T>::w((int)(v & cmask), kk);
+  return nk;
+}
+
+// the kept words of a column to the arena
+template <typename Grp>
+__device__ void snn_to_arena(int64_t j, int nk, const uint32_t* tab, int* off, const Grp& g,
+                             unsigned long long* __restrict__ used, uint32_t* __restrict__ arena,
+                             int64_t* __restrict__ kept, int64_t* __restrict__ at) {
+  if (g.rank() == 0) {
+    const int64_t o = (int64_t)atomicAdd(used, (unsigned long long)nk);
+    kept[j] = nk;
+    at[j] = o;
+    *(int64_t*)off = o;
   }
   g.sync();
-  return nk;
+  const int64_t o = *(const int64_t*)off;
+  for (int i = g.rank(); i < nk; i += g.size()) arena[o + i] = tab[i];
+  g.sync();
+}
+
+template <typename T>
+__global__ void __launch_bounds__(SNN_BLOCK) k_snn_hash_warp(
+    const int32_t* __restrict__ list, int64_t nlist, const int32_t* __restrict__ G,
+    const int32_t* __restrict__ gcnt, const int64_t* __restrict__ rptr, const int32_t* __restrict__ rlist,
+    int k, int kparam, T prune, int cb, unsigned long long* __restrict__ used, uint32_t* __restrict__ arena,
+    int64_t* __restrict__ kept, int64_t* __restrict__ at, int* status) {
+  extern __shared__ __align__(16) unsigned char snn_dyn[];   // SLOTS_WARP words per warp, then the weights
+  __shared__ __align__(8) int off[SNN_BLOCK / 32][34];
+  __shared__ int64_t rp[SNN_BLOCK / 32][32];
+  const int wid = threadIdx.x >> 5;
+  uint32_t* tab = (uint32_t*)snn_dyn + wid * SLOTS_WARP;
+  WTab<T> wt;
+  wt.build(snn_dyn + (size_t)(SNN_BLOCK / 32) * SLOTS_WARP * 4, k, kparam >= 0 ? kparam : k, prune);
+  __syncthreads();
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  WarpG g;
+  for (int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; t < nlist; t += nwarps) {
+    const int64_t j = list[t];
+    const int nk = snn_column_hash<T>(j, G, gcnt, rptr, rlist, k, kparam, wt, cb, tab, off[wid], rp[wid],
+                                      nullptr, g, status);
+    snn_to_arena(j, nk, tab, off[wid], g, used, arena, kept, at);
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(1024) k_snn_hash_block(
+    const int32_t* __restrict__ list, int64_t nlist, const int32_t* __restrict__ G,
+    const int32_t* __restrict__ gcnt, const int64_t* __restrict__ rptr, const int32_t* __restrict__ rlist,
+    int k, int kparam, T prune, int cb, unsigned long long* __restrict__ used, uint32_t* __restrict__ arena,
+    int64_t* __restrict__ kept, int64_t* __restrict__ at, int* status) {
+  extern __shared__ __align__(16) unsigned char snn_dyn[];   // SLOTS_BLOCK words, then the weights
+  __shared__ __align__(8) int off[34];
+  __shared__ int64_t rp[32];
+  __shared__ int wsum[32];
+  WTab<T> wt;
+  wt.build(snn_dyn + (size_t)SLOTS_BLOCK * 4, k, kparam >= 0 ? kparam : k, prune);
+  BlockG g;
+  for (int64_t t = blockIdx.x; t < nlist; t += gridDim.x) {
+    __syncthreads();
+    const int64_t j = list[t];
+    const int nk = snn_column_hash<T>(j, G, gcnt, rptr, rlist, k, kparam, wt, cb, (uint32_t*)snn_dyn, off, rp,
+                                      wsum, g, status);
+    snn_to_arena(j, nk, (uint32_t*)snn_dyn, off, g, used, arena, kept, at);
+  }
+}
+
+// rows and weights of the columns in the arena, a warp per column
+template <typename T>
+__global__ void __launch_bounds__(256) k_snn_emit(
+    const int32_t* __restrict__ list, int64_t nlist, const int32_t* __restrict__ gcnt, int k, int kparam,
+    T prune, int cb, const uint32_t* __restrict__ arena, const int64_t* __restrict__ at,
+    const int64_t* __restrict__ colptr, int32_t* __restrict__ orow, T* __restrict__ oval) {
+  extern __shared__ __align__(16) unsigned char snn_dyn[];
+  WTab<T> wt;
+  wt.build(snn_dyn, k, kparam >= 0 ? kparam : k, prune);
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const uint32_t cmask = (1u << cb) - 1u;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; t < nlist; t += nwarps) {
+    const int64_t j = list[t];
+    const int64_t o = at[j], b = colptr[j], nk = colptr[j + 1] - b;
+    const int kk = kparam >= 0 ? kparam : gcnt[j];
+    for (int64_t i = lane; i < nk; i += 32) {
+      const uint32_t v = arena[o + i];
+      const int c = (int)(v & cmask);
+      orow[b + i] = (int32_t)((v >> cb) - 1u);
+      oval[b + i] = kk == wt.kk ? wt.w[c] : Wt<T>::w(c, kk);
+    }
+  }
 }
 
 template <typename T, bool WRITE>
@@ -332,21 +486,18 @@ __global__ void __launch_bounds__(SNN_BLOCK) k_snn_warp(
     const int32_t* __restrict__ list, int64_t nlist, const int32_t* __restrict__ G,
     const int32_t* __restrict__ gcnt, const int64_t* __restrict__ rptr,
     const int32_t* __restrict__ rlist, int k, int kparam, T prune, int64_t* __restrict__ kept,
-    const int64_t* __restrict__ colptr, int32_t* __restrict__ orow, T* __restrict__ oval, int cb,
-    int* status) {
-  extern __shared__ int32_t sbuf[];   // SLOTS_WARP words per warp
+    const int64_t* __restrict__ colptr, int32_t* __restrict__ orow, T* __restrict__ oval) {
+  extern __shared__ int32_t sbuf[];   // CAP_WARP words per warp
   int wid = threadIdx.x >> 5;
-  int32_t* buf = sbuf + wid * SLOTS_WARP;
+  int32_t* buf = sbuf + wid * CAP_WARP;
   int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   WarpG g;
   for (int64_t t = warp; t < nlist; t += nwarps) {
     int64_t j = list[t];
     int64_t base = WRITE ? colptr[j] : 0;
-    int64_t c = cb > 0 ? snn_column_hash<T, WRITE>(j, G, gcnt, rptr, rlist, k, kparam, prune, cb,
-                                                   (uint32_t*)buf, nullptr, g, base, orow, oval, status)
-                       : snn_column<T, WRITE>(j, G, gcnt, rptr, rlist, k, kparam, prune, buf, nullptr, g,
-                                              base, orow, oval);
+    int64_t c = snn_column<T, WRITE>(j, G, gcnt, rptr, rlist, k, kparam, prune, buf, nullptr, g, base, orow,
+                                     oval);
     if (!WRITE && g.rank() == 0) kept[j] = c;
   }
 }
@@ -357,7 +508,7 @@ __global__ void __launch_bounds__(1024) k_snn_block(
     const int32_t* __restrict__ gcnt, const int64_t* __restrict__ rptr,
     const int32_t* __restrict__ rlist, int k, int kparam, T prune, int64_t* __restrict__ kept,
     const int64_t* __restrict__ colptr, int32_t* __restrict__ orow, T* __restrict__ oval,
-    int32_t* __restrict__ gscratch, int64_t scratch_per_block, int cb, int* status) {
+    int32_t* __restrict__ gscratch, int64_t scratch_per_block) {
   extern __shared__ int32_t dbuf[];
   __shared__ int wsum[32];
   int32_t* buf = gscratch ? gscratch + blockIdx.x * scratch_per_block : dbuf;
@@ -365,10 +516,8 @@ __global__ void __launch_bounds__(1024) k_snn_block(
   for (int64_t t = blockIdx.x; t < nlist; t += gridDim.x) {
     int64_t j = list[t];
     int64_t base = WRITE ? colptr[j] : 0;
-    int64_t c = cb > 0 ? snn_column_hash<T, WRITE>(j, G, gcnt, rptr, rlist, k, kparam, prune, cb,
-                                                   (uint32_t*)buf, wsum, g, base, orow, oval, status)
-                       : snn_column<T, WRITE>(j, G, gcnt, rptr, rlist, k, kparam, prune, buf, wsum, g,
-                                              base, orow, oval);
+    int64_t c = snn_column<T, WRITE>(j, G, gcnt, rptr, rlist, k, kparam, prune, buf, wsum, g, base, orow,
+                                     oval);
     if (!WRITE && threadIdx.x == 0) kept[j] = c;
     __syncthreads();
   }
@@ -396,15 +545,17 @@ void snn_run(sv_context* ctx, const int32_t* nn, int64_t n, int k, int64_t kpara
   sv_launch(ctx, "snn_reverse", k_snn_reverse, dim3(gridt), dim3(256), 0, (const int32_t*)G.get(),
             (const int32_t*)gcnt.get(), n, k, rc.get(), rlist.get());
   DevBuf<int32_t> lists((size_t)3 * n);
-  DevBuf<unsigned long long> lcnt(4);
-  sv_memset(ctx, lcnt.get(), 0, 32);
+  DevBuf<unsigned long long> lcnt(36);   // three list lengths, largest hub, candidates by block mod 32
+  sv_memset(ctx, lcnt.get(), 0, 36 * 8);
   sv_launch(ctx, "snn_classify", k_snn_classify, dim3(gridt), dim3(256), 0, (const int32_t*)G.get(),
             (const int32_t*)gcnt.get(), (const int64_t*)rptr.get(), n, k, lists.get(), lcnt.get(),
             lcnt.get() + 3);
-  unsigned long long hl[4];
-  sv_d2h(ctx, hl, lcnt.get(), 32);
+  unsigned long long hl[36];
+  sv_d2h(ctx, hl, lcnt.get(), 36 * 8);
   int64_t nl[3] = {(int64_t)hl[0], (int64_t)hl[1], (int64_t)hl[2]};
   int64_t maxtot = (int64_t)hl[3];
+  int64_t cands = 0;
+  for (int b = 0; b < 32; ++b) cands += (int64_t)hl[4 + b];
   int64_t big_n2 = 1;
   while (big_n2 < maxtot) big_n2 <<= 1;
   int big_blocks = (int)std::min<int64_t>(std::max<int64_t>(nl[2], 1), (int64_t)ctx->num_sms);
@@ -415,53 +566,69 @@ void snn_run(sv_context* ctx, const int32_t* nn, int64_t n, int k, int64_t kpara
   // count bits of the hash words: any count <= k; rows + 1 in the remaining bits
   int cb = 32 - __builtin_clz((unsigned)k);
   if ((uint64_t)(n + 1) >= (1ull << (32 - cb))) cb = 0;   // does not fit: the sorting form
-  const size_t warp_smem = (size_t)(SNN_BLOCK / 32) * SLOTS_WARP * 4;
-  const size_t block_smem = (size_t)(cb > 0 ? SLOTS_BLOCK : CAP_BLOCK) * 4;
-  for (auto kern : {k_snn_warp<T, false>, k_snn_warp<T, true>})
-    SV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)warp_smem));
+  // an entry is kept with cmin shared neighbours or more: the arena's bound
+  int cmin = 1;
+  if (kparam >= 0)
+    while (cmin < k && !((T)cmin / ((T)(int)kparam + ((T)(int)kparam - (T)cmin)) > prune)) ++cmin;
+  size_t arena_words = (size_t)(cands / cmin) + 1;
+  if (arena_words * 4 > ctx->pool->keep) cb = 0;
+  const bool hash = cb > 0;
+  DevBuf<uint32_t> arena(hash ? arena_words : 1);
+  DevBuf<int64_t> at(hash ? n : 1);
+  DevBuf<unsigned long long> used(1);
+  const size_t wtab = (size_t)(k + 1) * (sizeof(T) + 1);
+  const int gw = sv_grid_for(ctx, nl[0] * 32, SNN_BLOCK, 4);
+  const int gb = (int)std::min<int64_t>(std::max<int64_t>(nl[1], 1), (int64_t)ctx->num_sms * 2);
+  const int32_t* L0 = lists.get();
+  const int32_t* L1 = lists.get() + n;
+  const int32_t* L2 = lists.get() + 2 * n;
+  const int32_t* Gp = G.get();
+  const int32_t* gc = gcnt.get();
+  const int64_t* rp = rptr.get();
+  const int32_t* rl = rlist.get();
+  const int kp = (int)kparam;
+  if (hash) {
+    const size_t ws = (size_t)(SNN_BLOCK / 32) * SLOTS_WARP * 4 + wtab, bs = (size_t)SLOTS_BLOCK * 4 + wtab;
+    SV_CUDA(cudaFuncSetAttribute(k_snn_hash_warp<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ws));
+    SV_CUDA(cudaFuncSetAttribute(k_snn_hash_block<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bs));
+    sv_memset(ctx, used.get(), 0, 8);
+    sv_launch(ctx, "snn_hash_warp", k_snn_hash_warp<T>, dim3(nl[0] ? gw : 0), dim3(SNN_BLOCK), ws, L0, nl[0],
+              Gp, gc, rp, rl, k, kp, prune, cb, used.get(), arena.get(), kept.get(), at.get(), ctx->d_status);
+    sv_launch(ctx, "snn_hash_block", k_snn_hash_block<T>, dim3(nl[1] ? gb : 0), dim3(1024), bs, L1, nl[1], Gp,
+              gc, rp, rl, k, kp, prune, cb, used.get(), arena.get(), kept.get(), at.get(), ctx->d_status);
+  }
+  const size_t warp_smem = (size_t)(SNN_BLOCK / 32) * CAP_WARP * 4, block_smem = (size_t)CAP_BLOCK * 4;
   for (auto kern : {k_snn_block<T, false>, k_snn_block<T, true>})
     SV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)block_smem));
-  for (int pass = 0; pass < 2; ++pass) {
-    bool W = pass == 1;
+  // the sorting form of pass `W`: every column when nothing is hashed, else the hubs
+  auto sorted = [&](bool W) {
     int32_t* orow = W ? out->rowidx.get() : nullptr;
     T* oval = W ? (T*)out->val.get() : nullptr;
     const int64_t* cp = W ? (const int64_t*)out->colptr.get() : nullptr;
-    int gw = sv_grid_for(ctx, nl[0] * 32, SNN_BLOCK, 4);
-    int gb = (int)std::min<int64_t>(std::max<int64_t>(nl[1], 1), (int64_t)ctx->num_sms * 2);
-    if (W) {
-      sv_launch(ctx, "snn_columns_warp", k_snn_warp<T, true>, dim3(nl[0] ? gw : 0), dim3(SNN_BLOCK),
-                warp_smem, (const int32_t*)lists.get(), nl[0], (const int32_t*)G.get(),
-                (const int32_t*)gcnt.get(), (const int64_t*)rptr.get(), (const int32_t*)rlist.get(), k,
-                (int)kparam, prune, kept.get(), cp, orow, oval, cb, ctx->d_status);
-      sv_launch(ctx, "snn_columns_block", k_snn_block<T, true>, dim3(nl[1] ? gb : 0), dim3(1024),
-                block_smem, (const int32_t*)lists.get() + n, nl[1], (const int32_t*)G.get(),
-                (const int32_t*)gcnt.get(), (const int64_t*)rptr.get(), (const int32_t*)rlist.get(), k,
-                (int)kparam, prune, kept.get(), cp, orow, oval, (int32_t*)nullptr, (int64_t)0, cb,
-                ctx->d_status);
-      sv_launch(ctx, "snn_columns_big", k_snn_block<T, true>, dim3(nl[2] ? big_blocks : 0), dim3(1024),
-                (size_t)0, (const int32_t*)lists.get() + 2 * n, nl[2], (const int32_t*)G.get(),
-                (const int32_t*)gcnt.get(), (const int64_t*)rptr.get(), (const int32_t*)rlist.get(), k,
-                (int)kparam, prune, kept.get(), cp, orow, oval, gscratch.get(), big_n2, 0, ctx->d_status);
-    } else {
-      sv_launch(ctx, "snn_columns_warp", k_snn_warp<T, false>, dim3(nl[0] ? gw : 0), dim3(SNN_BLOCK),
-                warp_smem, (const int32_t*)lists.get(), nl[0], (const int32_t*)G.get(),
-                (const int32_t*)gcnt.get(), (const int64_t*)rptr.get(), (const int32_t*)rlist.get(), k,
-                (int)kparam, prune, kept.get(), cp, orow, oval, cb, ctx->d_status);
-      sv_launch(ctx, "snn_columns_block", k_snn_block<T, false>, dim3(nl[1] ? gb : 0), dim3(1024),
-                block_smem, (const int32_t*)lists.get() + n, nl[1], (const int32_t*)G.get(),
-                (const int32_t*)gcnt.get(), (const int64_t*)rptr.get(), (const int32_t*)rlist.get(), k,
-                (int)kparam, prune, kept.get(), cp, orow, oval, (int32_t*)nullptr, (int64_t)0, cb,
-                ctx->d_status);
-      sv_launch(ctx, "snn_columns_big", k_snn_block<T, false>, dim3(nl[2] ? big_blocks : 0), dim3(1024),
-                (size_t)0, (const int32_t*)lists.get() + 2 * n, nl[2], (const int32_t*)G.get(),
-                (const int32_t*)gcnt.get(), (const int64_t*)rptr.get(), (const int32_t*)rlist.get(), k,
-                (int)kparam, prune, kept.get(), cp, orow, oval, gscratch.get(), big_n2, 0, ctx->d_status);
-      sv_scan_i64(ctx, kept.get(), out->colptr.get(), n);
-      out->nnz = sv_read_i64(ctx, out->colptr.get() + n);
-      out->rowidx.alloc(std::max<int64_t>(1, out->nnz));
-      out->val.alloc(std::max<int64_t>(1, out->nnz) * es);
+    if (!hash) {
+      sv_launch(ctx, "snn_columns_warp", W ? k_snn_warp<T, true> : k_snn_warp<T, false>, dim3(nl[0] ? gw : 0),
+                dim3(SNN_BLOCK), warp_smem, L0, nl[0], Gp, gc, rp, rl, k, kp, prune, kept.get(), cp, orow, oval);
+      sv_launch(ctx, "snn_columns_block", W ? k_snn_block<T, true> : k_snn_block<T, false>,
+                dim3(nl[1] ? gb : 0), dim3(1024), block_smem, L1, nl[1], Gp, gc, rp, rl, k, kp, prune,
+                kept.get(), cp, orow, oval, (int32_t*)nullptr, (int64_t)0);
     }
+    sv_launch(ctx, "snn_columns_big", W ? k_snn_block<T, true> : k_snn_block<T, false>,
+              dim3(nl[2] ? big_blocks : 0), dim3(1024), (size_t)0, L2, nl[2], Gp, gc, rp, rl, k, kp, prune,
+              kept.get(), cp, orow, oval, gscratch.get(), big_n2);
+  };
+  sorted(false);
+  sv_scan_i64(ctx, kept.get(), out->colptr.get(), n);
+  out->nnz = sv_read_i64(ctx, out->colptr.get() + n);
+  out->rowidx.alloc(std::max<int64_t>(1, out->nnz));
+  out->val.alloc(std::max<int64_t>(1, out->nnz) * es);
+  if (hash) {
+    for (int cls = 0; cls < 2; ++cls)
+      sv_launch(ctx, "snn_emit", k_snn_emit<T>, dim3(nl[cls] ? sv_grid_for(ctx, nl[cls] * 32, 256, 8) : 0),
+                dim3(256), wtab, cls ? L1 : L0, nl[cls], gc, k, kp, prune, cb, (const uint32_t*)arena.get(),
+                (const int64_t*)at.get(), (const int64_t*)out->colptr.get(), out->rowidx.get(),
+                (T*)out->val.get());
   }
+  sorted(true);
   sv_sync(ctx);
   sv_check_device_status(ctx, "snn");
 }
