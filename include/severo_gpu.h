@@ -434,6 +434,10 @@ int sv_graph_info(const sv_graph* g, int64_t* n, int64_t* nnz);
  * (nnz) as 1-based Int64, nzval (nnz) in the graph's dtype.  Any may be NULL. */
 int sv_graph_download(sv_context* ctx, const sv_graph* g, int64_t* colptr, int64_t* rowval,
                       void* nzval);
+/* The same as 0-based Int32 pointers and indices (SciPy's CSC; the indices as the
+ * device holds them); SV_ERR_ARG when nnz does not fit.  Any may be NULL. */
+int sv_graph_download_csc32(sv_context* ctx, const sv_graph* g, int32_t* indptr, int32_t* indices,
+                            void* data);
 /* Hand-off to Louvain: the arrays of Network(snn) (src/modularity.jl:163-194)
  * written in Julia's isbits layouts, so that the caller's Vector{Node{T}} and
  * Vector{Edge{T}} receive them without a host rebuild:

@@ -776,6 +776,13 @@ class Graph(_Handle):
     def to_csc(self, dtype):
         n, nnz = C.c_int64(), C.c_int64()
         L.check(self.ctx.lib.sv_graph_info(self.h, C.byref(n), C.byref(nnz)))
+        if nnz.value < 2 ** 31 - 1:
+            # the index type that scipy gives these arrays anyway
+            cp = np.empty(n.value + 1, np.int32)
+            rv = np.empty(nnz.value, np.int32)
+            vv = np.empty(nnz.value, dtype)
+            L.check(self.ctx.lib.sv_graph_download_csc32(self.ctx.h, self.h, _ptr(cp), _ptr(rv), _ptr(vv)))
+            return sp.csc_matrix((vv, rv, cp), shape=(n.value, n.value))
         cp = np.empty(n.value + 1, np.int64)
         rv = np.empty(nnz.value, np.int64)
         vv = np.empty(nnz.value, dtype)

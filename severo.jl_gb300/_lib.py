@@ -119,6 +119,7 @@ SIGNATURES = {
     "sv_snn_knn": (i32, [vp, vp, i64, dbl, i32, P(vp)]),
     "sv_graph_info": (i32, [vp, P(i64), P(i64)]),
     "sv_graph_download": (i32, [vp, vp, vp, vp, vp]),
+    "sv_graph_download_csc32": (i32, [vp, vp, vp, vp, vp]),
     "sv_graph_network": (i32, [vp, vp, P(i64), vp, vp, vp]),
     "sv_graph_free": (i32, [vp]),
     "sv_batch_create": (i32, [vp, vp, vp, i64, vp, i64, C.c_double, P(vp)]),

@@ -656,6 +656,11 @@ __global__ void k_graph_out(const int64_t* __restrict__ cp, const int32_t* __res
   }
 }
 
+__global__ void k_ptr32(const int64_t* __restrict__ p, int64_t n, int32_t* __restrict__ o) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    o[i] = (int32_t)p[i];
+}
+
 void snn_dispatch(sv_context* ctx, const int32_t* nn, int64_t n, int k, int64_t kparam, double prune,
                   int dtype, sv_graph* g) {
   g->ctx = ctx;
@@ -800,6 +805,23 @@ SV_API int sv_graph_download(sv_context* ctx, const sv_graph* g, int64_t* colptr
     if (rowval) sv_d2h(ctx, rowval, ori.get(), g->nnz * 8);
   }
   if (nzval) sv_d2h(ctx, nzval, g->val.get(), g->nnz * sv_elem_size(g->dtype));
+  SV_CATCH
+}
+
+SV_API int sv_graph_download_csc32(sv_context* ctx, const sv_graph* g, int32_t* indptr, int32_t* indices,
+                                   void* data) {
+  SV_TRY
+  sv_ctx_check(ctx);
+  SV_REQUIRE(g && g->ctx == ctx, "bad handle");
+  SV_REQUIRE(g->nnz < (1ll << 31), "nnz exceeds Int32 pointers");
+  if (indptr) {
+    DevBuf<int32_t> p(g->n + 1);
+    sv_launch(ctx, "snn_out", k_ptr32, dim3(sv_grid_for(ctx, g->n + 1, 256, 8)), dim3(256), 0,
+              (const int64_t*)g->colptr.get(), g->n + 1, p.get());
+    sv_d2h(ctx, indptr, p.get(), (g->n + 1) * 4);
+  }
+  if (indices) sv_d2h(ctx, indices, g->rowidx.get(), g->nnz * 4);
+  if (data) sv_d2h(ctx, data, g->val.get(), g->nnz * sv_elem_size(g->dtype));
   SV_CATCH
 }
 
