@@ -4,8 +4,9 @@
 // Stage 1 (candidates): every query scans every point.  The distance key is the
 // GEMM form |p|^2 - 2 q.p (|q|^2 is constant per query); each query keeps its
 // K2 >= 2k smallest keys.  Two implementations:
-//   * FP32 CUDA cores (k_knn_fp32): one query per thread, the point tile staged
-//     in shared memory and broadcast to the block;
+//   * FP32 CUDA cores (k_knn_fp32): 64 queries x 64 points per block and tile;
+//     from KNN_ORDER_MIN points up in the order of sv_knn_order, tiles out of
+//     every query's reach left out;
 //   * BF16 tcgen05 tensor cores with FP32 accumulation in TMEM (sv_knn_tc.cu).
 // Stage 2 (k_rerank): exact FP32 distances sum (q_c - p_c)^2 of the K2
 // candidates, sorted by (distance, index); the point itself first when
@@ -14,6 +15,7 @@
 // Layout in HBM: points row-major FP32 [n][dp] (dp = d rounded up to 8, zero
 // padded) plus FP32 squared norms; candidates [n][K2]; results [n][k] (0-based).
 #include "sv_internal.cuh"
+#include "sv_knn_order.cuh"
 #include <float.h>
 
 int sv_knn_tc_candidates(sv_context* ctx, const float* X32, const float* sq, int64_t n, int dp, int d,
@@ -23,8 +25,10 @@ sv_context* sv_default_context();
 
 namespace {
 
-constexpr int KNN_THREADS = 128;
-constexpr int KNN_TILE = 64;
+constexpr int KNN_THREADS = 256;
+constexpr int KNN_TILE = 64;       // points per tile and queries per block
+constexpr int KNN_LIST = 64;       // most candidates of a query
+constexpr int64_t KNN_ORDER_MIN = 2048;
 
 // X (n x d, column-major, leading dim ld, FP32 or FP64) -> row-major FP32 [n][dp]
 // (optionally unit-normalised rows for the cosine metric) and squared norms.
@@ -52,96 +56,261 @@ __global__ void k_pack_rows(const T* __restrict__ X, int64_t ld, int64_t n, int 
   }
 }
 
-template <int DP, int K2>
-__global__ void __launch_bounds__(KNN_THREADS) k_knn_fp32(const float* __restrict__ X,
-                                                          const float* __restrict__ sq, int64_t n,
-                                                          int include_self,
-                                                          int32_t* __restrict__ cand) {
-  __shared__ __align__(16) float tile[KNN_TILE * DP];
-  __shared__ float tsq[KNN_TILE];
-  __shared__ float kslot[KNN_THREADS][9];
-  int64_t qi = (int64_t)blockIdx.x * KNN_THREADS + threadIdx.x;
-  bool active = qi < n;
-  float q[DP];
-#pragma unroll
-  for (int c = 0; c < DP; c += 4) {
-    float4 v = active ? *(const float4*)(X + qi * DP + c) : make_float4(0, 0, 0, 0);
-    q[c] = -2.f * v.x;
-    q[c + 1] = -2.f * v.y;
-    q[c + 2] = -2.f * v.z;
-    q[c + 3] = -2.f * v.w;
-  }
-  float best[K2];
-  int bidx[K2];
-#pragma unroll
-  for (int t = 0; t < K2; ++t) {
-    best[t] = FLT_MAX;
-    bidx[t] = -1;
-  }
-  if (include_self && active) {
-    best[0] = -FLT_MAX;
-    bidx[0] = (int)qi;
-  }
-  for (int64_t p0 = 0; p0 < n; p0 += KNN_TILE) {
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < KNN_TILE * DP / 4; idx += KNN_THREADS) {
-      int r = idx / (DP / 4);
-      int64_t p = p0 + r;
-      float4 v = p < n ? *(const float4*)(X + p * DP + (idx % (DP / 4)) * 4) : make_float4(0, 0, 0, 0);
-      *(float4*)(tile + idx * 4) = v;
+// ---- FP32 candidates -----------------------------------------------------------
+// Points tile by tile, dimension-major within a tile (Xt[tile][c][64], zero rows
+// past the end) with their norms (FLT_MAX past the end) and original indices; the
+// largest norm (float bits) for the pruning margin.
+__global__ void k_tiles_fp32(const float* __restrict__ X, const float* __restrict__ sq, const int* __restrict__ perm,
+                             int64_t n, int dp, int64_t npad, float* __restrict__ Xt, float* __restrict__ sqt,
+                             int* __restrict__ orig, unsigned* __restrict__ pmax) {
+  const int q4 = dp / 4;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < npad * q4;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    // 64 consecutive threads: the rows of one tile, the same four dimensions
+    const int64_t t = e / (KNN_TILE * q4);
+    const int r = (int)(e % KNN_TILE), c4 = (int)(e / KNN_TILE % q4);
+    const int64_t i = t * KNN_TILE + r, src = i < n ? (perm ? perm[i] : i) : 0;
+    const float4 v = i < n ? ((const float4*)X)[src * q4 + c4] : make_float4(0, 0, 0, 0);
+    float* o = Xt + t * KNN_TILE * dp + (int64_t)c4 * 4 * KNN_TILE + r;
+    o[0] = v.x;
+    o[KNN_TILE] = v.y;
+    o[2 * KNN_TILE] = v.z;
+    o[3 * KNN_TILE] = v.w;
+    if (c4 == 0) {
+      const float s = i < n ? sq[src] : FLT_MAX;
+      sqt[i] = s;
+      orig[i] = i < n ? (int)src : -1;
+      if (i < n) atomicMax(pmax, __float_as_uint(s));
     }
-    for (int r = threadIdx.x; r < KNN_TILE; r += KNN_THREADS) tsq[r] = p0 + r < n ? sq[p0 + r] : FLT_MAX;
-    __syncthreads();
-    // 8 candidates at a time: 8 independent FMA chains; padded rows have key FLT_MAX
-#pragma unroll 1
-    for (int r0 = 0; r0 < KNN_TILE; r0 += 8) {
-      float acc[8];
+  }
+}
+
+__device__ __forceinline__ unsigned key_bits(float v) {
+  const unsigned u = __float_as_uint(v);
+  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float key_float(unsigned b) {
+  return __uint_as_float((b & 0x80000000u) ? (b & 0x7fffffffu) : ~b);
+}
+
+// 64 values over a warp, element lane + 32 r in v[r]: the compare-exchange of
+// element e with e ^ stride, ascending where (e & dir) == 0
+__device__ __forceinline__ void w64_step(unsigned long long (&v)[2], int stride, int dir) {
+  const int lane = threadIdx.x & 31;
+  if (stride == 32) {
+    const bool up = (lane & dir) == 0;
+    if ((v[0] > v[1]) == up) {
+      const unsigned long long t = v[0];
+      v[0] = v[1];
+      v[1] = t;
+    }
+    return;
+  }
 #pragma unroll
-      for (int u = 0; u < 8; ++u) acc[u] = tsq[r0 + u];
+  for (int r = 0; r < 2; ++r) {
+    const unsigned long long o = __shfl_xor_sync(0xffffffffu, v[r], stride);
+    const bool up = ((lane + 32 * r) & dir) == 0, low = (lane & stride) == 0;
+    if ((low == up) ? o < v[r] : o > v[r]) v[r] = o;
+  }
+}
+
+// The K2 smallest keys |p|^2 - 2 q.p of every query, equal keys by index.  Block of
+// 64 queries; per tile of 64 points a thread forms a 4 x 4 patch of keys (two
+// 16-byte shared loads per 16 FMAs; each key one chain over the dimensions), and
+// keys that pass their query's threshold are appended to the query's buffer in
+// shared memory.  A buffer above half full is merged into the query's sorted list
+// by a warp (bitonic sort and merge of 64 packed (key, index) words), which
+// lowers the threshold; keys that found a full buffer try again after that.  With
+// a list of the tiles by their lower bound (sv_knn_order) the scan ends at the
+// first tile beyond every query's threshold + |q|^2 + a margin for the keys' FP32
+// rounding (2^-15 (|q|^2 + max |p|^2), several times its bound).
+// 30,011 points in 50 dimensions, 40 candidates: 1.5 ms (2.4 ms with the boxes'
+// bound alone); a query per thread with 64 candidates in registers over every
+// tile, 235 blocks of four warps, took 7.5 ms.
+template <int DP>
+__global__ void __launch_bounds__(KNN_THREADS, 2) k_knn_fp32(
+    const float* __restrict__ Xt, const float* __restrict__ sqt, const int* __restrict__ orig, int64_t n,
+    int K2, int32_t* __restrict__ cand, const unsigned long long* __restrict__ lists,
+    const unsigned* __restrict__ pmax) {
+  extern __shared__ __align__(16) unsigned char knn_dyn[];
+  float* Q = (float*)knn_dyn;                       // [DP][64], times -2
+  float* Pt = Q + DP * KNN_TILE;                    // [DP][64]
+  unsigned long long* ent = (unsigned long long*)(Pt + DP * KNN_TILE);   // [query][list 64, buffer 64]
+  __shared__ __align__(16) float thr[KNN_TILE], psq[KNN_TILE];
+  __shared__ unsigned long long thr64[KNN_TILE];
+  __shared__ int cnt[KNN_TILE], pid[KNN_TILE];
+  __shared__ float bound[KNN_TILE], wm[KNN_THREADS / 32];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, tx = tid & 15, ty = tid >> 4;
+  const int64_t ntiles = (n + KNN_TILE - 1) / KNN_TILE;
+  const int own = blockIdx.x;
+  const unsigned long long* list = lists ? lists + (int64_t)blockIdx.x * ntiles : nullptr;
+  constexpr int NV = (DP * KNN_TILE / 4 + KNN_THREADS - 1) / KNN_THREADS;   // float4 per thread and tile
+  float4 pre[NV];
+  auto fetch = [&](int64_t t) {
+    const float4* src = (const float4*)(Xt + t * KNN_TILE * DP);
 #pragma unroll
-      for (int c = 0; c < DP; c += 4) {
+    for (int u = 0; u < NV; ++u)
+      if (tid + u * KNN_THREADS < DP * KNN_TILE / 4) pre[u] = src[tid + u * KNN_THREADS];
+  };
+  fetch(own);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          float4 v = ((const float4*)(tile + (r0 + u) * DP))[c / 4];
-          acc[u] = fmaf(q[c], v.x, acc[u]);
-          acc[u] = fmaf(q[c + 1], v.y, acc[u]);
-          acc[u] = fmaf(q[c + 2], v.z, acc[u]);
-          acc[u] = fmaf(q[c + 3], v.w, acc[u]);
-        }
+  for (int u = 0; u < NV; ++u)
+    if (tid + u * KNN_THREADS < DP * KNN_TILE / 4)
+      ((float4*)Q)[tid + u * KNN_THREADS] =
+          make_float4(-2.f * pre[u].x, -2.f * pre[u].y, -2.f * pre[u].z, -2.f * pre[u].w);
+  for (int k = tid; k < KNN_TILE * 2 * KNN_LIST; k += KNN_THREADS) ent[k] = ~0ull;
+  if (tid < KNN_TILE) {
+    thr[tid] = FLT_MAX;
+    thr64[tid] = (unsigned long long)key_bits(FLT_MAX) << 32;
+    cnt[tid] = 0;
+    const bool in = own * (int64_t)KNN_TILE + tid < n;
+    bound[tid] = in ? __int_as_float(0x7f800000) : -FLT_MAX;
+  }
+  if (tid < KNN_THREADS / 32) wm[tid] = __int_as_float(0x7f800000);
+  unsigned long long e0 = list ? list[0] : 0;
+  int64_t t = list ? knn_list_tile(e0, own) : 0;
+  if (t != own) fetch(t);
+  // merges a query's buffer into its list (a warp)
+  auto merge = [&](int q) {
+    unsigned long long* L = ent + (size_t)q * 2 * KNN_LIST;
+    const int m = min(cnt[q], KNN_LIST);
+    unsigned long long b[2], a[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      a[r] = L[lane + 32 * r];
+      b[r] = lane + 32 * r < m ? L[KNN_LIST + lane + 32 * r] : ~0ull;
+    }
+#pragma unroll
+    for (int k = 2; k <= 64; k <<= 1)
+#pragma unroll
+      for (int s = k >> 1; s > 0; s >>= 1) w64_step(b, s, k);
+    // the 64 smallest of two ascending sequences: min(a[e], b[63 - e]), bitonic
+    const unsigned long long r0 = __shfl_sync(0xffffffffu, b[1], 31 - lane);
+    const unsigned long long r1 = __shfl_sync(0xffffffffu, b[0], 31 - lane);
+    a[0] = a[0] < r0 ? a[0] : r0;
+    a[1] = a[1] < r1 ? a[1] : r1;
+#pragma unroll
+    for (int s = 32; s > 0; s >>= 1) w64_step(a, s, 64);
+    L[lane] = a[0];
+    L[lane + 32] = a[1];
+    const unsigned long long last = K2 > 32 ? a[1] : a[0];
+    if (lane == ((K2 - 1) & 31)) {
+      if (last != ~0ull) {
+        thr[q] = key_float((unsigned)(last >> 32));
+        thr64[q] = last;
       }
-      float thr = best[K2 - 1];
-      uint32_t m = 0;
+      cnt[q] = 0;
+      const int64_t qi = own * (int64_t)KNN_TILE + q;
+      if (last != ~0ull && qi < n) {
+        const float v = thr[q] + sqt[qi] + 0x1p-15f * (sqt[qi] + __uint_as_float(*pmax));
+        bound[q] = v != v ? __int_as_float(0x7f800000) : v;   // no bound from a NaN
+      }
+    }
+    __syncwarp();
+  };
+  for (int64_t it = 0; it < ntiles; ++it) {
+    __syncthreads();                                // the previous tile is done with Pt
+    if (list && it > 0) {
+      float T = wm[0];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) m |= (acc[u] < thr ? 1u : 0u) << u;
-      if (m) {
-        float* slot = kslot[threadIdx.x];
+      for (int u = 1; u < KNN_THREADS / 32; ++u) T = fmaxf(T, wm[u]);
+      if (knn_list_bound(e0) > T) break;
+    }
 #pragma unroll
-        for (int u = 0; u < 8; ++u) slot[u] = acc[u];
-        while (m) {
-          int u = __ffs(m) - 1;
-          m &= m - 1;
-          int pid = (int)(p0 + r0 + u);
-          float cd = slot[u];
-          if (pid == qi || !(cd < best[K2 - 1])) continue;
-          int ci = pid;
+    for (int u = 0; u < NV; ++u)
+      if (tid + u * KNN_THREADS < DP * KNN_TILE / 4) ((float4*)Pt)[tid + u * KNN_THREADS] = pre[u];
+    if (tid < KNN_TILE) {
+      psq[tid] = sqt[t * KNN_TILE + tid];
+      pid[tid] = orig[t * KNN_TILE + tid];
+    }
+    const int64_t tc = t;
+    if (it + 1 < ntiles) {
+      e0 = list ? list[it + 1] : 0;
+      t = list ? knn_list_tile(e0, own) : it + 1;
+      fetch(t);
+    }
+    __syncthreads();
+    float acc[4][4];
+    {
+      const float4 v = *(const float4*)(psq + 4 * tx);
 #pragma unroll
-          for (int t = 0; t < K2; ++t) {
-            if (cd < best[t]) {
-              float td = best[t];
-              int ti = bidx[t];
-              best[t] = cd;
-              bidx[t] = ci;
-              cd = td;
-              ci = ti;
+      for (int i = 0; i < 4; ++i) {
+        acc[i][0] = v.x;
+        acc[i][1] = v.y;
+        acc[i][2] = v.z;
+        acc[i][3] = v.w;
+      }
+    }
+#pragma unroll 8
+    for (int c = 0; c < DP; ++c) {
+      const float4 qv = *(const float4*)(Q + c * KNN_TILE + 4 * ty);
+      const float4 pv = *(const float4*)(Pt + c * KNN_TILE + 4 * tx);
+      const float qa[4] = {qv.x, qv.y, qv.z, qv.w}, pa[4] = {pv.x, pv.y, pv.z, pv.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc[i][u] = fmaf(qa[i], pa[u], acc[i][u]);
+    }
+    unsigned todo = 0;
+    {
+      const float4 tv = *(const float4*)(thr + 4 * ty);
+      const float ta[4] = {tv.x, tv.y, tv.z, tv.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (acc[i][u] <= ta[i] && pid[4 * tx + u] >= 0 && !(tc == own && 4 * ty + i == 4 * tx + u))
+            todo |= 1u << (4 * i + u);
+    }
+    while (true) {
+      if (todo) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            if (todo & (1u << (4 * i + u))) {
+              const int q = 4 * ty + i;
+              const unsigned long long e =
+                  ((unsigned long long)key_bits(acc[i][u]) << 32) | (unsigned)pid[4 * tx + u];
+              if (e < thr64[q]) {
+                const int pos = atomicAdd(&cnt[q], 1);
+                if (pos < KNN_LIST) {
+                  ent[(size_t)q * 2 * KNN_LIST + KNN_LIST + pos] = e;
+                  todo &= ~(1u << (4 * i + u));
+                }
+              } else {
+                todo &= ~(1u << (4 * i + u));
+              }
             }
           }
         }
       }
+      const int again = __syncthreads_or(todo != 0);
+      bool did = false;
+      for (int q = w; q < KNN_TILE; q += KNN_THREADS / 32)
+        if (cnt[q] > KNN_LIST / 2) {
+          merge(q);
+          did = true;
+        }
+      if (did) {
+        float v = lane < KNN_TILE / (KNN_THREADS / 32) ? bound[w + lane * (KNN_THREADS / 32)] : -FLT_MAX;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+        if (lane == 0) wm[w] = v;
+      }
+      if (!again) break;
+      __syncthreads();
     }
   }
-  if (active) {
-#pragma unroll
-    for (int t = 0; t < K2; ++t) cand[qi * K2 + t] = bidx[t];
+  __syncthreads();
+  for (int q = w; q < KNN_TILE; q += KNN_THREADS / 32) {
+    const int64_t qi = own * (int64_t)KNN_TILE + q;
+    if (qi >= n) break;
+    if (cnt[q] > 0) merge(q);
+    __syncwarp();
+    const unsigned long long* L = ent + (size_t)q * 2 * KNN_LIST;
+    int32_t* o = cand + (int64_t)orig[qi] * K2;
+    for (int k = lane; k < K2; k += 32) o[k] = L[k] == ~0ull ? -1 : (int32_t)(unsigned)L[k];
   }
 }
 
@@ -217,13 +386,23 @@ __global__ void k_rerank(const float* __restrict__ X, int64_t n, const int32_t* 
 }
 
 template <int DP>
-void launch_fp32(sv_context* ctx, const float* X, const float* sq, int64_t n, int K2, int inc,
-                 int32_t* cand) {
-  dim3 grid((unsigned)((n + KNN_THREADS - 1) / KNN_THREADS));
-  if (K2 == 32)
-    sv_launch(ctx, "knn_fp32_tiles", k_knn_fp32<DP, 32>, grid, dim3(KNN_THREADS), 0, X, sq, n, inc, cand);
-  else
-    sv_launch(ctx, "knn_fp32_tiles", k_knn_fp32<DP, 64>, grid, dim3(KNN_THREADS), 0, X, sq, n, inc, cand);
+void launch_fp32(sv_context* ctx, const float* X, const float* sq, int64_t n, int d, int K2, int32_t* cand) {
+  const int64_t ntiles = (n + KNN_TILE - 1) / KNN_TILE, npad = ntiles * KNN_TILE;
+  KnnOrder ord;
+  const bool listed = n >= KNN_ORDER_MIN && sv_knn_order(ctx, X, n, DP, d, KNN_TILE, KNN_TILE, ord);
+  DevBuf<float> Xt((size_t)npad * DP), sqt(npad);
+  DevBuf<int> orig(npad);
+  DevBuf<unsigned> pmax(1);
+  sv_memset(ctx, pmax.get(), 0, 4);
+  sv_launch(ctx, "knn_tiles_layout", k_tiles_fp32, dim3(sv_grid_for(ctx, npad * DP / 4, 256, 8)), dim3(256), 0, X, sq,
+            listed ? (const int*)ord.perm.get() : (const int*)nullptr, n, DP, npad, Xt.get(), sqt.get(), orig.get(),
+            pmax.get());
+  const size_t smem = (size_t)2 * DP * KNN_TILE * 4 + (size_t)KNN_TILE * 2 * KNN_LIST * 8;
+  SV_CUDA(cudaFuncSetAttribute(k_knn_fp32<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  sv_launch(ctx, "knn_fp32_tiles", k_knn_fp32<DP>, dim3((unsigned)ntiles), dim3(KNN_THREADS), smem,
+            (const float*)Xt.get(), (const float*)sqt.get(), (const int*)orig.get(), n, K2, cand,
+            listed ? (const unsigned long long*)ord.lists.get() : (const unsigned long long*)nullptr,
+            (const unsigned*)pmax.get());
 }
 
 template <int DP>
@@ -263,10 +442,9 @@ __global__ void k_to_host_layout(const int32_t* __restrict__ idx, const float* _
 static void knn_core(sv_context* ctx, const float* X32, const float* sq, int64_t n, int dp, int d, int k,
                      int include_self, int cosine, int precision, sv_knn* out,
                      const std::vector<int64_t>* segs = nullptr) {
-  // candidates per query: at least 2k; the tensor-core stage always keeps 64
-  // candidates per query: 32 or 64 from the FP32 tiles, 40 (k <= 20) or 64 from
-  // the tensor-core tiles
-  int K2 = precision == SV_KNN_BF16 ? (2 * k <= 40 ? 40 : 64) : (2 * k <= 32 ? 32 : 64);
+  // candidates per query: at least 2k; a multiple of 8 from the FP32 tiles, 40 (k <=
+  // 20) or 64 from the tensor-core tiles
+  int K2 = precision == SV_KNN_BF16 ? (2 * k <= 40 ? 40 : 64) : std::max(16, (2 * k + 7) / 8 * 8);
   if (2 * k > 64) sv_throw(SV_ERR_UNSUPPORTED, "k = %d exceeds the supported maximum of 32", k);
   DevBuf<int32_t> cand((size_t)n * K2);
   bool done = false;
@@ -286,14 +464,14 @@ static void knn_core(sv_context* ctx, const float* X32, const float* sq, int64_t
       const float* qs = sq + o;
       int32_t* cs = cand.get() + o * K2;
       switch (dp) {
-        case 8: launch_fp32<8>(ctx, Xs, qs, ns, K2, include_self, cs); break;
-        case 16: launch_fp32<16>(ctx, Xs, qs, ns, K2, include_self, cs); break;
-        case 24: launch_fp32<24>(ctx, Xs, qs, ns, K2, include_self, cs); break;
-        case 32: launch_fp32<32>(ctx, Xs, qs, ns, K2, include_self, cs); break;
-        case 40: launch_fp32<40>(ctx, Xs, qs, ns, K2, include_self, cs); break;
-        case 48: launch_fp32<48>(ctx, Xs, qs, ns, K2, include_self, cs); break;
-        case 56: launch_fp32<56>(ctx, Xs, qs, ns, K2, include_self, cs); break;
-        case 64: launch_fp32<64>(ctx, Xs, qs, ns, K2, include_self, cs); break;
+        case 8: launch_fp32<8>(ctx, Xs, qs, ns, d, K2, cs); break;
+        case 16: launch_fp32<16>(ctx, Xs, qs, ns, d, K2, cs); break;
+        case 24: launch_fp32<24>(ctx, Xs, qs, ns, d, K2, cs); break;
+        case 32: launch_fp32<32>(ctx, Xs, qs, ns, d, K2, cs); break;
+        case 40: launch_fp32<40>(ctx, Xs, qs, ns, d, K2, cs); break;
+        case 48: launch_fp32<48>(ctx, Xs, qs, ns, d, K2, cs); break;
+        case 56: launch_fp32<56>(ctx, Xs, qs, ns, d, K2, cs); break;
+        case 64: launch_fp32<64>(ctx, Xs, qs, ns, d, K2, cs); break;
         default: sv_throw(SV_ERR_UNSUPPORTED, "padded dimension %d", dp);
       }
       if (o > 0)

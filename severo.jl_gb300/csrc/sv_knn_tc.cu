@@ -17,6 +17,7 @@
 // an error, drains its own outstanding copies and MMAs (bounded as well),
 // releases its tensor memory and returns.
 #include "sv_internal.cuh"
+#include "sv_knn_order.cuh"
 #include "sv_tc.cuh"
 #include <cuda.h>
 #include <float.h>
@@ -550,32 +551,6 @@ __global__ void k_pack_fold(const float* __restrict__ X, int64_t n, int dp, int 
 }
 
 // ---- locality order of the points ----------------------------------------------
-// Per-dimension sums and sums of squares (FP64, atomics: only the choice of the
-// widest dimension depends on them).
-__global__ void k_dim_moments(const float* __restrict__ X, int64_t n, int dp, double* __restrict__ acc) {
-  __shared__ double s1[256], s2[256];
-  const int c = threadIdx.x % dp, r0 = threadIdx.x / dp, rstep = blockDim.x / dp;
-  double a = 0, b = 0;
-  if (r0 < rstep)
-    for (int64_t i = blockIdx.x * (int64_t)rstep + r0; i < n; i += (int64_t)gridDim.x * rstep) {
-      double v = X[i * dp + c];
-      a += v;
-      b += v * v;
-    }
-  s1[threadIdx.x] = a;
-  s2[threadIdx.x] = b;
-  __syncthreads();
-  if (threadIdx.x < dp) {
-    double ta = 0, tb = 0;
-    for (int r = 0; r < rstep; ++r) {
-      ta += s1[r * dp + threadIdx.x];
-      tb += s2[r * dp + threadIdx.x];
-    }
-    atomicAdd(acc + threadIdx.x, ta);
-    atomicAdd(acc + dp + threadIdx.x, tb);
-  }
-}
-
 // sort key: sample in the high word, the coordinate (order-preserving bits) low
 __global__ void k_locality_keys(const float* __restrict__ X, int dp, int dim, const int64_t* __restrict__ off,
                                 int nseg, int64_t n, unsigned long long* __restrict__ key, int* __restrict__ val) {
@@ -626,20 +601,7 @@ int sv_knn_tc_candidates(sv_context* ctx, const float* X32, const float* sq_unus
     int dim = 0;
     if (around) {
       int nseg = segs ? (int)segs->size() - 1 : 1;
-      DevBuf<double> mom(2 * dp);
-      sv_memset(ctx, mom.get(), 0, 2 * dp * 8);
-      sv_launch(ctx, "knn_order", k_dim_moments, dim3(sv_grid_for(ctx, n, 256, 2)), dim3(256 / dp * dp), 0,
-                X32, n, dp, mom.get());
-      std::vector<double> hm(2 * dp);
-      sv_d2h(ctx, hm.data(), mom.get(), 2 * dp * 8);
-      double best = -1;
-      for (int c = 0; c < d; ++c) {
-        double mean = hm[c] / (double)n, var = hm[dp + c] / (double)n - mean * mean;
-        if (var > best) {
-          best = var;
-          dim = c;
-        }
-      }
+      dim = sv_knn_widest_dim(ctx, X32, n, dp, d);
       int64_t n2 = 2048;
       while (n2 < n) n2 <<= 1;
       DevBuf<unsigned long long> key(n2);
