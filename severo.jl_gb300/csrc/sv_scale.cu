@@ -338,16 +338,30 @@ __global__ void k_hsub_write(const int64_t* __restrict__ rowptr, const int32_t* 
   for (int64_t r = warp; r < n_rows; r += nwarps) {
     int64_t s = rowptr[r], e = rowptr[r + 1];
     int64_t pos = hrowptr[r];
-    for (int64_t i0 = s; i0 < e; i0 += 32) {
-      int64_t i = i0 + lane;
-      int32_t f = i < e ? __ldg(gene_map + col[i]) : -1;
-      unsigned m = __ballot_sync(0xffffffffu, f >= 0);
-      if (f >= 0) {
-        int64_t p = pos + __popc(m & ((1u << lane) - 1));
-        hcol[p] = (IdxT)f;
-        hval[p] = val[i];
+    // four groups of 32 entries in flight (one: 1.23 ms for 250 M entries of
+    // 100,000 cells, four: 0.66 ms)
+    for (int64_t i0 = s; i0 < e; i0 += 128) {
+      int32_t f[4];
+      ValT v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int64_t i = i0 + 32 * u + lane;
+        f[u] = i < e ? col[i] : -1;
+        if (i < e) v[u] = val[i];
       }
-      pos += __popc(m);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (f[u] >= 0) f[u] = __ldg(gene_map + f[u]);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const unsigned m = __ballot_sync(0xffffffffu, f[u] >= 0);
+        if (f[u] >= 0) {
+          const int64_t p = pos + __popc(m & ((1u << lane) - 1));
+          hcol[p] = (IdxT)f[u];
+          hval[p] = v[u];
+        }
+        pos += __popc(m);
+      }
     }
   }
 }
@@ -1027,8 +1041,14 @@ __global__ void k_rb_count(const int64_t* __restrict__ fstart, const int64_t* __
     const int64_t s = fstart[f], e = fend[f];
     const int64_t lo = lower_bound_rows(rowidx, s, e, rb_first_row(row0, b));
     const int64_t hi = lower_bound_rows(rowidx, lo, e, rb_first_row(row0, b + 1));
-    int64_t pads = 0;
-    for (int64_t t = lo + 1 + lane; t < hi; t += 32) pads += rb_pads((int64_t)rowidx[t] - rowidx[t - 1]);
+    int pads = 0;
+    for (int64_t t = lo + 1 + lane; t < hi; t += 128) {
+      int step[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) step[u] = t + 32 * u < hi ? rowidx[t + 32 * u] - rowidx[t + 32 * u - 1] : 0;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) pads += rb_pads(step[u]);
+    }
     pads = sv_warp_sum(pads);
     if (lane == 0) {
       const int64_t n = hi - lo + pads;
@@ -1038,64 +1058,111 @@ __global__ void k_rb_count(const int64_t* __restrict__ fstart, const int64_t* __
   }
 }
 
-// one warp per (row block, feature): the coded rows (ocode zeroed beforehand,
-// bit fields or-ed in) and the values, padding included
+// One warp per (row block, feature): the coded rows and the values, padding
+// included.  Entries and padding pass through a ring of RC_RING places per warp in
+// shared memory; whenever it holds 256, each lane codes one group of 8 and writes
+// its word and values at once (a 64-bit atomic or per entry and scalar value
+// stores took 1.77 ms for 117 M FP32 entries of 100,000 cells, this 1.08 ms).
+constexpr int RC_RING = 512;
+constexpr int RC_WARPS = 8;
 template <typename ValT>
-__global__ void k_rb_copy(const int64_t* __restrict__ src, const int64_t* __restrict__ dst,
-                          const int64_t* __restrict__ fend, const int32_t* __restrict__ rowidx,
-                          const ValT* __restrict__ val, int64_t npairs, int64_t nf,
-                          unsigned long long* __restrict__ ocode, ValT* __restrict__ oval,
-                          const int64_t* __restrict__ row0) {
-  const int lane = threadIdx.x & 31;
+__global__ void __launch_bounds__(RC_WARPS * 32) k_rb_copy(
+    const int64_t* __restrict__ src, const int64_t* __restrict__ dst, const int64_t* __restrict__ fend,
+    const int32_t* __restrict__ rowidx, const ValT* __restrict__ val, int64_t npairs, int64_t nf,
+    unsigned long long* __restrict__ ocode, ValT* __restrict__ oval, const int64_t* __restrict__ row0) {
+  __shared__ __align__(16) uint16_t ring_r[RC_WARPS][RC_RING];
+  __shared__ __align__(16) ValT ring_v[RC_WARPS][RC_RING];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint16_t* rr = ring_r[w];
+  ValT* rv = ring_v[w];
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t p = warp; p < npairs; p += nwarps) {
     const int64_t b = p / nf;
-    const int64_t first = rb_first_row(row0, b);
-    const int64_t s = src[p], d = dst[p], dend = dst[p + 1];
+    const int first = (int)rb_first_row(row0, b);
+    const int64_t s = src[p], d = dst[p];
     const int64_t hi = lower_bound_rows(rowidx, s, fend[p % nf], rb_first_row(row0, b + 1));
-    // entry q (from d) at row r; the previous entry at row rp
-    auto put = [&](int64_t q, int64_t r, int64_t rp, ValT v) {
-      const int64_t rel = q - d;
-      const int slot = (int)(rel % RB_GROUP);
-      const unsigned long long field =
-          slot == 0 ? (unsigned long long)r : (unsigned long long)(r - rp) << (16 + 6 * (slot - 1));
-      if (field) atomicOr(&ocode[q / RB_GROUP], field);
-      oval[q] = v;
-    };
-    int64_t o = d;
-    int64_t last_row = 0;
-    for (int64_t t0 = s; t0 < hi; t0 += 32) {
-      const int64_t t = t0 + lane;
-      int64_t r = 0, rp = 0;
-      int k = 0;
-      if (t < hi) {
-        r = (int64_t)rowidx[t] - first;
-        rp = t > s ? (int64_t)rowidx[t - 1] - first : r;
-        k = t > s ? rb_pads(r - rp) : 0;
-      }
-      int incl = t < hi ? k + 1 : 0;
+    int64_t word = d / RB_GROUP;   // the next word to write
+    int head = 0, cur = 0;         // ring: cur places from head
+    // writes the first `words` groups of the ring
+    auto flush = [&](int words) {
+      __syncwarp();
+      if (lane < words) {
+        const int at = (head + RB_GROUP * lane) & (RC_RING - 1);
+        const uint4 r4 = *(const uint4*)(rr + at);
+        const unsigned q[4] = {r4.x, r4.y, r4.z, r4.w};
+        int prev = (int)(q[0] & 0xffffu);
+        unsigned long long code = (unsigned long long)prev;
 #pragma unroll
-      for (int sh = 1; sh < 32; sh <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, incl, sh);
-        if (lane >= sh) incl += y;
-      }
-      const int tot = __shfl_sync(0xffffffffu, incl, 31);
-      if (t < hi) {
-        int64_t q = o + incl - (k + 1);
-        int64_t prev = rp;
-        for (int u = 1; u <= k; ++u, ++q) {
-          put(q, rp + 63 * u, prev, ValT(0.f));
-          prev = rp + 63 * u;
+        for (int t = 1; t < RB_GROUP; ++t) {
+          const int r = (int)((t & 1) ? q[t >> 1] >> 16 : q[t >> 1] & 0xffffu);
+          code |= (unsigned long long)(r - prev) << (16 + 6 * (t - 1));
+          prev = r;
         }
-        put(q, r, prev, val[t]);
+        ocode[word + lane] = code;
+        const uint4* v4 = (const uint4*)(rv + at);
+        uint4* o4 = (uint4*)(oval + (word + lane) * RB_GROUP);
+#pragma unroll
+        for (int u = 0; u < (int)sizeof(ValT) * RB_GROUP / 16; ++u) o4[u] = v4[u];
       }
-      const int64_t lr = __shfl_sync(0xffffffffu, r, (tot > 0 ? min(31, (int)(hi - 1 - t0)) : 0));
-      if (hi > t0) last_row = lr;
-      o += tot;
+      word += words;
+      head = (head + RB_GROUP * words) & (RC_RING - 1);
+      cur -= RB_GROUP * words;
+      __syncwarp();
+    };
+    int last = 0;                  // the row before t0
+    int64_t t0 = s;
+    int nrow = s + lane < hi ? rowidx[s + lane] : 0;     // one group ahead
+    ValT nval = s + lane < hi ? val[s + lane] : ValT(0.f);
+    while (t0 < hi) {
+      const bool on = t0 + lane < hi;
+      const int r = nrow - first;
+      const ValT v = nval;
+      const int up = __shfl_up_sync(0xffffffffu, r, 1);
+      const int rp = lane > 0 ? up : t0 > s ? last : r;
+      const int k = on ? rb_pads(r - rp) : 0;
+      int incl = lane + 1;                                 // no padding: one place each
+      if (__any_sync(0xffffffffu, k > 0)) {
+        incl = on ? k + 1 : 0;
+#pragma unroll
+        for (int sh = 1; sh < 32; sh <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, incl, sh);
+          if (lane >= sh) incl += y;
+        }
+      }
+      // as many entries as 256 places take (one entry takes at most 261)
+      const unsigned fit = __ballot_sync(0xffffffffu, on && (incl <= 256 || lane == 0));
+      const int m = __popc(fit);
+      const int tot = __shfl_sync(0xffffffffu, incl, m - 1);
+      last = __shfl_sync(0xffffffffu, r, m - 1);
+      const int64_t tn = t0 + m;
+      if (cur + tot > RC_RING) flush(cur / RB_GROUP);   // fewer than 256 places: at most 31 words
+      if (tn + lane < hi) {
+        nrow = rowidx[tn + lane];
+        nval = val[tn + lane];
+      }
+      if (lane < m) {
+        int q = head + cur + incl - (k + 1);
+        for (int u = 1; u <= k; ++u, ++q) {
+          rr[q & (RC_RING - 1)] = (uint16_t)(rp + 63 * u);
+          rv[q & (RC_RING - 1)] = ValT(0.f);
+        }
+        rr[q & (RC_RING - 1)] = (uint16_t)r;
+        rv[q & (RC_RING - 1)] = v;
+      }
+      cur += tot;
+      t0 = tn;
+      if (cur >= 256) flush(32);
     }
     // value-0 entries up to the group boundary, at the last row
-    for (int64_t q = o + lane; q < dend; q += 32) put(q, last_row, last_row, ValT(0.f));
+    const int fill = (RB_GROUP - cur % RB_GROUP) % RB_GROUP;
+    if (lane < fill) {
+      rr[(head + cur + lane) & (RC_RING - 1)] = (uint16_t)last;
+      rv[(head + cur + lane) & (RC_RING - 1)] = ValT(0.f);
+    }
+    cur += fill;
+    if (cur >= 256) flush(32);
+    if (cur > 0) flush(cur / RB_GROUP);
   }
 }
 
@@ -1615,7 +1682,6 @@ static void rb_build(sv_context* ctx, const sv_counts* C, const sv_data* data, c
              (long long)nnz_h);
   size_t es2 = sv_elem_size(data->dtype);
   rb_idx.alloc(std::max<int64_t>(1, tot / RB_GROUP));
-  sv_memset(ctx, rb_idx.get(), 0, std::max<int64_t>(1, tot / RB_GROUP) * 8);
   rb_val.alloc(std::max<int64_t>(1, tot) * es2);
   rb_partial.alloc(std::max<int64_t>(1, np));
   int gridc = sv_grid_for(ctx, np * 32, 256, 8);
