@@ -1,14 +1,19 @@
 // normalize_cells on both copies of the count matrix (src/normalize.jl:17-55).
 //
-//   K1a  csr: one warp per cell; 128-bit loads of the counts, warp-shuffle sum
-//        s_c (integer, normalize.jl:24).  Lane l then evaluates the value of
-//        count l + 1 in that cell, f(l + 1, s_c) -- the division and log1p
-//        once per lane instead of once per entry -- and the row's values are
-//        written with one shuffle per entry (counts above 32 are evaluated
-//        directly; the second read of the row hits L1/L2): 509 -> 380 us at
-//        100,000 cells.
-//   K1b  csc: a flat map over the non-zeros: b = f(a, s[row]) with s gathered
-//        from the per-cell totals (10 MB at 1.3M cells, L2-resident).
+//   K1a  csr: one warp per cell; 128-bit loads of the counts, four in flight,
+//        warp-shuffle sum s_c (integer, normalize.jl:24).  Lane l then evaluates
+//        the value of count l + 1 in that cell, f(l + 1, s_c) -- the division
+//        and log1p once per lane instead of once per entry -- and the row's
+//        values are written with one shuffle per entry (counts above 32 are
+//        evaluated directly; the second read of the row hits L1/L2).  At 1,000 M
+//        entries of 500,000 cells to BF16: 1.18 ms, 0.75 of the copy bandwidth
+//        (1.80 with one load in flight and 64-bit offsets); 250 M entries of
+//        100,000 cells to FP32: 0.395 ms.
+//   K1b  csc: a flat map over the non-zeros: b = f(a, s[row]) by a gather from
+//        the table of values that K1a leaves (evaluated per entry: FP64 165 us
+//        for 2 M entries, bound by the FP64 pipe, gathered 14; FP32 0.88 -> 0.59
+//        ms for 250 M; BF16 3.44 -> 1.85 ms for 1,000 M).  What is left is the
+//        gathers: one L2 sector per entry of a sparse gene.
 //
 // Every value is the same expression f(a, s) = log1p((sf * a) / s) (or the
 // relative count) evaluated in the output type, whichever kernel and path
@@ -19,6 +24,8 @@
 #include "sv_internal.cuh"
 
 namespace {
+
+constexpr int NORM_TABLE = 32;   // counts whose values a cell's table holds: one per lane
 
 struct NormArgs {
   double sf;
@@ -104,77 +111,121 @@ template <typename OutT>
 __global__ void __launch_bounds__(256) k_norm_csr(const int64_t* __restrict__ rowptr,
                                                   const int32_t* __restrict__ cnt, int64_t n_rows,
                                                   NormArgs p, OutT* __restrict__ out,
-                                                  int64_t* __restrict__ totals) {
+                                                  int64_t* __restrict__ totals, OutT* __restrict__ table) {
   int lane = threadIdx.x & 31;
   int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t r = warp; r < n_rows; r += nwarps) {
     int64_t s = rowptr[r], e = rowptr[r + 1];
-    int64_t a0 = s & ~3ll;
+    const int64_t a0 = s & ~3ll;
+    const int32_t* rc = cnt + a0;
+    OutT* ro = out + a0;
+    const int head = (int)(s - a0), len = (int)(e - a0);
     int64_t sum = 0;
-    for (int64_t g = a0 + 4 * lane; g < e; g += 128) {
-      int v[4];
-      load4(cnt, g, v);
+    for (int g0 = 4 * lane; g0 < len; g0 += 512) {
+      int v[4][4];
 #pragma unroll
-      for (int t = 0; t < 4; ++t)
-        if (g + t >= s && g + t < e) sum += v[t];
+      for (int u = 0; u < 4; ++u) {
+        v[u][0] = v[u][1] = v[u][2] = v[u][3] = 0;
+        if (g0 + 128 * u < len) load4(rc, g0 + 128 * u, v[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+          if (g0 + 128 * u + t >= head && g0 + 128 * u + t < len) sum += v[u][t];
     }
     sum = sv_warp_sum(sum);
     if (lane == 0) totals[r] = sum;
     if (e == s) continue;
     const OutT tv = NormOp<OutT>::apply(lane + 1, sum, p);    // the value of count lane + 1
+    if (table) table[lane * n_rows + r] = tv;
     // every lane takes every pass: the shuffles need the whole warp
-    for (int64_t g0 = a0; g0 < e; g0 += 128) {
-      const int64_t g = g0 + 4 * lane;
-      int v[4] = {0, 0, 0, 0};
-      if (g < e) load4(cnt, g, v);
-      OutT o[4];
+    for (int g0 = 0; g0 < len; g0 += 256) {
+      int v[2][4];
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const bool tabbed = v[t] >= 1 && v[t] <= 32;
-        const OutT sh = shfl_out(tv, tabbed ? v[t] - 1 : 0);
-        o[t] = tabbed ? sh : NormOp<OutT>::apply(v[t], sum, p);
+      for (int u = 0; u < 2; ++u) {
+        v[u][0] = v[u][1] = v[u][2] = v[u][3] = 1;
+        if (g0 + 128 * u + 4 * lane < len) load4(rc, g0 + 128 * u + 4 * lane, v[u]);
       }
-      if (g < e) store4(out, g, s, e, o);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int g = g0 + 128 * u + 4 * lane;
+        OutT o[4];
+        bool tabbed = true;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          o[t] = shfl_out(tv, v[u][t] - 1);
+          tabbed = tabbed && (unsigned)(v[u][t] - 1) < 32u;
+        }
+        if (!tabbed) {
+#pragma unroll
+          for (int t = 0; t < 4; ++t)
+            if ((unsigned)(v[u][t] - 1) >= 32u) o[t] = NormOp<OutT>::apply(v[u][t], sum, p);
+        }
+        if (g < len) store4(ro, g, head, len, o);
+      }
     }
   }
 }
 
-// K1b: flat map over the CSC non-zeros, 4 per thread; s gathered from the
-// per-cell totals (10 MB at 1.3M cells, L2-resident).  (Gathering the value
-// from a per-cell table of the small counts instead measured slower: 825 vs
-// 691 us at 100,000 cells.)
-template <typename OutT>
+// K1b: flat map over the CSC non-zeros, 4 per thread.  The value of a count up to
+// NORM_TABLE is gathered from the table that K1a left, count-major: almost all
+// entries have the lowest counts, so a gather touches n_cells values and not
+// NORM_TABLE times as many, and the rows of a column, which ascend, share sectors.
+template <typename OutT, bool TABLE>
 __global__ void __launch_bounds__(256) k_norm_csc(const int32_t* __restrict__ rowidx,
                                                   const int32_t* __restrict__ cnt, int64_t nnz,
                                                   const int64_t* __restrict__ totals, NormArgs p,
-                                                  OutT* __restrict__ out) {
-  int64_t ngroups = (nnz + 3) >> 2;
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < ngroups;
-       q += (int64_t)gridDim.x * blockDim.x) {
-    int64_t g = q << 2;
-    int rv[4], cv[4];
-    load4(rowidx, g, rv);
-    load4(cnt, g, cv);
-    OutT o[4];
+                                                  OutT* __restrict__ out, const OutT* __restrict__ table,
+                                                  int64_t n_cells) {
+  const int64_t ngroups = (nnz + 3) >> 2;
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < ngroups; q += 2 * step) {
+    int rv[2][4], cv[2][4];
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      if (g + t < nnz) o[t] = NormOp<OutT>::apply(cv[t], __ldg(totals + rv[t]), p);
-      else o[t] = OutT(0.0f);
+    for (int u = 0; u < 2; ++u)
+      if (q + u * step < ngroups) {
+        load4(rowidx, (q + u * step) << 2, rv[u]);
+        load4(cnt, (q + u * step) << 2, cv[u]);
+      }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (q + u * step >= ngroups) break;
+      const int64_t g = (q + u * step) << 2;
+      OutT o[4];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        o[t] = OutT(0.0f);
+        if (TABLE && cv[u][t] >= 1 && cv[u][t] <= NORM_TABLE && g + t < nnz)
+          o[t] = table[(cv[u][t] - 1) * n_cells + rv[u][t]];
+      }
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+        if (g + t < nnz && !(TABLE && cv[u][t] >= 1 && cv[u][t] <= NORM_TABLE))
+          o[t] = NormOp<OutT>::apply(cv[u][t], __ldg(totals + rv[u][t]), p);
+      store4(out, g, 0, nnz, o);
     }
-    store4(out, g, 0, nnz, o);
   }
 }
 
 template <typename OutT>
 void run_normalize(sv_context* ctx, const sv_counts* c, sv_data* d, NormArgs p) {
   int64_t nnz = c->nnz;
+  // The table has NORM_TABLE values a cell, written a sector each: with a few
+  // entries a cell that costs more than the entries do (from twice as many
+  // entries as table values on, the table is at most a fifth of the writes).
+  const bool tabled = nnz >= 2 * NORM_TABLE * c->n_cells;
+  DevBuf<OutT> table;
+  if (tabled) table.alloc(NORM_TABLE * c->n_cells);
   sv_launch(ctx, "normalize_csr", k_norm_csr<OutT>, dim3(sv_grid_for(ctx, c->n_cells * 32, 256, 8)),
             dim3(256), 0, (const int64_t*)c->csr_rowptr.get(), (const int32_t*)c->csr_count.get(),
-            c->n_cells, p, (OutT*)d->csr_val.get(), d->totals.get());
-  sv_launch(ctx, "normalize_csc", k_norm_csc<OutT>, dim3(sv_grid_for(ctx, (nnz + 3) / 4, 256, 8)),
+            c->n_cells, p, (OutT*)d->csr_val.get(), d->totals.get(), tabled ? table.get() : (OutT*)nullptr);
+  sv_launch(ctx, "normalize_csc", tabled ? k_norm_csc<OutT, true> : k_norm_csc<OutT, false>,
+            dim3(sv_grid_for(ctx, (nnz + 3) / 4, 256, 8)),
             dim3(256), 0, (const int32_t*)c->csc_rowidx.get(), (const int32_t*)c->csc_count.get(),
-            nnz, (const int64_t*)d->totals.get(), p, (OutT*)d->csc_val.get());
+            nnz, (const int64_t*)d->totals.get(), p, (OutT*)d->csc_val.get(),
+            tabled ? (const OutT*)table.get() : (const OutT*)nullptr, c->n_cells);
 }
 
 }  // namespace
