@@ -386,6 +386,7 @@ __global__ void k_hsub_write(const int64_t* __restrict__ rowptr, const int32_t* 
 // the product gained 1% and the reordering cost more than it saved.
 constexpr int BO_EMPTY = 1024;   // most empty slots a segment may have to be reordered
 constexpr int BO_WARPS = 8;
+constexpr int XV_DEPTH = 4;      // groups per lane in flight of the double-float X v loop
 constexpr int XV_EPL16 = 8;      // entries per lane and group of the BF16 X v loop
 
 template <int NC, int EPL>
@@ -659,7 +660,7 @@ __global__ void __launch_bounds__(256) k_spmv_csr(
 }
 
 // ---- X v for the Lanczos W side, double-float in and out (FP32 storage) -------
-// The same row loop as k_spmv_csr with every FP64 operation removed: this part
+// The rows of k_spmv_csr with every FP64 operation removed: this part
 // issues one warp-wide FP64 instruction per ~17 cycles per SM, and the FP64
 // prologue and epilogue of k_spmv_csr kept its FP64 pipe 30% busy.  The vector
 // arrives as a double-float basis column (its FP32 high part is the FP32 x of
@@ -669,6 +670,15 @@ __global__ void __launch_bounds__(256) k_spmv_csr(
 // With stacked samples (blk non-null) block b handles the cells of blk[b] of
 // sample s = blk[b].seg with that sample's feature parameters (x, 1/std, clip,
 // mu at offset s * nf) and csub[s].
+// Bound by HBM (525 M BF16 entries of 500,000 cells: 357 us, 5.9 TB/s; 62 M FP32
+// entries of 50,000 cells: 77 us).  What it took to get there from 419 us, where
+// the issue slots were the limit (22 instructions per entry of a warp): the guards
+// at a row's ends only in its first and last round of groups, as a bit mask, and
+// for the whole warp (each lane branching by itself ran both forms); the minimum
+// without a comparison; rows handed to the warps of a block one at a time, their
+// ends loaded one row ahead; XV_DEPTH groups in flight, each reloaded as soon as
+// it is added (2, 3, 4, 6 groups: 405, 378, 357, 367 us).  Every lane adds the
+// groups it always did in the same order.
 __device__ __forceinline__ void dfx_fma(float& sh, float& sl, float ah, float al, float bh, float bl) {
   float p = ah * bh;
   float e = fmaf(ah, bh, -p);
@@ -697,8 +707,8 @@ __device__ __forceinline__ bool xv_df_prologue(
   __shared__ float redh[32], redl[32];
   __shared__ float sc[4];
   int sg = 0;
-  o.rb0 = 0;
-  o.rb1 = n_rows;
+  o.rb0 = n_rows * blockIdx.x / gridDim.x;
+  o.rb1 = n_rows * (blockIdx.x + 1) / gridDim.x;
   if (blk) {
     const BlkRange br = blk[blockIdx.x];
     sg = br.seg;
@@ -714,12 +724,29 @@ __device__ __forceinline__ bool xv_df_prologue(
     mu_l += po;
   }
   float mh = 0.f, ml = 0.f;
-  for (int64_t f = threadIdx.x; f < nf; f += blockDim.x) {
-    float xs = xh[f];
-    float P = inv_f[f] * xs;
-    float Q = xs == 0.f ? 0.f : clip_f[f] * xs;
-    ((float2*)smem_raw)[f] = make_float2(P, Q);
-    dfx_fma(mh, ml, mu_h[f], mu_l[f], xs, xl[f]);
+  for (int64_t f0 = threadIdx.x; f0 < nf; f0 += 4 * blockDim.x) {
+    float in[4][6];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int64_t f = f0 + u * blockDim.x;
+      if (f >= nf) break;
+      in[u][0] = xh[f];
+      in[u][1] = xl[f];
+      in[u][2] = inv_f[f];
+      in[u][3] = clip_f[f];
+      in[u][4] = mu_h[f];
+      in[u][5] = mu_l[f];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int64_t f = f0 + u * blockDim.x;
+      if (f >= nf) break;
+      const float xs = in[u][0];
+      const float P = in[u][2] * xs;
+      const float Q = xs == 0.f ? 0.f : in[u][3] * xs;
+      ((float2*)smem_raw)[f] = make_float2(P, Q);
+      dfx_fma(mh, ml, in[u][4], in[u][5], xs, in[u][1]);
+    }
   }
   // mu.x: warp reduction in double-float, then warp 0 over the warps
 #pragma unroll
@@ -780,8 +807,45 @@ __device__ __forceinline__ void xv_df_store(float acc, const XvDf& p, bool has_z
   yh[r] = t;
 }
 
+// One lane's group of E consecutive entries of a row, as loaded: 16-byte loads of
+// indices and values where both are 16-bit, else 4 entries.
 template <typename ValT, typename IdxT>
-__global__ void __launch_bounds__(256) k_spmv_csr_df(
+struct XvGroup {
+  static constexpr int E = sizeof(ValT) == 2 && sizeof(IdxT) == 2 ? XV_EPL16 : 4;
+  unsigned i[E * sizeof(IdxT) / 4], v[E * sizeof(ValT) / 4];
+  template <int N>
+  static __device__ __forceinline__ void ld(unsigned (&w)[N], const void* p) {
+    if constexpr (N == 4) {
+      const uint4 x = __ldg((const uint4*)p);
+      w[0] = x.x;
+      w[1] = x.y;
+      w[2] = x.z;
+      w[3] = x.w;
+    } else {
+      const uint2 x = __ldg((const uint2*)p);
+      w[0] = x.x;
+      w[1] = x.y;
+    }
+  }
+  __device__ __forceinline__ void load(const IdxT* pi, const ValT* pv, int q) {
+    ld(i, pi + q);
+    ld(v, pv + q);
+  }
+  __device__ __forceinline__ unsigned index(int t) const {
+    return sizeof(IdxT) == 2 ? ((t & 1) ? i[t >> 1] >> 16 : i[t >> 1] & 0xffffu) : i[t];
+  }
+  // min(a P, Q) for P >= 0, max(a P, Q) for P < 0, as the sign of P on min(a |P|, |Q|)
+  // (P and Q have one sign): one minimum and no comparison
+  __device__ __forceinline__ float term(int t, float2 x) const {
+    const float a = __uint_as_float(
+        sizeof(ValT) == 2 ? ((t & 1) ? v[t >> 1] & 0xffff0000u : v[t >> 1] << 16) : v[t]);
+    const float m = fminf(a * fabsf(x.x), fabsf(x.y));
+    return __uint_as_float(__float_as_uint(m) ^ (__float_as_uint(x.x) & 0x80000000u));
+  }
+};
+
+template <typename ValT, typename IdxT>
+__global__ void __launch_bounds__(256, 4) k_spmv_csr_df(
     const int64_t* __restrict__ rowptr, const IdxT* __restrict__ hcol, const ValT* __restrict__ hval,
     int64_t n_rows, int64_t nf, const float* __restrict__ xh, const float* __restrict__ xl,
     const float* __restrict__ inv_f, const float* __restrict__ clip_f, const float* __restrict__ mu_h,
@@ -789,104 +853,67 @@ __global__ void __launch_bounds__(256) k_spmv_csr_df(
     const double* __restrict__ csub, const float* __restrict__ zh, const float* __restrict__ zl,
     const BlkRange* __restrict__ blk, const int* __restrict__ active) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int next_row;
   XvDf pr;
+  if (threadIdx.x == 0) next_row = 0;
   if (!xv_df_prologue(smem_raw, n_rows, nf, xh, xl, inv_f, clip_f, mu_h, mu_l, csub, blk, active, pr))
     return;
   const int64_t rb0 = pr.rb0, rb1 = pr.rb1;
+  const float2* pq = (const float2*)smem_raw;
 
-  int lane = threadIdx.x & 31;
-  int64_t warp, nwarps;
-  if (blk) {
-    warp = rb0 + (threadIdx.x >> 5);
-    nwarps = blockDim.x >> 5;
-  } else {
-    warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  }
-  for (int64_t r = warp; r < rb1; r += nwarps) {
-    int64_t s = rowptr[r], e = rowptr[r + 1];
-    int64_t a0 = s & ~3ll;
+  const int lane = threadIdx.x & 31;
+  constexpr int E = XvGroup<ValT, IdxT>::E;
+  constexpr int STEP = 32 * E;                 // entries of a warp's group round
+  auto take = [&](int64_t& r, int64_t& s, int64_t& e) {
+    int k = 0;
+    if (lane == 0) k = atomicAdd(&next_row, 1);
+    r = rb0 + __shfl_sync(0xffffffffu, k, 0);
+    if (r < rb1) {
+      s = rowptr[r];
+      e = rowptr[r + 1];
+    }
+  };
+  int64_t r, s = 0, e = 0;
+  take(r, s, e);
+  while (r < rb1) {
+    int64_t rn, sn = 0, en = 0;                // the next row's ends arrive meanwhile
+    take(rn, sn, en);
+    const int64_t b0 = s & ~(int64_t)(E - 1);
+    const IdxT* pi = hcol + b0;
+    const ValT* pv = hval + b0;
+    const int ls = (int)(s - b0), le = (int)(e - b0);
+    XvGroup<ValT, IdxT> buf[XV_DEPTH];
+#pragma unroll
+    for (int h = 0; h < XV_DEPTH; ++h)
+      if (STEP * h + E * lane < le) buf[h].load(pi, pv, STEP * h + E * lane);
     float acc = 0.f;
-    // two 4-element groups per lane in flight, the first load pair
-    // unconditional (a loop over guarded groups -- 2 or 4 of them -- measured
-    // 20-30% slower at the atlas size)
-    if constexpr (sizeof(ValT) == 2 && sizeof(IdxT) == 2) {
-      // 16-byte loads of 8 entries per lane and group, two groups (512
-      // entries per warp) in flight: a row of ~1,000 entries takes three load
-      // rounds instead of five (1.31 -> 1.18 ms per product at the atlas
-      // size); 32-bit offsets within the row from its start rounded down to
-      // 8 entries; words unpacked at use
-      constexpr int E = XV_EPL16;
-      const int64_t b0 = s & ~(int64_t)(E - 1);
-      const uint16_t* pi = (const uint16_t*)hcol + b0;
-      const uint16_t* pv = (const uint16_t*)hval + b0;
-      const int ls = (int)(s - b0), le = (int)(e - b0);
-      for (int q = E * lane; q < le; q += 64 * E) {
-        uint4 ri[2], rv[2];
-        const bool two = q + 32 * E < le;
-        ri[0] = __ldg((const uint4*)(pi + q));
-        rv[0] = __ldg((const uint4*)(pv + q));
-        if (two) {
-          ri[1] = __ldg((const uint4*)(pi + q + 32 * E));
-          rv[1] = __ldg((const uint4*)(pv + q + 32 * E));
-        }
+    for (int k0 = 0; k0 < le; k0 += STEP * XV_DEPTH) {
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          if (h == 1 && !two) break;
-          const int qh = q + 32 * E * h;
-          const unsigned wi[4] = {ri[h].x, ri[h].y, ri[h].z, ri[h].w};
-          const unsigned wv[4] = {rv[h].x, rv[h].y, rv[h].z, rv[h].w};
-          if (qh >= ls && qh + E <= le) {
-            // a group inside the row (all but a row's first and last): no guards
+      for (int h = 0; h < XV_DEPTH; ++h) {
+        const int k = k0 + STEP * h;
+        if (k >= le) break;
+        const int q = k + E * lane;
+        if (k >= ls && k + STEP <= le) {
 #pragma unroll
-            for (int t = 0; t < E; ++t) {
-              const int ci = (t & 1) ? (int)(wi[t >> 1] >> 16) : (int)(wi[t >> 1] & 0xffffu);
-              const float av = __uint_as_float((t & 1) ? (wv[t >> 1] & 0xffff0000u) : (wv[t >> 1] << 16));
-              const float2 pq = ((const float2*)smem_raw)[ci];
-              const float rr = av * pq.x;
-              acc += pq.x >= 0.f ? fminf(rr, pq.y) : fmaxf(rr, pq.y);
-            }
-          } else {
+          for (int t = 0; t < E; ++t) acc += buf[h].term(t, pq[buf[h].index(t)]);
+        } else if (q < le) {
+          unsigned in = 0xffu >> max(0, 8 - (le - q));         // entries q .. of [ls, le)
+          if (q < ls) in &= 0xffu << (ls - q);
 #pragma unroll
-            for (int t = 0; t < E; ++t) {
-              if (qh + t >= ls && qh + t < le) {
-                const int ci = (t & 1) ? (int)(wi[t >> 1] >> 16) : (int)(wi[t >> 1] & 0xffffu);
-                const float av = __uint_as_float((t & 1) ? (wv[t >> 1] & 0xffff0000u) : (wv[t >> 1] << 16));
-                const float2 pq = ((const float2*)smem_raw)[ci];
-                const float rr = av * pq.x;
-                acc += pq.x >= 0.f ? fminf(rr, pq.y) : fmaxf(rr, pq.y);
-              }
-            }
+          for (int t = 0; t < E; ++t) {
+            const bool on = in & (1u << t);
+            const float m = buf[h].term(t, pq[on ? buf[h].index(t) : 0]);
+            acc += on ? m : 0.f;
           }
         }
-      }
-    } else
-    for (int64_t g = a0 + 4 * lane; g < e; g += 256) {
-      int ci[2][4];
-      float av[2][4];
-      bool two = g + 128 < e;
-      ld4(hcol, g, ci[0]);
-      ld4v(hval, g, av[0]);
-      if (two) {
-        ld4(hcol, g + 128, ci[1]);
-        ld4v(hval, g + 128, av[1]);
-      }
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        if (h == 1 && !two) break;
-        int64_t gh = g + 128 * h;
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          if (gh + t >= s && gh + t < e) {
-            float2 pq = ((const float2*)smem_raw)[ci[h][t]];
-            float rr = av[h][t] * pq.x;
-            acc += pq.x >= 0.f ? fminf(rr, pq.y) : fmaxf(rr, pq.y);
-          }
-        }
+        if (q + STEP * XV_DEPTH < le) buf[h].load(pi, pv, q + STEP * XV_DEPTH);
       }
     }
     acc = sv_warp_sum(acc);
     if (lane == 0) xv_df_store(acc, pr, zh != nullptr, zh ? zh[r] : 0.f, zh ? zl[r] : 0.f, yh, yl, r);
+    r = rn;
+    s = sn;
+    e = en;
   }
 }
 
@@ -1010,6 +1037,7 @@ __global__ void k_spmv_t_finish(const AccT* __restrict__ partial, int nblocks, i
 // BF16 value) and no gather reaches L2.
 constexpr int64_t RB_ROWS = 16384;
 constexpr int RB_THREADS = 512;
+constexpr int RB_DEPTH2 = 4, RB_DEPTH4 = 3;   // groups per lane in flight, BF16 and FP32
 
 // first row of row block b: b * RB_ROWS, or row0[b] for blocks aligned to
 // sample boundaries
@@ -1166,51 +1194,66 @@ __global__ void __launch_bounds__(RC_WARPS * 32) k_rb_copy(
   }
 }
 
-// sum over a segment of whole groups (g0 .. g1) of min(a (1/sigma), clip) u[row];
-// two groups per lane in flight, lane-local decoding
+// One lane's group of 8 entries of the row-blocked copy, as loaded.
+template <typename ValT>
+struct RbGroup {
+  unsigned long long c;
+  uint4 v[sizeof(ValT) == 2 ? 1 : 2];
+  __device__ __forceinline__ void load(const unsigned long long* __restrict__ code, const ValT* __restrict__ pv) {
+    c = __ldg(code);
+    v[0] = __ldg((const uint4*)pv);
+    if constexpr (sizeof(ValT) == 4) v[1] = __ldg((const uint4*)pv + 1);
+  }
+  __device__ __forceinline__ void add(float& acc, float inv, float clip, const float* us) const {
+    // byte offsets into us: a field is shifted to bit 2 and masked
+    const unsigned lo = (unsigned)c, hi = (unsigned)(c >> 32);
+    unsigned r = (lo & 0xffffu) << 2;
+#pragma unroll
+    for (int t = 0; t < RB_GROUP; ++t) {
+      if (t > 0) {
+        const int at = 16 + 6 * (t - 1) - 2;
+        r += (at >= 32 ? hi >> (at - 32) : at + 8 > 32 ? __funnelshift_r(lo, hi, at) : lo >> at) & 0xfcu;
+      }
+      float a;
+      if constexpr (sizeof(ValT) == 2) {
+        const unsigned w = (&v[0].x)[t >> 1];
+        a = __uint_as_float((t & 1) ? (w & 0xffff0000u) : (w << 16));
+      } else {
+        a = __uint_as_float((&v[t >> 2].x)[t & 3]);
+      }
+      acc += fminf(a * inv, clip) * *(const float*)((const char*)us + r);
+    }
+  }
+};
+
+// sum over a segment of n groups of min(a (1/sigma), clip) u[row]; lane-local
+// decoding, a group reloaded as soon as it is added
 template <typename ValT>
 __device__ __forceinline__ float rb_seg_dot(const unsigned long long* __restrict__ code,
-                                           const ValT* __restrict__ pv, int64_t g0, int64_t g1,
+                                           const ValT* __restrict__ pv, int n,
                                            float inv, float clip, const float* us, int lane) {
+  constexpr int D = sizeof(ValT) == 2 ? RB_DEPTH2 : RB_DEPTH4;
+  RbGroup<ValT> buf[D];
+#pragma unroll
+  for (int h = 0; h < D; ++h) {
+    const int g = lane + 32 * h;
+    if (g < n) buf[h].load(code + g, pv + RB_GROUP * g);
+  }
   float acc = 0.f;
-  for (int64_t g = g0 + lane; g < g1; g += 64) {
-    unsigned long long c[2];
-    uint4 rv[2][sizeof(ValT) == 2 ? 1 : 2];
+  for (int g0 = lane; g0 < n; g0 += 32 * D) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
-      if (g + 32 * h < g1) {
-        c[h] = __ldg(code + g + 32 * h);
-        const uint4* vp = (const uint4*)(pv + (g + 32 * h) * RB_GROUP);
-        rv[h][0] = __ldg(vp);
-        if constexpr (sizeof(ValT) == 4) rv[h][1] = __ldg(vp + 1);
-      }
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      if (g + 32 * h >= g1) break;
-      int r = (int)(c[h] & 0xffffu);
-      unsigned long long st = c[h] >> 16;
-#pragma unroll
-      for (int t = 0; t < RB_GROUP; ++t) {
-        if (t > 0) {
-          r += (int)(st & 63u);
-          st >>= 6;
-        }
-        float a;
-        if constexpr (sizeof(ValT) == 2) {
-          const unsigned w = (&rv[h][0].x)[t >> 1];
-          a = __uint_as_float((t & 1) ? (w & 0xffff0000u) : (w << 16));
-        } else {
-          a = __uint_as_float((&rv[h][t >> 2].x)[t & 3]);
-        }
-        acc += fminf(a * inv, clip) * us[r];
-      }
+    for (int h = 0; h < D; ++h) {
+      const int g = g0 + 32 * h;
+      if (g >= n) break;
+      buf[h].add(acc, inv, clip, us);
+      if (g + 32 * D < n) buf[h].load(code + g + 32 * D, pv + RB_GROUP * (g + 32 * D));
     }
   }
   return acc;
 }
 
 template <typename ValT>
-__global__ void __launch_bounds__(RB_THREADS) k_spmv_rb(
+__global__ void __launch_bounds__(RB_THREADS, 2) k_spmv_rb(
     const int64_t* __restrict__ rb_ptr, const unsigned long long* __restrict__ rb_code,
     const ValT* __restrict__ rb_val, int64_t nf, int64_t n_cells, const float* __restrict__ inv_f,
     const float* __restrict__ clip_f, const float* __restrict__ uf, float* __restrict__ partial,
@@ -1238,7 +1281,7 @@ __global__ void __launch_bounds__(RB_THREADS) k_spmv_rb(
   for (int64_t f = g + (int64_t)fg * w; f < nf; f += (int64_t)fg * nw) {
     int64_t s = rb_ptr[b * nf + f], e = rb_ptr[b * nf + f + 1];
     float inv = inv_f[f], clip = clip_f[f];
-    float acc = rb_seg_dot<ValT>(rb_code, rb_val, s / RB_GROUP, e / RB_GROUP, inv, clip, us, lane);
+    float acc = rb_seg_dot<ValT>(rb_code + s / RB_GROUP, rb_val + s, (int)((e - s) / RB_GROUP), inv, clip, us, lane);
     acc = sv_warp_sum(acc);
     if (lane == 0) partial[b * nf + f] = acc;
   }
@@ -1246,16 +1289,20 @@ __global__ void __launch_bounds__(RB_THREADS) k_spmv_rb(
 
 // The same product for one sample, as a single wave of resident blocks: tasks
 // (row block b, feature group g) taken round-robin (b-major), the features of
-// a task (g, g + fg, ...) handed to the warps one at a time through a shared
-// counter, so that dense and sparse features even out within the block and no
-// partial last wave is left (the grid form above ran 3.2 waves of blocks with
-// 43% of its warps active).  Same loop and partials as k_spmv_rb.
+// a task (order[g], order[g + fg], ...: long ones first) handed to the warps one
+// at a time through a shared counter, so that dense and sparse features even out
+// within the block.  Same sums and partials as k_spmv_rb.  525 M BF16 entries of
+// 500,000 cells: 321 us, 4.9 TB/s (368 us with groups of whatever size gave six
+// tasks a block -- seven to some -- and features in their own order); 62 M FP32
+// entries of 50,000 cells: 74 us.  The gathers are what is left: 32 rows anywhere
+// in the vector take 3.4 passes over the shared-memory banks, and the data pipe of
+// L1 is busy 0.7 of the time.  48 warps an SM in place of 32 measured the same.
 template <typename ValT>
 __global__ void __launch_bounds__(RB_THREADS, 2) k_spmv_rb_waves(
     const int64_t* __restrict__ rb_ptr, const unsigned long long* __restrict__ rb_code,
     const ValT* __restrict__ rb_val, int64_t nf, int64_t n_cells, int64_t n_rb, int fg,
     const float* __restrict__ inv_f, const float* __restrict__ clip_f, const float* __restrict__ uf,
-    float* __restrict__ partial) {
+    float* __restrict__ partial, const int32_t* __restrict__ order) {
   extern __shared__ __align__(16) float us[];
   __shared__ int next_f;
   const int lane = threadIdx.x & 31;
@@ -1269,19 +1316,54 @@ __global__ void __launch_bounds__(RB_THREADS, 2) k_spmv_rb_waves(
     for (int64_t i = threadIdx.x; i < RB_ROWS; i += blockDim.x) us[i] = i < nr ? uf[r0 + i] : 0.f;
     if (threadIdx.x == 0) next_f = 0;
     __syncthreads();
-    while (true) {
+    // a warp's next feature and its segment arrive while it adds this one's
+    auto take = [&](int64_t& f, int64_t& s, int64_t& e, float& inv, float& clip) {
       int fi = 0;
       if (lane == 0) fi = atomicAdd(&next_f, 1);
-      fi = __shfl_sync(0xffffffffu, fi, 0);
-      const int64_t f = g + (int64_t)fi * fg;
-      if (f >= nf) break;
-      const int64_t s = rb_ptr[b * nf + f], e = rb_ptr[b * nf + f + 1];
-      const float inv = inv_f[f], clip = clip_f[f];
-      float acc = rb_seg_dot<ValT>(rb_code, rb_val, s / RB_GROUP, e / RB_GROUP, inv, clip, us, lane);
+      f = g + (int64_t)__shfl_sync(0xffffffffu, fi, 0) * fg;
+      if (f < nf) {
+        f = order[f];
+        s = rb_ptr[b * nf + f];
+        e = rb_ptr[b * nf + f + 1];
+        inv = inv_f[f];
+        clip = clip_f[f];
+      }
+    };
+    int64_t f, s = 0, e = 0;
+    float inv = 0.f, clip = 0.f;
+    take(f, s, e, inv, clip);
+    while (f < nf) {
+      int64_t fn, sn = 0, en = 0;
+      float invn = 0.f, clipn = 0.f;
+      take(fn, sn, en, invn, clipn);
+      float acc = rb_seg_dot<ValT>(rb_code + s / RB_GROUP, rb_val + s, (int)((e - s) / RB_GROUP), inv, clip, us, lane);
       acc = sv_warp_sum(acc);
       if (lane == 0) partial[b * nf + f] = acc;
+      f = fn;
+      s = sn;
+      e = en;
+      inv = invn;
+      clip = clipn;
     }
   }
+}
+
+// order[rank] = f, features by falling number of entries: the warps of a task take
+// the long ones first, and what they wait for at its end is a short one.
+__global__ void __launch_bounds__(256) k_rb_order(const int64_t* __restrict__ fstart,
+                                                  const int64_t* __restrict__ fend, int64_t nf,
+                                                  int32_t* __restrict__ order) {
+  const int lane = threadIdx.x & 31;
+  const int64_t f = blockIdx.x * 8ll + (threadIdx.x >> 5);
+  if (f >= nf) return;
+  const int64_t n = fend[f] - fstart[f];
+  int rank = 0;
+  for (int64_t o = lane; o < nf; o += 32) {
+    const int64_t m = fend[o] - fstart[o];
+    rank += m > n || (m == n && o < f);
+  }
+  rank = sv_warp_sum(rank);
+  if (lane == 0) order[rank] = (int32_t)f;
 }
 
 // y_f = alpha * (sum_b partial[b][f] - mu_f * sum(u)) + beta*y_f - csub*z_f
@@ -1473,23 +1555,22 @@ constexpr int UPREP_BLOCKS = SV_UPREP_BLOCKS;
 // row-blocked CSC: u (FP32) staged per row block in shared memory
 static void launch_rb(sv_context* ctx, const sv_centered* S, const float* uf) {
   sv_centered* Sm = const_cast<sv_centered*>(S);
-  // one wave of resident blocks, ~6 tasks (row block, feature group) each,
-  // at least 32 features per task
-  const int resident = ctx->num_sms * S->rb_per_sm;
-  const int fg = (int)std::max<int64_t>(
-      1, std::min<int64_t>(std::max<int64_t>(1, S->nf / 32), (6 * resident + S->n_rb - 1) / S->n_rb));
+  const int64_t resident = ctx->num_sms * S->rb_per_sm;
+  const int fg = S->rb_fg;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(resident, S->n_rb * fg));
   size_t smem = RB_ROWS * sizeof(float);
   if (S->dtype == SV_F32)
     sv_launch(ctx, "spmv_rb", k_spmv_rb_waves<float>, dim3(grid), dim3(RB_THREADS), smem,
               (const int64_t*)S->rb_ptr.get(), (const unsigned long long*)S->rb_idx.get(),
               (const float*)S->rb_val.get(), S->nf, S->n_cells, S->n_rb, fg,
-              (const float*)S->inv_std_f.get(), (const float*)S->clip_f.get(), uf, Sm->rb_partial.get());
+              (const float*)S->inv_std_f.get(), (const float*)S->clip_f.get(), uf, Sm->rb_partial.get(),
+              (const int32_t*)S->rb_order.get());
   else
     sv_launch(ctx, "spmv_rb", k_spmv_rb_waves<__nv_bfloat16>, dim3(grid), dim3(RB_THREADS), smem,
               (const int64_t*)S->rb_ptr.get(), (const unsigned long long*)S->rb_idx.get(),
               (const __nv_bfloat16*)S->rb_val.get(), S->nf, S->n_cells, S->n_rb, fg,
-              (const float*)S->inv_std_f.get(), (const float*)S->clip_f.get(), uf, Sm->rb_partial.get());
+              (const float*)S->inv_std_f.get(), (const float*)S->clip_f.get(), uf, Sm->rb_partial.get(),
+              (const int32_t*)S->rb_order.get());
 }
 
 // CSC chunks over the feature ranges: u FP32 (uf) or, for FP64 data, FP64 (ud)
@@ -1666,6 +1747,30 @@ static std::vector<int32_t> feature_genes(const sv_counts* C, const int64_t* fea
 // (row block, feature) the block's entries of the feature, their rows within
 // the block coded in groups of 8 (see k_rb_count) and their values.  Row blocks of RB_ROWS rows, or with
 // first rows row0 (n_rb + 1 entries, device) when aligned to samples.
+// Feature groups per row block: the tasks (row block, group) go round robin to
+// `resident` blocks, so the time is that of the block with the most; each task also
+// loads its row block's vector (~2.5 us, here as bytes of a block's share of the
+// bandwidth), and 16 features at least are left to its 16 warps.
+static int rb_groups(int64_t resident, int64_t n_cells, int64_t nf, int64_t nnz, size_t es) {
+  const int64_t full = n_cells / RB_ROWS, part = n_cells % RB_ROWS;
+  const double row_bytes = (double)nnz * (es + 1) / n_cells;       // of a row over all features
+  const double load = 2.5e-6 * 6.8e12 / resident;
+  int64_t best = 1;
+  double least = 0;
+  for (int64_t fg = 1; fg <= std::max<int64_t>(1, nf / 16); ++fg) {
+    // block 0 has the most full tasks; the partial row block's tasks come last
+    const int64_t nt = full * fg + (part ? fg : 0);
+    const int64_t most = (full * fg + resident - 1) / resident;
+    const bool extra = part && (nt + resident - 1) / resident > most;
+    const double t = most * (row_bytes * RB_ROWS / fg + load) + (extra ? row_bytes * part / fg + load : 0);
+    if (fg == 1 || t < least) {
+      least = t;
+      best = fg;
+    }
+  }
+  return (int)best;
+}
+
 static void rb_build(sv_context* ctx, const sv_counts* C, const sv_data* data, const int64_t* fstart,
                      const int64_t* fend, int64_t nf, int64_t nnz_h, int64_t n_rb, const int64_t* row0,
                      DevBuf<int64_t>& rb_ptr, DevBuf<unsigned long long>& rb_idx, DevBuf<unsigned char>& rb_val,
@@ -1883,6 +1988,10 @@ static sv_centered* make_centered(sv_context* ctx, const sv_data* data, const st
           SV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_spmv_rb_waves<__nv_bfloat16>, RB_THREADS,
                                                                 RB_ROWS * sizeof(float)));
         S->rb_per_sm = std::max(1, per);
+        S->rb_fg = rb_groups(ctx->num_sms * S->rb_per_sm, C->n_cells, nf, nnz_h, sv_elem_size(data->dtype));
+        S->rb_order.alloc(nf);
+        sv_launch(ctx, "scale_rb_order", k_rb_order, dim3((unsigned)((nf + 7) / 8)), dim3(256), 0,
+                  (const int64_t*)S->feat_start.get(), (const int64_t*)S->feat_end.get(), nf, S->rb_order.get());
         sv_sync(ctx);
       }
     }
