@@ -292,7 +292,7 @@ struct sv_centered {
   // row-blocked CSC copy of the subset for X^T u (FP32 / BF16 storage)
   int64_t rb_rows = 0, n_rb = 0;      // rows per block, number of row blocks
   int rb_per_sm = 3;                  // resident blocks per SM of the X^T u kernel
-  int rb_fg = 1;                      // feature groups of its tasks
+  int rb_fg = 1, rb_fg_beside = 1;    // feature groups of its tasks: on all SMs, on all but one
   DevBuf<int32_t> rb_order;           // nf: features by falling number of entries
   DevBuf<int64_t> rb_ptr;             // n_rb * nf + 1 entry offsets, ordered (block, feature)
   DevBuf<unsigned long long> rb_idx;  // rows within the block, one coded word per 8 entries

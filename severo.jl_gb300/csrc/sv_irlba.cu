@@ -48,7 +48,7 @@ void sv_batch_apply_T(sv_context* ctx, const sv_batch* b, const double* u, doubl
                       const double* csub, const double* z, const int* active);
 
 void sv_centered_apply_t_part(sv_context* ctx, const sv_centered* S, const double* ud, const float* uf,
-                              SvTPart* o);
+                              SvTPart* o, bool beside);
 
 namespace {
 
@@ -1590,6 +1590,9 @@ __global__ void __launch_bounds__(1024) k_vside(const double* __restrict__ F0,
 // accumulated rotations J are held as (hi, lo) FP32 pairs in shared memory and
 // updated on the FP32 pipe, and the rotation parameters are formed in FP32 and
 // normalised in double-float.
+// Bound by the issue slots of its one SM (19 warps of ~320 instructions a round at
+// m = 37, two thirds of the slots): 389 us, 126 us at m = 22 (417 and 155 with J's
+// rotation in the chain, entries rotated one by one, and 32 warps).
 // Columns are paired by the circle method (slot 0 fixed, the others rotating),
 // one warp per pair; a pair is rotated while |a_p . a_q| > tau |a_p| |a_q| with
 // tau = 1e-12 max(1, m / 16): a double-float dot product of m terms carries an
@@ -1629,6 +1632,23 @@ __device__ __forceinline__ void df_rot(float& xh, float& xl, float& yh, float& y
   yl = bl - (yh - bh);
 }
 
+// The same on pairs of entries (rows or matrices), rotated by the same (c, s)
+__device__ __forceinline__ void df_rot2(f2_t& xh, f2_t& xl, f2_t& yh, f2_t& yl, float ch, float cl,
+                                        float sh, float sl) {
+  const f2_t c = f2_pack(ch, ch), nc = f2_pack(-ch, -ch), c2 = f2_pack(cl, cl);
+  const f2_t s = f2_pack(sh, sh), ns = f2_pack(-sh, -sh), s2 = f2_pack(sl, sl), ns2 = f2_pack(-sl, -sl);
+  f2_t ah = 0ull, al = 0ull, bh = 0ull, bl = 0ull;
+  df_fma2(ah, al, c, nc, c2, xh, xl);
+  df_fma2(ah, al, ns, s, ns2, yh, yl);
+  df_fma2(bh, bl, s, ns, s2, xh, xl);
+  df_fma2(bh, bl, c, nc, c2, yh, yl);
+  xh = f2_add(ah, al);
+  xl = f2_sub(al, f2_sub(xh, ah));
+  yh = f2_add(bh, bl);
+  yl = f2_sub(bl, f2_sub(yh, bh));
+}
+
+template <int R>
 __global__ void __launch_bounds__(1024) k_jacobi_svd(const double* __restrict__ B0, int m,
                                                      double* __restrict__ Pout0,
                                                      double* __restrict__ sout0,
@@ -1673,6 +1693,36 @@ __global__ void __launch_bounds__(1024) k_jacobi_svd(const double* __restrict__ 
   int npairs = mp / 2;
   int lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
   const float tau = 1e-12f * fmaxf(1.f, (float)m / 16.f);
+  // With two rows per lane J follows one round behind: its rotation is off the
+  // chain from one round's columns to the next one's.  A round's pairs are
+  // disjoint, and all of them are done with it before the next round's end.
+  float ch = 0.f, cl = 0.f, sh = 0.f, sl = 0.f;
+  int jp = 0, jq = 0;
+  bool on = false;
+  auto rotate_j = [&]() {
+    const int r0 = lane, r1 = lane + 32 < m ? lane + 32 : lane;
+    f2_t x2 = f2_pack(Jh[jp + r0], Jh[jp + r1]), x2l = f2_pack(Jl[jp + r0], Jl[jp + r1]);
+    f2_t y2 = f2_pack(Jh[jq + r0], Jh[jq + r1]), y2l = f2_pack(Jl[jq + r0], Jl[jq + r1]);
+    df_rot2(x2, x2l, y2, y2l, ch, cl, sh, sl);
+    if (on) {
+      float v[8];
+      f2_unpack(x2, v[0], v[1]);
+      f2_unpack(x2l, v[2], v[3]);
+      f2_unpack(y2, v[4], v[5]);
+      f2_unpack(y2l, v[6], v[7]);
+      Jh[jp + r0] = v[0];
+      Jl[jp + r0] = v[2];
+      Jh[jq + r0] = v[4];
+      Jl[jq + r0] = v[6];
+      if (lane + 32 < m) {
+        Jh[jp + r1] = v[1];
+        Jl[jp + r1] = v[3];
+        Jh[jq + r1] = v[5];
+        Jl[jq + r1] = v[7];
+      }
+    }
+  };
+  int ka = wid - 1, kb = mp - 2 - wid;     // R <= 2: the slots of the warp's pair
   int sweep = 0;
   for (; sweep < max_sweeps; ++sweep) {
     if (tid == 0) rotated = 0;
@@ -1688,23 +1738,40 @@ __global__ void __launch_bounds__(1024) k_jacobi_svd(const double* __restrict__ 
     __syncthreads();
     for (int round = 0; round < mp - 1; ++round) {
       for (int pi = wid; pi < npairs; pi += nw) {
-        int a = pi == 0 ? 0 : 1 + (pi - 1 + round) % (mp - 1);
-        int b = 1 + (mp - 2 - pi + round) % (mp - 1);
-        if (a >= m || b >= m) continue;
-        int p = min(a, b), q = max(a, b);
-        float* aph = Ah + p * m;
-        float* apl = Al + p * m;
-        float* aqh = Ah + q * m;
-        float* aql = Al + q * m;
+        int a, b;
+        if constexpr (R <= 2) {              // the warp's only pair
+          a = pi == 0 ? 0 : 1 + ka;
+          b = 1 + kb;
+          ka = ka == mp - 2 ? 0 : ka + 1;
+          kb = kb == mp - 2 ? 0 : kb + 1;
+        } else {
+          a = pi == 0 ? 0 : 1 + (pi - 1 + round) % (mp - 1);
+          b = 1 + (mp - 2 - pi + round) % (mp - 1);
+        }
+        const bool pair = a < m && b < m;    // no dummy among them
+        const int p = pair ? min(a, b) : 0, q = pair ? max(a, b) : 0;
+        float xh[R], xl[R], yh[R], yl[R];
+#pragma unroll
+        for (int t = 0; t < R; ++t) {
+          const int r = lane + 32 * t;
+          xh[t] = r < m ? Ah[p * m + r] : 0.f;
+          xl[t] = r < m ? Al[p * m + r] : 0.f;
+          yh[t] = r < m ? Ah[q * m + r] : 0.f;
+          yl[t] = r < m ? Al[q * m + r] : 0.f;
+        }
         const float alh = cnh[p], all = cnl[p], beh = cnh[q], bel = cnl[q];
+        if constexpr (R == 2) rotate_j();    // the last round's, beside this one's sums
         float gah = 0.f, gal = 0.f;
-        for (int r = lane; r < m; r += 32) df_fma(gah, gal, aph[r], apl[r], aqh[r], aql[r]);
+#pragma unroll
+        for (int t = 0; t < R; ++t)
+          if (lane + 32 * t < m) df_fma(gah, gal, xh[t], xl[t], yh[t], yl[t]);
         df_warp_sum(gah, gal);
         // every lane holds the sums; the test and the angle are FP32 (from
         // double-float sums): the angle only steers convergence, while the
         // orthogonality of the applied rotation comes from normalising (c, s)
         // in double-float
-        if (fabsf(gah) > tau * sqrtf(alh) * sqrtf(beh) && gah != 0.f) {
+        on = pair && fabsf(gah) > tau * sqrtf(alh) * sqrtf(beh) && gah != 0.f;
+        if (on) {
           // be - al in double-float: close singular values still give an
           // accurate angle
           float dh = beh, dl = bel;
@@ -1720,12 +1787,42 @@ __global__ void __launch_bounds__(1024) k_jacobi_svd(const double* __restrict__ 
           df_fma(qh, ql, s0, 0.f, s0, 0.f);
           float d = (qh - 1.f) + ql;
           float fh = 1.f, fl = -0.5f * d;
-          float ch = 0.f, cl = 0.f, sh = 0.f, sl = 0.f;
+          ch = cl = sh = sl = 0.f;
           df_fma(ch, cl, c0, 0.f, fh, fl);
           df_fma(sh, sl, s0, 0.f, fh, fl);
-          for (int r = lane; r < m; r += 32) {
-            df_rot(aph[r], apl[r], aqh[r], aql[r], ch, cl, sh, sl);
-            df_rot(Jh[p * m + r], Jl[p * m + r], Jh[q * m + r], Jl[q * m + r], ch, cl, sh, sl);
+          if constexpr (R == 2) {
+            f2_t x2 = f2_pack(xh[0], xh[1]), x2l = f2_pack(xl[0], xl[1]);
+            f2_t y2 = f2_pack(yh[0], yh[1]), y2l = f2_pack(yl[0], yl[1]);
+            df_rot2(x2, x2l, y2, y2l, ch, cl, sh, sl);
+            f2_unpack(x2, xh[0], xh[1]);
+            f2_unpack(x2l, xl[0], xl[1]);
+            f2_unpack(y2, yh[0], yh[1]);
+            f2_unpack(y2l, yl[0], yl[1]);
+            jp = p * m;
+            jq = q * m;
+          } else {
+            // A and J in one packed rotation per row
+#pragma unroll
+            for (int t = 0; t < R; ++t) {
+              const int r = lane + 32 * t;
+              if (r >= m) break;
+              f2_t x2 = f2_pack(xh[t], Jh[p * m + r]), x2l = f2_pack(xl[t], Jl[p * m + r]);
+              f2_t y2 = f2_pack(yh[t], Jh[q * m + r]), y2l = f2_pack(yl[t], Jl[q * m + r]);
+              df_rot2(x2, x2l, y2, y2l, ch, cl, sh, sl);
+              f2_unpack(x2, xh[t], Jh[p * m + r]);
+              f2_unpack(x2l, xl[t], Jl[p * m + r]);
+              f2_unpack(y2, yh[t], Jh[q * m + r]);
+              f2_unpack(y2l, yl[t], Jl[q * m + r]);
+            }
+          }
+#pragma unroll
+          for (int t = 0; t < R; ++t) {
+            const int r = lane + 32 * t;
+            if (r >= m) break;
+            Ah[p * m + r] = xh[t];
+            Al[p * m + r] = xl[t];
+            Ah[q * m + r] = yh[t];
+            Al[q * m + r] = yl[t];
           }
           if (lane == 0) {
             rotated = 1;
@@ -1744,7 +1841,9 @@ __global__ void __launch_bounds__(1024) k_jacobi_svd(const double* __restrict__ 
     if (!rotated) break;
     __syncthreads();
   }
+  if constexpr (R == 2) rotate_j();
   if (sweep >= max_sweeps && tid == 0) atomicOr(status, SV_STATUS_LIMIT);
+  __syncthreads();
   // singular values and ordering
   for (int c = wid; c < m; c += nw) {
     float sh = 0.f, sl = 0.f;
@@ -1756,18 +1855,14 @@ __global__ void __launch_bounds__(1024) k_jacobi_svd(const double* __restrict__ 
     if (lane == 0) nrm[c] = sqrt(df_val(sh, sl));
   }
   __syncthreads();
-  if (tid == 0) {
-    // stable insertion sort, descending
-    for (int i = 0; i < m; ++i) order[i] = i;
-    for (int i = 1; i < m; ++i) {
-      int v = order[i];
-      int t = i - 1;
-      while (t >= 0 && nrm[order[t]] < nrm[v]) {
-        order[t + 1] = order[t];
-        --t;
-      }
-      order[t + 1] = v;
-    }
+  // descending, equal ones in column order (NaN leaves the order it has)
+  for (int i = tid; i < m; i += blockDim.x) order[i] = i;
+  __syncthreads();
+  for (int i = tid; i < m; i += blockDim.x) {
+    const double v = nrm[i];
+    int rank = 0;
+    for (int o = 0; o < m; ++o) rank += nrm[o] > v || (nrm[o] == v && o < i);
+    if (v == v) order[rank] = i;
   }
   __syncthreads();
   for (int idx = tid; idx < m * m; idx += blockDim.x) {
@@ -1785,7 +1880,7 @@ __global__ void __launch_bounds__(1024) k_jacobi_svd(const double* __restrict__ 
     summary[m + i] = s > 0 ? df_val(Ah[order[i] * m + (m - 1)], Al[order[i] * m + (m - 1)]) / s : 0.0;
   }
   if (tid == 0) {
-    summary[2 * m] = rf ? *rf : 0.0;
+    if (rf) summary[2 * m] = *rf;     // else written by the step that has it
     summary[2 * m + 1] = (double)sweep;
     double smax = fmax(ctl[CTL_SMAX], nrm[order[0]]);
     ctl[CTL_SMAX] = smax;
@@ -1938,7 +2033,9 @@ struct Op {
   // A^T x up to its partial sums (x as FP64 and FP32), which k_gstep finishes,
   // where the operator has that form
   virtual bool has_part() const { return false; }
-  virtual void T_part(const double* x, const float* xf, SvTPart* o) { (void)x, (void)xf, (void)o; }
+  virtual void T_part(const double* x, const float* xf, SvTPart* o, bool beside) {
+    (void)x, (void)xf, (void)o, (void)beside;
+  }
   // true when N and T only enqueue device work (no host round trip), so that a
   // Lanczos cycle over them can be captured as a CUDA graph
   virtual bool device_only() const { return false; }
@@ -1963,8 +2060,8 @@ struct CenteredOp : Op {
     sv_centered_apply(ctx, S, 'T', x, y, 1.0, 0.0, csub, z);
   }
   bool has_part() const override { return S->n_rb > 0 || S->t_blocks == 0; }
-  void T_part(const double* x, const float* xf, SvTPart* o) override {
-    sv_centered_apply_t_part(ctx, S, x, xf, o);
+  void T_part(const double* x, const float* xf, SvTPart* o, bool beside) override {
+    sv_centered_apply_t_part(ctx, S, x, xf, o, beside);
   }
   bool device_only() const override { return true; }
   bool N_df(const float* xh, const float* xl, float* yh, float* yl, const double* csub,
@@ -2242,8 +2339,9 @@ struct Lanczos {
     hsum = (double*)sv_ctx_run_stage(ctx, (size_t)nseg * (2 * work + 2) * 8 + (size_t)nseg * 4);
     hflags = (int*)(hsum + (size_t)nseg * (2 * work + 2));
     op->bind_active(active.get());
-    SV_CUDA(cudaFuncSetAttribute(k_jacobi_svd, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 4 * MAX_WORK * MAX_WORK * 4));
+    for (auto kern : {k_jacobi_svd<1>, k_jacobi_svd<2>, k_jacobi_svd<3>})
+      SV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   4 * MAX_WORK * MAX_WORK * 4));
     for (auto kern : {k_rotate_df<10>, k_rotate_df<16>, k_rotate_df<26>})
       SV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    MAX_WORK * (MAX_WORK / 2 + 13) * 16));
@@ -2330,7 +2428,10 @@ struct Lanczos {
       cudaGetLastError();
     }
     if (vfused && !ctx->side) {
-      SV_CUDA(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
+      // what runs there is short or narrow: before the product beside it
+      int least = 0, greatest = 0;
+      SV_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+      SV_CUDA(cudaStreamCreateWithPriority(&ctx->side, cudaStreamNonBlocking, greatest));
       for (cudaEvent_t& e : ctx->fork_ev) SV_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
   }
@@ -2523,6 +2624,17 @@ struct Lanczos {
     else w_settle_nj<12>(col);
   }
 
+  // SVD of B; rf: the residual norms for the summary, or null when the step that
+  // forms them writes them there.  A warp per column pair.
+  void svd(const double* rf) {
+    static_assert(MAX_WORK <= 96, "rows per lane");
+    auto kern = work <= 32 ? k_jacobi_svd<1> : work <= 64 ? k_jacobi_svd<2> : k_jacobi_svd<3>;
+    const int threads = 32 * std::min(32, (work + 1) / 2);
+    sv_launch(ctx, "irlba_svd", kern, dim3(nseg), dim3(threads), (size_t)4 * work * work * 4,
+              (const double*)B.get(), work, P.get(), sig.get(), Q.get(), summary.get(), rf, 60, ctx->d_status,
+              ctl(), eps_b, (const int*)active.get());
+  }
+
   // One cycle, enqueued on the context stream without any host round trip:
   // for a restart, V <- V Q_k, W <- W P_k, V[:, k] = f/|f| and B reset; the
   // Lanczos steps k..work-1; the SVD of B; the summaries copied to hsum.
@@ -2576,7 +2688,16 @@ struct Lanczos {
       // F = A^T W[:, j] - S V[:, j]; CGS2 against V[:, :j+1]
       SvTPart tp;
       if (vfused) {
-        op->T_part(Ws.cur.get(), uf.get(), &tp);
+        // B is complete: its SVD, on one SM, beside the residual's product and
+        // step (2,000 cells FP64: 33.0 -> 26.1 ms together with the SVD's own gain;
+        // 500,000 cells BF16: all of its 374 us, 11 times)
+        const bool last = j + 1 == work;
+        if (last) {
+          fork();
+          svd(nullptr);
+          split();
+        }
+        op->T_part(Ws.cur.get(), uf.get(), &tp, last && capturing);
       } else {
         op->T(Ws.cur.get(), F.get(), s0, Vs.cur.get());
         g_col(j);
@@ -2601,7 +2722,7 @@ struct Lanczos {
         scale_col(Ws, j + 1, s0, c, (int64_t)(j + 1) * work + j + 1, seed, step++);
         ++j;
       } else {
-        if (vfused) vside_fused(tp, j, -1, s1, c, -1, seed, step++);   // residual f and |f|
+        if (vfused) vside_fused(tp, j, -1, summary.get() + 2 * work, c, -1, seed, step++);   // residual f and |f|
         else vside(j + 1, -1, s1, c, -1, seed, step++);
         break;
       }
@@ -2609,9 +2730,8 @@ struct Lanczos {
     // the last cell-side column's second projection: W is complete for the
     // restart rotation and the final U
     if (pending) w_settle(j);
-    sv_launch(ctx, "irlba_svd", k_jacobi_svd, dim3(nseg), dim3(1024), (size_t)4 * work * work * 4,
-              (const double*)B.get(), work, P.get(), sig.get(), Q.get(), summary.get(),
-              (const double*)s1, 60, ctx->d_status, ctl(), eps_b, act);
+    if (vfused) join();
+    else svd(s1);
     SV_CUDA(cudaMemcpyAsync(hsum, summary.get(), (size_t)nseg * (2 * work + 2) * 8,
                             cudaMemcpyDeviceToHost, ctx->stream));
     return nmv;

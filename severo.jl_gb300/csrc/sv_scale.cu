@@ -1553,10 +1553,10 @@ constexpr int UPREP_BLOCKS = SV_UPREP_BLOCKS;
 // internal product entry points (device vectors), used by irlba too
 // ---------------------------------------------------------------------------
 // row-blocked CSC: u (FP32) staged per row block in shared memory
-static void launch_rb(sv_context* ctx, const sv_centered* S, const float* uf) {
+static void launch_rb(sv_context* ctx, const sv_centered* S, const float* uf, bool beside = false) {
   sv_centered* Sm = const_cast<sv_centered*>(S);
-  const int64_t resident = ctx->num_sms * S->rb_per_sm;
-  const int fg = S->rb_fg;
+  const int64_t resident = (ctx->num_sms - (beside ? 1 : 0)) * (int64_t)S->rb_per_sm;
+  const int fg = beside ? S->rb_fg_beside : S->rb_fg;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(resident, S->n_rb * fg));
   size_t smem = RB_ROWS * sizeof(float);
   if (S->dtype == SV_F32)
@@ -1574,9 +1574,11 @@ static void launch_rb(sv_context* ctx, const sv_centered* S, const float* uf) {
 }
 
 // CSC chunks over the feature ranges: u FP32 (uf) or, for FP64 data, FP64 (ud)
-static void launch_chunks(sv_context* ctx, const sv_centered* S, const double* ud, const float* uf) {
+static void launch_chunks(sv_context* ctx, const sv_centered* S, const double* ud, const float* uf,
+                          bool beside = false) {
   sv_centered* Sm = const_cast<sv_centered*>(S);
   int grid = sv_grid_for(ctx, S->n_chunks * 32, 256, 8);
+  if (beside) grid = std::min(grid, 8 * (ctx->num_sms - 1));
   const sv_data* D = S->data;
   const int32_t* rowidx = D->counts->csc_rowidx.get();
 #define LAUNCH_CSC(VT)                                                                            \
@@ -1596,16 +1598,17 @@ static void launch_chunks(sv_context* ctx, const sv_centered* S, const double* u
 
 // The partial sums of X^T u alone, for a caller that finishes them itself (the
 // Lanczos feature side): u as FP64 and as FP32.  Not for the form over CSR_h.
+// beside: a block of another kernel runs at the same time; its place is left free.
 void sv_centered_apply_t_part(sv_context* ctx, const sv_centered* S, const double* ud, const float* uf,
-                              SvTPart* o) {
+                              SvTPart* o, bool beside) {
   o->mu = S->mu.get();
   o->nf = S->nf;
   if (S->n_rb > 0) {
-    launch_rb(ctx, S, uf);
+    launch_rb(ctx, S, uf, beside);
     o->rb = S->rb_partial.get();
     o->n_rb = S->n_rb;
   } else {
-    launch_chunks(ctx, S, ud, uf);
+    launch_chunks(ctx, S, ud, uf, beside);
     o->chunk = S->chunk_partial.get();
     o->foff = S->feat_chunk_off.get();
   }
@@ -1989,6 +1992,8 @@ static sv_centered* make_centered(sv_context* ctx, const sv_data* data, const st
                                                                 RB_ROWS * sizeof(float)));
         S->rb_per_sm = std::max(1, per);
         S->rb_fg = rb_groups(ctx->num_sms * S->rb_per_sm, C->n_cells, nf, nnz_h, sv_elem_size(data->dtype));
+        S->rb_fg_beside =
+            rb_groups((ctx->num_sms - 1) * S->rb_per_sm, C->n_cells, nf, nnz_h, sv_elem_size(data->dtype));
         S->rb_order.alloc(nf);
         sv_launch(ctx, "scale_rb_order", k_rb_order, dim3((unsigned)((nf + 7) / 8)), dim3(256), 0,
                   (const int64_t*)S->feat_start.get(), (const int64_t*)S->feat_end.get(), nf, S->rb_order.get());
