@@ -1,7 +1,7 @@
-// Locality order of the points and per-block tile lists for the FP32 kNN search
-// (sv_knn.cu).
+// Locality order of the points and per-block tile lists for the exact kNN
+// searches (sv_knn.cu, sv_knn_tc.cu).
 //
-// The candidate kernel scans tiles of points for blocks of queries and may skip
+// The candidate kernels scan tiles of points for blocks of queries and may skip
 // a tile whose distance to the block exceeds every query's current threshold.
 // How many tiles that leaves depends on the order of the points.  Here every
 // point goes to the nearest of P of the points themselves (pivots, spread evenly
@@ -13,9 +13,13 @@
 // for its extent in every dimension, a projection once).  Each query block gets
 // its tiles sorted by the larger: the nearest first, so that thresholds fall at
 // once, and the first tile out of reach ends the scan.
-// (The tensor-core search keeps its order along the widest dimension: its
-// shortlists are per half tile of that order, and in another one a row in 10^5
-// shortlists another point where the BF16 keys misjudge a neighbour.)
+// (Along the widest dimension alone, 300,000 points in 60 clusters x 50
+// dimensions left most of the 1,172 tiles to be scanned.)
+// The tensor-core search shortlists the points of the two halves of its tiles
+// apart, and which points share a half decides which of them the BF16 keys may
+// misjudge.  There the halves are those of the tiles along the widest dimension
+// (halves_of), as they are for stacked samples; each half is ordered by itself, and
+// a tile takes the next part of both.
 #include "sv_internal.cuh"
 #include "sv_knn_order.cuh"
 
@@ -130,11 +134,13 @@ __global__ void __launch_bounds__(PV_MAX) k_pivots(const float* __restrict__ X, 
   }
 }
 
-// Sort key of every point: its nearest pivot's place, then its widest coordinate.
+// Sort key of every point: its half (if any), its nearest pivot's place, then its
+// widest coordinate.
 template <int DP>
 __global__ void __launch_bounds__(PV_THREADS) k_pivot_assign(const float* __restrict__ X, int64_t n,
                                                              const float* __restrict__ rows,
                                                              const float* __restrict__ norms, int P, int dim,
+                                                             const unsigned char* __restrict__ half,
                                                              unsigned long long* __restrict__ key,
                                                              int* __restrict__ val) {
   __shared__ __align__(16) float tile[PV_TILE * DP];
@@ -183,14 +189,33 @@ __global__ void __launch_bounds__(PV_THREADS) k_pivot_assign(const float* __rest
     }
   }
   if (i < n) {
-    key[i] = ((unsigned long long)best << 32) | ordered_bits(X[i * DP + dim]);
+    const unsigned place = (unsigned)best | (half && half[i] ? 0x80000000u : 0u);
+    key[i] = ((unsigned long long)place << 32) | ordered_bits(X[i * DP + dim]);
     val[i] = (int)i;
   }
 }
 
+// The half of the tiles (bp points) of an order that every point lies in.
+__global__ void k_halves(const int* __restrict__ perm, int64_t n, int bp, unsigned char* __restrict__ half) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    half[perm[i]] = (i % bp) >= bp / 2;
+}
+
+// Points sorted by half (n0 of the first) to tiles with a part of each: the i-th
+// point of a half is in tile i / (bp / 2).
+__global__ void k_join_halves(const int* __restrict__ in, int64_t n, int64_t n0, int bp, int* __restrict__ out) {
+  const int h = bp / 2;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t k = i < n0 ? i : i - n0;
+    out[k / h * bp + k % h + (i < n0 ? 0 : h)] = in[i];
+  }
+}
+
 // Bounding boxes of groups of `rows` consecutive rows (permuted), dimension-major
-// (lo[c * ng + g]).  mean, meant (optional): the groups' means, row-major with zero rows up to a multiple of 64 groups, and
+// (lo[c * ng + g]); BF16: of the rounded coordinates.  mean, meant (optional):
+// the groups' means, row-major with zero rows up to a multiple of 64 groups, and
 // dimension-major.
+template <bool BF16>
 __global__ void __launch_bounds__(256) k_boxes(const float* __restrict__ X, const int* __restrict__ perm,
                                                int64_t n, int dp, int rows, int64_t ng, float* __restrict__ lo,
                                                float* __restrict__ hi, float* __restrict__ mean,
@@ -201,7 +226,8 @@ __global__ void __launch_bounds__(256) k_boxes(const float* __restrict__ X, cons
   float a = FLT_MAX, b = -FLT_MAX, m = 0.f;
   const int64_t e = min(n, (g + 1) * rows);
   for (int64_t i = g * rows + r0; i < e; i += rs) {
-    const float v = X[(int64_t)perm[i] * dp + c];
+    float v = X[(int64_t)perm[i] * dp + c];
+    if (BF16) v = __bfloat162float(__float2bfloat16_rn(v));
     a = fminf(a, v);
     b = fmaxf(b, v);
     m += v;
@@ -259,7 +285,7 @@ __global__ void __launch_bounds__(1024) k_far(const float* __restrict__ lo, cons
 // tiles' projections on the line through their means is (sep_XY + sep_YX) /
 // |m_X - m_Y|.
 constexpr int SEP_THREADS = 256;
-template <int DP>
+template <int DP, bool BF16>
 __global__ void __launch_bounds__(SEP_THREADS) k_sep(const float* __restrict__ X, const int* __restrict__ perm,
                                                      int64_t n, int bp, int64_t nt,
                                                      const float* __restrict__ mean, float* __restrict__ sep) {
@@ -274,9 +300,12 @@ __global__ void __launch_bounds__(SEP_THREADS) k_sep(const float* __restrict__ X
     const int r = k % 64 + 64 * (k / (16 * DP)), c4 = k / 64 % (DP / 4);
     float4 v = make_float4(0, 0, 0, 0);
     if (i0 + r < n) v = *(const float4*)(X + (int64_t)perm[i0 + r] * DP + 4 * c4);
-    const float e[4] = {v.x, v.y, v.z, v.w};
+    float e[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-    for (int u = 0; u < 4; ++u) Q[((r >> 6) * DP + 4 * c4 + u) * 64 + (r & 63)] = e[u];
+    for (int u = 0; u < 4; ++u) {
+      if (BF16) e[u] = __bfloat162float(__float2bfloat16_rn(e[u]));
+      Q[((r >> 6) * DP + 4 * c4 + u) * 64 + (r & 63)] = e[u];
+    }
   }
   __syncthreads();
   for (int r = tid; r < bp; r += SEP_THREADS) {
@@ -417,7 +446,9 @@ int sv_knn_widest_dim(sv_context* ctx, const float* X32, int64_t n, int dp, int 
   return dim;
 }
 
-bool sv_knn_order(sv_context* ctx, const float* X32, int64_t n, int dp, int d, int bq, int bp, KnnOrder& o) {
+bool sv_knn_order(sv_context* ctx, const float* X32, int64_t n, int dp, int d, int bq, int bp, KnnOrder& o,
+                  const int* halves_of) {
+  const bool bf16 = halves_of != nullptr;
   const int64_t nq = (n + bq - 1) / bq, np = (n + bp - 1) / bp;
   // worth it from a few tiles up; the lists have to fit (sorted in shared memory,
   // kept in 1/4 of what the pool keeps: 4 GB, 4 M points)
@@ -433,12 +464,17 @@ bool sv_knn_order(sv_context* ctx, const float* X32, int64_t n, int dp, int d, i
   int64_t n2 = 2048;
   while (n2 < n) n2 <<= 1;
   DevBuf<unsigned long long> key(n2);
+  DevBuf<unsigned char> half;
+  if (halves_of) {
+    half.alloc(n);
+    sv_launch(ctx, "knn_halves", k_halves, dim3(sv_grid_for(ctx, n, 256)), dim3(256), 0, halves_of, n, bp, half.get());
+  }
   o.perm.alloc(n2);
   const dim3 ga((unsigned)((n + PV_THREADS - 1) / PV_THREADS));
 #define PV_CASE(D)                                                                                       \
   case D:                                                                                                \
     sv_launch(ctx, "knn_assign", k_pivot_assign<D>, ga, dim3(PV_THREADS), 0, X32, n, (const float*)rows.get(), \
-              (const float*)norms.get(), P, dim, key.get(), o.perm.get());                              \
+              (const float*)norms.get(), P, dim, (const unsigned char*)half.get(), key.get(), o.perm.get());                              \
     break;
   switch (dp) {
     PV_CASE(8) PV_CASE(16) PV_CASE(24) PV_CASE(32) PV_CASE(40) PV_CASE(48) PV_CASE(56) PV_CASE(64)
@@ -446,13 +482,21 @@ bool sv_knn_order(sv_context* ctx, const float* X32, int64_t n, int dp, int d, i
   }
 #undef PV_CASE
   sv_sort_pairs(ctx, key.get(), o.perm.get(), n, n2);
+  if (halves_of) {
+    DevBuf<int> joined(n);
+    const int64_t n0 = n / bp * (bp / 2) + std::min<int64_t>(n % bp, bp / 2);
+    sv_launch(ctx, "knn_join_halves", k_join_halves, dim3(sv_grid_for(ctx, n, 256)), dim3(256), 0,
+              (const int*)o.perm.get(), n, n0, bp, joined.get());
+    o.perm = std::move(joined);
+  }
   DevBuf<float> ql((size_t)nq * dp), qh((size_t)nq * dp), pl((size_t)np * dp), ph((size_t)np * dp);
   DevBuf<float> mean((size_t)npad * dp), meant((size_t)np * dp), sep((size_t)(np * np)), rmax(1);
+  auto boxes = bf16 ? k_boxes<true> : k_boxes<false>;
   const dim3 bt(256 / dp * dp);
   const int* pm = o.perm.get();
-  sv_launch(ctx, "knn_boxes", k_boxes, dim3((unsigned)nq), bt, 0, X32, pm, n, dp, bq, nq, ql.get(), qh.get(),
+  sv_launch(ctx, "knn_boxes", boxes, dim3((unsigned)nq), bt, 0, X32, pm, n, dp, bq, nq, ql.get(), qh.get(),
             (float*)nullptr, (float*)nullptr);
-  sv_launch(ctx, "knn_boxes", k_boxes, dim3((unsigned)npad), bt, 0, X32, pm, n, dp, bp, np, pl.get(), ph.get(),
+  sv_launch(ctx, "knn_boxes", boxes, dim3((unsigned)npad), bt, 0, X32, pm, n, dp, bp, np, pl.get(), ph.get(),
             mean.get(), meant.get());
   sv_launch(ctx, "knn_far", k_far, dim3(1), dim3(1024), 0, (const float*)pl.get(), (const float*)ph.get(), np, dp,
             rmax.get());
@@ -460,8 +504,9 @@ bool sv_knn_order(sv_context* ctx, const float* X32, int64_t n, int dp, int d, i
   const dim3 gs((unsigned)np, (unsigned)std::max<int64_t>(1, std::min<int64_t>(npad / 64, 1 + 8 * ctx->num_sms / np)));
 #define SEP_CASE(D)                                                                                       \
   case D: {                                                                                               \
-    SV_CUDA(cudaFuncSetAttribute(k_sep<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm));       \
-    sv_launch(ctx, "knn_sep", k_sep<D>, gs, dim3(SEP_THREADS), ssm, X32, pm, n, bp, np, (const float*)mean.get(), \
+    auto kern = bf16 ? k_sep<D, true> : k_sep<D, false>;                                                  \
+    SV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm));           \
+    sv_launch(ctx, "knn_sep", kern, gs, dim3(SEP_THREADS), ssm, X32, pm, n, bp, np, (const float*)mean.get(), \
               sep.get());                                                                                 \
     break;                                                                                                \
   }

@@ -20,7 +20,10 @@ __device__ __forceinline__ int knn_list_tile(unsigned long long e, int own) {
 }
 
 // Orders the points and lists the tiles (bp points) of every block of bq queries;
-// false when the input is too small or too large for it.
-bool sv_knn_order(sv_context* ctx, const float* X32, int64_t n, int dp, int d, int bq, int bp, KnnOrder& o);
+// false when the input is too small or too large for it.  halves_of: an order (place
+// -> point) whose tiles' halves are kept, for BF16 operands: bounds of the rounded
+// coordinates; bp is even.
+bool sv_knn_order(sv_context* ctx, const float* X32, int64_t n, int dp, int d, int bq, int bp, KnnOrder& o,
+                  const int* halves_of = nullptr);
 // the dimension of largest variance
 int sv_knn_widest_dim(sv_context* ctx, const float* X32, int64_t n, int dp, int d);

@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(THREADS, 1)
              const float* __restrict__ sqpad, int64_t n, int ntiles, int32_t* __restrict__ cand,
              int* __restrict__ status, const int64_t* __restrict__ sched, int around,
              const float* __restrict__ coord, const float* __restrict__ nrm,
-             const unsigned* __restrict__ pmax) {
+             const unsigned* __restrict__ pmax, const unsigned long long* __restrict__ lists) {
   extern __shared__ unsigned char smem_raw[];
   Smem* s = (Smem*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -238,7 +238,9 @@ __global__ void __launch_bounds__(THREADS, 1)
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    // Chooses the tile sequence.  With the points in locality order (coord: the
+    // Chooses the tile sequence.  With a list of the tiles by their lower bound
+    // (sv_knn_order) it follows the list to the first tile beyond every query's
+    // current threshold.  With the points in locality order (coord: the
     // sort coordinate of every point, as the BF16 operand holds it) a tile whose
     // coordinate gap to this CTA's queries already exceeds every query's
     // current threshold is skipped, and so is every tile beyond it: the squared
@@ -249,6 +251,8 @@ __global__ void __launch_bounds__(THREADS, 1)
       mbar_expect_tx(&s->abar, BM * BK * 2);
       tma_load_2d(s->A, &tmapA, 0, (int)q0, &s->abar);
       const bool prune = coord != nullptr;
+      const unsigned long long* list = lists ? lists + (int64_t)blockIdx.x * ntiles : nullptr;
+      unsigned long long ent = list ? list[0] : 0;   // loaded one step ahead of its use
       float qlo = 0.f, qhi = 0.f;
       if (prune) {
         int64_t ql = q0 + BM < qend ? q0 + BM : qend;
@@ -268,7 +272,17 @@ __global__ void __launch_bounds__(THREADS, 1)
       int t = 0;
       for (;; ++t) {
         int tile;
-        if (!prune) {
+        if (list) {
+          if (t >= ntiles) break;
+          const unsigned long long e = ent;
+          if (t + 1 < ntiles) ent = list[t + 1];
+          volatile float* wm = s->wmax;
+          float T = wm[0];
+#pragma unroll
+          for (int w = 1; w < EPI_WARPS; ++w) T = fmaxf(T, wm[w]);
+          if (knn_list_bound(e) > T) break;
+          tile = knn_list_tile(e, t0);
+        } else if (!prune) {
           if (t >= ntiles) break;
           tile = tile_at(t, t0, ntiles, around);
         } else if (t == 0) {
@@ -388,7 +402,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     // pruning bound of this query: threshold + |q|^2 + a margin for the FP32
     // accumulation of the MMA (2^-15 (|q|^2 + max |p|^2), several times its bound)
     float qn = 0.f;
-    if (coord && q < qend) qn = nrm[q] + 0x1p-15f * (nrm[q] + __uint_as_float(*pmax));
+    if (nrm && q < qend) qn = nrm[q] + 0x1p-15f * (nrm[q] + __uint_as_float(*pmax));
     for (int t = 0;; ++t) {
       int ab = t & 1;
       uint32_t aph = (t >> 1) & 1;
@@ -460,10 +474,11 @@ __global__ void __launch_bounds__(THREADS, 1)
           }
         }
       }
-      if (coord && (t & 3) == 3) {
-        // every fourth tile; keys only fall, so a stale (larger) bound read by
+      if (lists || (coord && (t & 3) == 3)) {
+        // every fourth tile (every tile of a list); keys only fall, so a stale (larger) bound read by
         // the producer is safe
         float v = q < qend ? best[KH - 1] + qn : -FLT_MAX;
+        if (v != v) v = __int_as_float(0x7f800000);   // no bound from a NaN
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
         if (lane == 0) ((volatile float*)s->wmax)[ew] = v;
@@ -554,8 +569,8 @@ __global__ void k_pack_fold(const float* __restrict__ X, int64_t n, int dp, int 
     }
     if (!on) continue;
     if (part == 0) {
-      if (coord) {
-        coord[i] = __bfloat162float(__float2bfloat16_rn(X[src * dp + dim]));
+      if (coord) coord[i] = __bfloat162float(__float2bfloat16_rn(X[src * dp + dim]));
+      if (nrm) {
         nrm[i] = s;
         atomicMax(pmax, __float_as_uint(s));
       }
@@ -581,7 +596,7 @@ __global__ void k_pack_fold(const float* __restrict__ X, int64_t n, int dp, int 
   }
 }
 
-// ---- locality order of the points ----------------------------------------------
+// ---- order along the widest dimension (stacked samples, very many points) --------
 // sort key: sample in the high word, the coordinate (order-preserving bits) low
 __global__ void k_locality_keys(const float* __restrict__ X, int dp, int dim, const int64_t* __restrict__ off,
                                 int nseg, int64_t n, unsigned long long* __restrict__ key, int* __restrict__ val) {
@@ -647,13 +662,20 @@ int sv_knn_tc_candidates(sv_context* ctx, const float* X32, const float* sq_unus
                 segs ? (const int64_t*)doff.get() : (const int64_t*)nullptr, nseg, n, key.get(), perm.get());
       sv_sort_pairs(ctx, key.get(), perm.get(), n, n2);
     }
+    // one set of points: each half of the tiles by cells of pivots, and tile lists
+    // (300,000 clustered points in 50 dimensions: tiles 14.5 -> 5.3 ms, the order
+    // and the lists 2.3 ms; 10,000 points: 1.12 -> 0.87 ms in all); stacked samples
+    // (a CTA sees its own sample's tiles only): as they are
+    KnnOrder ord;
+    const bool listed = prune && !segs && sv_knn_order(ctx, X32, n, dp, d, BM, BN, ord, perm.get());
+    if (listed) perm = std::move(ord.perm);
     const int* pm = around ? (const int*)perm.get() : (const int*)nullptr;
     DevBuf<__nv_bfloat16> Xq((size_t)n * BK), Xp;
     DevBuf<float> sq(npad);
     DevBuf<float> coord, nrm;
     DevBuf<unsigned> pmax;
     if (prune) {
-      coord.alloc(n);
+      if (!listed) coord.alloc(n);
       nrm.alloc(n);
       pmax.alloc(1);
       sv_memset(ctx, pmax.get(), 0, sizeof(unsigned));
@@ -708,7 +730,8 @@ int sv_knn_tc_candidates(sv_context* ctx, const float* X32, const float* sq_unus
                                  (int)smem));                                                       \
     sv_launch(ctx, "knn_tc_tiles", k_knn_tc<FOLD, KHV>, dim3(nblocks), dim3(THREADS), smem, tmapA,   \
               tmapB, (const float*)sq.get(), n, ntiles, cout, ctx->d_status,                        \
-              (const int64_t*)sched.get(), (int)around, CO, NR, PM);                               \
+              (const int64_t*)sched.get(), (int)around, CO, NR, PM,                           \
+              listed ? (const unsigned long long*)ord.lists.get() : (const unsigned long long*)nullptr);   \
   } while (0)
     // 20 candidates per column half (40 per query) for k <= 20, else 32
     if (fold) {
