@@ -212,6 +212,43 @@ k_moments_part(const ValT* __restrict__ val, const int64_t* __restrict__ cs,
     double S1 = 0.0, S2 = 0.0;
     DfAcc acc;
     const int64_t va = (a + N - 1) / N, vb = b / N;   // whole 16-byte vectors in [a, b)
+    if constexpr (sizeof(ValT) == 4 && !V::DF) {
+      // Counts below 2^15 (a part's squares then sum to less than 2^45): every FP64
+      // partial sum is an exact integer, whatever the order, and integers give the
+      // same sums without the FP64 pipe (60 M counts: 0.51 -> 0.14 ms)
+      long long i1 = 0, i2 = 0;
+      bool small = true;
+      auto take = [&](int c) {
+        small = small && (unsigned)(c + 32768) < 65536u;
+        i1 += c;
+        i2 += (long long)c * c;
+      };
+      for (int64_t i = a + lane; i < min(b, va * N); i += 32) take(val[i]);
+      if (va < vb) {
+        for (int64_t i = vb * N + lane; i < b; i += 32) take(val[i]);
+        const int4* vp = reinterpret_cast<const int4*>(val);
+        for (int64_t v0 = va + lane; v0 < vb; v0 += 32 * MOM_UNROLL) {
+          int4 w[MOM_UNROLL];
+#pragma unroll
+          for (int u = 0; u < MOM_UNROLL; ++u) w[u] = v0 + 32 * u < vb ? __ldg(vp + v0 + 32 * u) : make_int4(0, 0, 0, 0);
+#pragma unroll
+          for (int u = 0; u < MOM_UNROLL; ++u) {
+            take(w[u].x);
+            take(w[u].y);
+            take(w[u].z);
+            take(w[u].w);
+          }
+        }
+      } else {
+        for (int64_t i = max(a, va * N) + lane; i < b; i += 32) take(val[i]);
+      }
+      if (__all_sync(0xffffffffu, small)) {
+        i1 = sv_warp_sum(i1);
+        i2 = sv_warp_sum(i2);
+        if (lane == 0) part[task] = make_double2((double)i1, (double)i2);
+        continue;
+      }
+    }
     if (va < vb) {
       // head [a, va*N) and tail [vb*N, b): fewer than N elements each
       if (lane < va * N - a) V::scalar(val, a + lane, acc, S1, S2);
