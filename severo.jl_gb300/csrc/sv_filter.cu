@@ -40,63 +40,136 @@ __global__ void k_filter_cells(const int64_t* __restrict__ rowptr, const int32_t
   }
 }
 
-// one warp per gene over the CSC copy: cells (kept, count > 0) and kept entries
-__global__ void k_filter_genes(const int64_t* __restrict__ colptr, const int32_t* __restrict__ rowidx,
-                               const int32_t* __restrict__ cnt, int64_t n_genes,
-                               const unsigned char* __restrict__ cell_keep, int64_t min_cells,
-                               unsigned char* __restrict__ keep, int64_t* __restrict__ keep64,
-                               int64_t* __restrict__ newlen) {
-  int lane = threadIdx.x & 31;
-  int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t g = warp; g < n_genes; g += nwarps) {
-    int64_t s = colptr[g], e = colptr[g + 1];
-    long long cells = 0, kept = 0;
-    for (int64_t i = s + lane; i < e; i += 32) {
-      bool k = cell_keep[rowidx[i]];
-      kept += k;
-      cells += k && cnt[i] > 0;
+// A gene's entries are up to n_cells long and most genes have few: a block of
+// FG_WARPS warps per gene, FG_FLIGHT entries per thread in flight (a warp per gene
+// walked the longest columns alone, one round trip per 32 entries: 60 M entries of
+// 30,000 cells, 33,538 genes, k_filter_genes 0.58 -> 0.22 ms, k_filter_write 1.55 -> 0.25
+// ms).
+constexpr int FG_WARPS = 4;
+constexpr int FG_THREADS = FG_WARPS * 32;
+constexpr int FG_FLIGHT = 8;
+
+// per gene over the CSC copy: cells (kept, count > 0) and kept entries
+__global__ void __launch_bounds__(FG_THREADS) k_filter_genes(
+    const int64_t* __restrict__ colptr, const int32_t* __restrict__ rowidx, const int32_t* __restrict__ cnt,
+    int64_t n_genes, const unsigned char* __restrict__ cell_keep, int64_t min_cells,
+    unsigned char* __restrict__ keep, int64_t* __restrict__ keep64, int64_t* __restrict__ newlen) {
+  __shared__ int part[2][FG_WARPS][2];   // by turns of genes
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int turn = 0;
+  for (int64_t g = blockIdx.x; g < n_genes; g += gridDim.x, turn ^= 1) {
+    const int64_t s = colptr[g], e = colptr[g + 1];
+    int cells = 0, kept = 0;
+    for (int64_t i0 = s + threadIdx.x; i0 < e; i0 += FG_FLIGHT * FG_THREADS) {
+      int32_t r[FG_FLIGHT], v[FG_FLIGHT];
+#pragma unroll
+      for (int u = 0; u < FG_FLIGHT; ++u) {
+        const int64_t i = i0 + u * FG_THREADS;
+        r[u] = i < e ? rowidx[i] : -1;
+        v[u] = i < e ? cnt[i] : 0;
+      }
+#pragma unroll
+      for (int u = 0; u < FG_FLIGHT; ++u) {
+        const bool k = r[u] >= 0 && cell_keep[r[u]];
+        kept += k;
+        cells += k && v[u] > 0;
+      }
     }
     cells = sv_warp_sum(cells);
     kept = sv_warp_sum(kept);
     if (lane == 0) {
-      bool k = cells >= min_cells;
+      part[turn][w][0] = cells;
+      part[turn][w][1] = kept;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int64_t tc = 0, tk = 0;
+#pragma unroll
+      for (int o = 0; o < FG_WARPS; ++o) {
+        tc += part[turn][o][0];
+        tk += part[turn][o][1];
+      }
+      const bool k = tc >= min_cells;
       keep[g] = k;
       keep64[g] = k;
-      newlen[g] = k ? kept : 0;
+      newlen[g] = k ? tk : 0;
     }
   }
 }
 
-// one warp per kept gene: copy its kept entries in order (warp ballot
-// compaction), rows renumbered; writes the new column pointer
-__global__ void k_filter_write(const int64_t* __restrict__ colptr, const int32_t* __restrict__ rowidx,
-                               const int32_t* __restrict__ cnt, int64_t n_genes,
-                               const unsigned char* __restrict__ cell_keep,
-                               const int64_t* __restrict__ cell_new,
-                               const unsigned char* __restrict__ gene_keep,
-                               const int64_t* __restrict__ gene_new, const int64_t* __restrict__ start,
-                               int64_t* __restrict__ out_colptr, int32_t* __restrict__ out_row,
-                               int32_t* __restrict__ out_cnt) {
-  int lane = threadIdx.x & 31;
-  int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t g = warp; g < n_genes; g += nwarps) {
+// per kept gene: its kept entries in order, rows renumbered; the new column
+// pointer.  A warp takes a quarter of the column; where every entry is kept they
+// go straight to their places, else the quarters are counted first (warp ballot
+// compaction).
+__global__ void __launch_bounds__(FG_THREADS) k_filter_write(
+    const int64_t* __restrict__ colptr, const int32_t* __restrict__ rowidx, const int32_t* __restrict__ cnt,
+    int64_t n_genes, const unsigned char* __restrict__ cell_keep, const int64_t* __restrict__ cell_new,
+    const unsigned char* __restrict__ gene_keep, const int64_t* __restrict__ gene_new,
+    const int64_t* __restrict__ start, int64_t* __restrict__ out_colptr, int32_t* __restrict__ out_row,
+    int32_t* __restrict__ out_cnt) {
+  __shared__ int part[FG_WARPS];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int64_t g = blockIdx.x; g < n_genes; g += gridDim.x) {
     if (!gene_keep[g]) continue;
     int64_t dst = start[g];
-    if (lane == 0) out_colptr[gene_new[g]] = dst;
-    int64_t s = colptr[g], e = colptr[g + 1];
-    for (int64_t b = s; b < e; b += 32) {
-      int64_t i = b + lane;
-      int32_t r = i < e ? rowidx[i] : 0;
-      bool k = i < e && cell_keep[r];
-      unsigned m = __ballot_sync(0xffffffffu, k);
-      if (k) {
-        int64_t o = dst + __popc(m & ((1u << lane) - 1u));
-        out_row[o] = (int32_t)cell_new[r];
-        out_cnt[o] = cnt[i];
+    if (threadIdx.x == 0) out_colptr[gene_new[g]] = dst;
+    const int64_t s = colptr[g], e = colptr[g + 1];
+    if (start[g + 1] - dst == e - s) {
+      for (int64_t i0 = s + threadIdx.x; i0 < e; i0 += FG_FLIGHT * FG_THREADS) {
+        int32_t r[FG_FLIGHT], v[FG_FLIGHT];
+#pragma unroll
+        for (int u = 0; u < FG_FLIGHT; ++u) {
+          const int64_t i = i0 + u * FG_THREADS;
+          if (i < e) {
+            r[u] = rowidx[i];
+            v[u] = cnt[i];
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < FG_FLIGHT; ++u) {
+          const int64_t i = i0 + u * FG_THREADS;
+          if (i < e) {
+            out_row[dst + (i - s)] = (int32_t)cell_new[r[u]];
+            out_cnt[dst + (i - s)] = v[u];
+          }
+        }
       }
-      dst += __popc(m);
+      continue;
+    }
+    const int64_t q = ((e - s + FG_THREADS - 1) / FG_THREADS) * 32;   // entries of a warp's part
+    const int64_t a = s + w * q, b = min(e, a + q);
+    int kept = 0;
+    for (int64_t i0 = a + lane; i0 < b; i0 += FG_FLIGHT * 32) {
+      int32_t r[FG_FLIGHT];
+#pragma unroll
+      for (int u = 0; u < FG_FLIGHT; ++u) r[u] = i0 + 32 * u < b ? rowidx[i0 + 32 * u] : -1;
+#pragma unroll
+      for (int u = 0; u < FG_FLIGHT; ++u) kept += r[u] >= 0 && cell_keep[r[u]];
+    }
+    kept = sv_warp_sum(kept);
+    __syncthreads();                       // the last gene's parts are read
+    if (lane == 0) part[w] = kept;
+    __syncthreads();
+    for (int o = 0; o < w; ++o) dst += part[o];
+    for (int64_t i0 = a; i0 < b; i0 += 4 * 32) {
+      int32_t r[4], v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int64_t i = i0 + 32 * u + lane;
+        r[u] = i < b ? rowidx[i] : -1;
+        v[u] = i < b ? cnt[i] : 0;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const bool k = r[u] >= 0 && cell_keep[r[u]];
+        const unsigned m = __ballot_sync(0xffffffffu, k);
+        if (k) {
+          const int64_t o = dst + __popc(m & ((1u << lane) - 1u));
+          out_row[o] = (int32_t)cell_new[r[u]];
+          out_cnt[o] = v[u];
+        }
+        dst += __popc(m);
+      }
     }
   }
 }
@@ -112,7 +185,7 @@ static sv_counts* compact(sv_context* ctx, const sv_counts* A, DevBuf<unsigned c
   const int64_t nc = A->n_cells, ng = A->n_genes;
   DevBuf<int64_t> cnew(nc + 1), gk64(ng + 1), gnew(ng + 1), glen(ng + 1), gstart(ng + 1);
   sv_scan_i64(ctx, ck64.get(), cnew.get(), nc);
-  sv_launch(ctx, "filter_genes", k_filter_genes, dim3(sv_grid_for(ctx, ng * 32, 256)), dim3(256), 0,
+  sv_launch(ctx, "filter_genes", k_filter_genes, dim3(sv_grid_for(ctx, ng, 1, 16)), dim3(FG_THREADS), 0,
             (const int64_t*)A->csc_colptr.get(), (const int32_t*)A->csc_rowidx.get(),
             (const int32_t*)A->csc_count.get(), ng, (const unsigned char*)ckeep.get(), min_cells,
             gkeep.get(), gk64.get(), glen.get());
@@ -130,7 +203,7 @@ static sv_counts* compact(sv_context* ctx, const sv_counts* A, DevBuf<unsigned c
     c->csc_colptr.alloc(ng2 + 1);
     c->csc_rowidx.alloc(std::max<int64_t>(1, nnz2));
     c->csc_count.alloc(std::max<int64_t>(1, nnz2));
-    sv_launch(ctx, "filter_write", k_filter_write, dim3(sv_grid_for(ctx, ng * 32, 256)), dim3(256), 0,
+    sv_launch(ctx, "filter_write", k_filter_write, dim3(sv_grid_for(ctx, ng, 1, 16)), dim3(FG_THREADS), 0,
               (const int64_t*)A->csc_colptr.get(), (const int32_t*)A->csc_rowidx.get(),
               (const int32_t*)A->csc_count.get(), ng, (const unsigned char*)ckeep.get(),
               (const int64_t*)cnew.get(), (const unsigned char*)gkeep.get(), (const int64_t*)gnew.get(),
