@@ -21,6 +21,7 @@
 // The kd-tree (a few dozen vertices) is built on the host from the sorted x;
 // the fits and the blend run on the device.
 #include "sv_internal.cuh"
+#include <limits.h>
 #include <math.h>
 
 void sv_count_moments(sv_context* ctx, const sv_counts* C, double* mean, double* sd);
@@ -182,13 +183,93 @@ std::vector<double> loess_kdtree_bounds(const std::vector<double>& xs, double sp
   return b;
 }
 
+// ---- ranks: a stable sort of up to VST_RANK_MAX values ------------------------------
+// rank[i] = values before the i-th in the order, equal ones by index: every pair is
+// compared, as ordered integers (33,538 values: 0.19 ms, with std::stable_sort and
+// std::partial_sort on the host feature selection took 2.4 ms more; the work grows with the square, the sort's not: beyond VST_RANK_MAX
+// the host sorts).  NaN has no place: the caller looks for it.
+constexpr int64_t VST_RANK_MAX = 1 << 17;
+constexpr int RANK_THREADS = 256, RANK_TILE = 1024;
+
+__global__ void k_rank_keys(const double* __restrict__ v, int64_t n, int descending,
+                            unsigned long long* __restrict__ key, int* __restrict__ rank) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    unsigned long long u = (unsigned long long)__double_as_longlong(v[i] + 0.0);   // -0 is 0
+    u = (u >> 63) ? ~u : u | (1ull << 63);
+    key[i] = descending ? ~u : u;
+    rank[i] = 0;
+  }
+}
+
+__global__ void __launch_bounds__(RANK_THREADS) k_rank(const unsigned long long* __restrict__ key, int64_t n,
+                                                       int* __restrict__ rank) {
+  __shared__ __align__(16) unsigned long long tile[RANK_TILE];
+  const int64_t i = blockIdx.x * (int64_t)RANK_THREADS + threadIdx.x;
+  const unsigned long long k = i < n ? key[i] : 0;
+  int r = 0;
+  for (int64_t j0 = (int64_t)blockIdx.y * RANK_TILE; j0 < n; j0 += (int64_t)gridDim.y * RANK_TILE) {
+    __syncthreads();
+    for (int t = threadIdx.x; t < RANK_TILE; t += RANK_THREADS) tile[t] = j0 + t < n ? key[j0 + t] : ~0ull;
+    __syncthreads();
+    // positions below before: those with an equal key count
+    const int before = (int)min((int64_t)RANK_TILE, max((int64_t)0, i - j0));
+    const int len = (int)min((int64_t)RANK_TILE, n - j0);
+    if (before == 0 || before >= len) {
+      const unsigned long long lim = before == 0 ? k : k + 1;   // no key is all ones but NaN's
+#pragma unroll 8
+      for (int t = 0; t < len; ++t) r += tile[t] < lim;
+    } else {
+      for (int t = 0; t < len; ++t) r += tile[t] < k || (tile[t] == k && t < before);
+    }
+  }
+  if (i < n && r) atomicAdd(rank + i, r);
+}
+
+__global__ void k_rank_scatter(const int* __restrict__ rank, int64_t n, const double* __restrict__ a,
+                               const double* __restrict__ b, double* __restrict__ as, double* __restrict__ bs) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    as[rank[i]] = a[i];
+    bs[rank[i]] = b[i];
+  }
+}
+
+__global__ void k_rank_gather(const int* __restrict__ rank, int64_t n, const double* __restrict__ s,
+                              double* __restrict__ o) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    o[i] = s[rank[i]];
+}
+
+__global__ void k_rank_first(const int* __restrict__ rank, int64_t n, int64_t m, int64_t* __restrict__ first) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    if (rank[i] < m) first[rank[i]] = i + 1;
+}
+
+void launch_ranks(sv_context* ctx, const double* v, int64_t n, bool descending, int* rank) {
+  DevBuf<unsigned long long> key(n);
+  sv_launch(ctx, "vst_rank", k_rank_keys, dim3(sv_grid_for(ctx, n, 256)), dim3(256), 0, v, n, (int)descending,
+            key.get(), rank);
+  const int64_t nb = (n + RANK_THREADS - 1) / RANK_THREADS, nt = (n + RANK_TILE - 1) / RANK_TILE;
+  const int64_t ny = std::max<int64_t>(1, std::min<int64_t>(nt, 16 * ctx->num_sms / nb));
+  sv_launch(ctx, "vst_rank", k_rank, dim3((unsigned)nb, (unsigned)ny), dim3(RANK_THREADS), 0,
+            (const unsigned long long*)key.get(), n, rank);
+}
+
 // one warp per gene: sum of min((x - mu) / esd, vmax)^2 over the stored
 // counts plus the implicit zeros' share, / (n - 1).  The square depends on the
 // count only: lane l holds it for the count l + 1, and a stored count in
-// 1..32 (nearly all of them) reads it from that lane instead of dividing.
-__global__ void k_vst_var(const int64_t* __restrict__ colptr, const int32_t* __restrict__ cnt,
+// 1..32 (nearly all of them) reads it from that lane instead of dividing.  A gene
+// with larger counts leaves squares up to its largest, VAR_TABLE at most, in shared
+// memory as they come up: the few genes with most counts above 32 divided once per
+// entry, one after the other, and the kernel waited for them (60 M entries of 33,538
+// genes: 0.95 -> 0.34 ms; the FP64 pipe needs 0.11 for the additions alone).
+constexpr int VAR_FLIGHT = 8;
+constexpr int VAR_THREADS = 256;
+constexpr int VAR_TABLE = 512;
+__global__ void __launch_bounds__(VAR_THREADS) k_vst_var(const int64_t* __restrict__ colptr, const int32_t* __restrict__ cnt,
                           int64_t n_genes, int64_t n_cells, const double* __restrict__ mu,
                           const double* __restrict__ esd, double vmax, double* __restrict__ out) {
+  __shared__ double table[VAR_THREADS / 32][VAR_TABLE];
+  double* sq = table[threadIdx.x >> 5];
   int lane = threadIdx.x & 31;
   int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -203,15 +284,40 @@ __global__ void k_vst_var(const int64_t* __restrict__ colptr, const int32_t* __r
     double tab = zl * zl;
     int64_t s = colptr[g], t = colptr[g + 1];
     double acc = 0;
-    for (int64_t b = s; b < t; b += 32) {   // every lane runs every round (the shuffle)
-      int64_t i = b + lane;
-      int c = i < t ? cnt[i] : 1;
-      double z2 = __shfl_sync(0xffffffffu, tab, (int)(((unsigned)c - 1u) & 31u));
-      if (c < 1 || c > 32) {
-        double z = fmin(((double)c - m) / e, vmax);
-        z2 = z * z;
+    int filled = 0;                         // counts in the table of the shared memory
+    __syncwarp();
+    // every lane runs every round (the shuffle); VAR_FLIGHT loads in flight
+    for (int64_t b = s; b < t; b += 32 * VAR_FLIGHT) {
+      int c[VAR_FLIGHT];
+#pragma unroll
+      for (int u = 0; u < VAR_FLIGHT; ++u) c[u] = b + 32 * u + lane < t ? cnt[b + 32 * u + lane] : 1;
+      int most = 0;
+#pragma unroll
+      for (int u = 0; u < VAR_FLIGHT; ++u) most = max(most, c[u] < 1 ? INT_MAX : c[u]);
+      most = __reduce_max_sync(0xffffffffu, most);
+      double z2[VAR_FLIGHT];
+      if (most <= 32) {
+#pragma unroll
+        for (int u = 0; u < VAR_FLIGHT; ++u) z2[u] = __shfl_sync(0xffffffffu, tab, c[u] - 1);
+      } else {
+        for (; filled < min(most, VAR_TABLE); filled += 32) {
+          const double z = fmin(((double)(filled + lane + 1) - m) / e, vmax);
+          sq[filled + lane] = z * z;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < VAR_FLIGHT; ++u) {
+          if (c[u] >= 1 && c[u] <= VAR_TABLE) {
+            z2[u] = sq[c[u] - 1];
+          } else {
+            const double z = fmin(((double)c[u] - m) / e, vmax);
+            z2[u] = z * z;
+          }
+        }
       }
-      if (i < t) acc += z2;
+#pragma unroll
+      for (int u = 0; u < VAR_FLIGHT; ++u)
+        if (b + 32 * u + lane < t) acc += z2[u];
     }
     acc = sv_warp_sum(acc);
     if (lane == 0) {
@@ -252,19 +358,41 @@ SV_API int sv_find_variable_features_vst_surface(sv_context* ctx, const sv_count
       lx[i] = log10(hm[nc[i]]);
       ly[i] = log10(hs[nc[i]]);
     }
-    std::vector<int64_t> ord(n);
-    for (int64_t i = 0; i < n; ++i) ord[i] = i;
-    std::stable_sort(ord.begin(), ord.end(), [&](int64_t a, int64_t b) { return lx[a] < lx[b]; });
-    std::vector<double> xs(n), ys(n), fit(n);
-    for (int64_t i = 0; i < n; ++i) {
-      xs[i] = lx[ord[i]];
-      ys[i] = ly[ord[i]];
+    // xs, ys: in the order of lx
+    bool ranked = n <= VST_RANK_MAX;
+    for (int64_t i = 0; i < n && ranked; ++i) ranked = lx[i] == lx[i];
+    DevBuf<double> dx(n), dy(n), df(n);
+    DevBuf<int> rank;
+    std::vector<double> xs;
+    std::vector<int64_t> ord;
+    if (ranked) {
+      DevBuf<double> ux(n), uy(n);
+      rank.alloc(n);
+      sv_h2d(ctx, ux.get(), lx.data(), n * 8);
+      sv_h2d(ctx, uy.get(), ly.data(), n * 8);
+      launch_ranks(ctx, ux.get(), n, false, rank.get());
+      sv_launch(ctx, "vst_rank", k_rank_scatter, dim3(sv_grid_for(ctx, n, 256)), dim3(256), 0,
+                (const int*)rank.get(), n, (const double*)ux.get(), (const double*)uy.get(), dx.get(), dy.get());
+      if (surface != SV_LOESS_DIRECT) {
+        xs.resize(n);
+        sv_d2h(ctx, xs.data(), dx.get(), n * 8);
+      }
+    } else {
+      ord.resize(n);
+      for (int64_t i = 0; i < n; ++i) ord[i] = i;
+      std::stable_sort(ord.begin(), ord.end(), [&](int64_t a, int64_t b) { return lx[a] < lx[b]; });
+      std::vector<double> ys(n);
+      xs.resize(n);
+      for (int64_t i = 0; i < n; ++i) {
+        xs[i] = lx[ord[i]];
+        ys[i] = ly[ord[i]];
+      }
+      sv_h2d(ctx, dx.get(), xs.data(), n * 8);
+      sv_h2d(ctx, dy.get(), ys.data(), n * 8);
     }
+    std::vector<double> fit(n);
     int64_t q = std::max<int64_t>(3, std::min<int64_t>(n, (int64_t)floor((double)n * loess_span)));
     if (q > n) q = n;
-    DevBuf<double> dx(n), dy(n), df(n);
-    sv_h2d(ctx, dx.get(), xs.data(), n * 8);
-    sv_h2d(ctx, dy.get(), ys.data(), n * 8);
     if (surface == SV_LOESS_DIRECT) {
       sv_launch(ctx, "vst_loess", k_loess, dim3(sv_grid_for(ctx, n, 1, 8)), dim3(LOESS_THREADS), 0,
                 (const double*)dx.get(), (const double*)dy.get(), n, q, (const double*)dx.get(), n, 0,
@@ -281,15 +409,18 @@ SV_API int sv_find_variable_features_vst_surface(sv_context* ctx, const sv_count
                 (const double*)dx.get(), n, (const double*)db.get(), nb, (const double*)dv.get(),
                 (const double*)ds.get(), surface == SV_LOESS_HERMITE ? 1 : 0, df.get());
     }
-    sv_d2h(ctx, fit.data(), df.get(), n * 8);
+    if (ranked)   // back to the genes' order
+      sv_launch(ctx, "vst_rank", k_rank_gather, dim3(sv_grid_for(ctx, n, 256)), dim3(256), 0,
+                (const int*)rank.get(), n, (const double*)df.get(), dy.get());
+    sv_d2h(ctx, fit.data(), ranked ? dy.get() : df.get(), n * 8);
     for (int64_t i = 0; i < n; ++i) {
       double e = pow(10.0, fit[i]);
-      esd[nc[ord[i]]] = std::isnan(e) ? 0.0 : e;   // variablefeatures.jl:46-47
+      esd[nc[ranked ? i : ord[i]]] = std::isnan(e) ? 0.0 : e;   // variablefeatures.jl:46-47
     }
   }
   DevBuf<double> desd(ng), dout(ng);
   sv_h2d(ctx, desd.get(), esd.data(), ng * 8);
-  sv_launch(ctx, "vst_var", k_vst_var, dim3(sv_grid_for(ctx, ng * 32, 256, 8)), dim3(256), 0,
+  sv_launch(ctx, "vst_var", k_vst_var, dim3(sv_grid_for(ctx, ng * 32, VAR_THREADS, 6)), dim3(VAR_THREADS), 0,
             (const int64_t*)C->csc_colptr.get(), (const int32_t*)C->csc_count.get(), ng, C->n_cells,
             (const double*)mean.get(), (const double*)desd.get(), sqrt((double)C->n_cells), dout.get());
   std::vector<double> hv(ng);
@@ -297,12 +428,23 @@ SV_API int sv_find_variable_features_vst_surface(sv_context* ctx, const sv_count
   if (metric) std::copy(hv.begin(), hv.end(), metric);
   if (features && nfeatures > 0) {
     // partialsortperm(metric, 1:nfeatures, rev=true): largest first, ties by index
-    std::vector<int64_t> idx(ng);
-    for (int64_t g = 0; g < ng; ++g) idx[g] = g;
-    std::partial_sort(idx.begin(), idx.begin() + nfeatures, idx.end(), [&](int64_t a, int64_t b) {
-      return hv[a] > hv[b] || (hv[a] == hv[b] && a < b);
-    });
-    for (int64_t i = 0; i < nfeatures; ++i) features[i] = idx[i] + 1;
+    bool ranked = ng <= VST_RANK_MAX;
+    for (int64_t g = 0; g < ng && ranked; ++g) ranked = hv[g] == hv[g];
+    if (ranked) {
+      DevBuf<int> rank(ng);
+      DevBuf<int64_t> first(nfeatures);
+      launch_ranks(ctx, dout.get(), ng, true, rank.get());
+      sv_launch(ctx, "vst_rank", k_rank_first, dim3(sv_grid_for(ctx, ng, 256)), dim3(256), 0,
+                (const int*)rank.get(), ng, nfeatures, first.get());
+      sv_d2h(ctx, features, first.get(), nfeatures * 8);
+    } else {
+      std::vector<int64_t> idx(ng);
+      for (int64_t g = 0; g < ng; ++g) idx[g] = g;
+      std::partial_sort(idx.begin(), idx.begin() + nfeatures, idx.end(), [&](int64_t a, int64_t b) {
+        return hv[a] > hv[b] || (hv[a] == hv[b] && a < b);
+      });
+      for (int64_t i = 0; i < nfeatures; ++i) features[i] = idx[i] + 1;
+    }
   }
   SV_CATCH
 }
