@@ -598,6 +598,20 @@ struct AccOf<double> {
   typedef double type;
 };
 
+// v > clip ? clip : v without the FP64 pipe, where a comparison costs as much as a
+// product: doubles compare as integers once the negative ones' bits are turned
+// round (and the same turns them back).  A clip that is NaN clips nothing, and
+// neither is a v that is NaN (a product's: quiet).
+__device__ __forceinline__ long long turned(long long b) { return b ^ ((b >> 63) & 0x7fffffffffffffffll); }
+__device__ __forceinline__ long long clip_key(double clip) {
+  return clip != clip ? 0x7fffffffffffffffll : turned(__double_as_longlong(clip));
+}
+__device__ __forceinline__ double clip_above(double v, long long key) {
+  const bool over = turned(__double_as_longlong(v)) > key &&
+                    ((unsigned)__double2hiint(v) & 0x7fffffffu) < 0x7ff80000u;
+  return over ? __longlong_as_double(turned(key)) : v;
+}
+
 // ---- X v over CSR_h ------------------------------------------------------------
 // y = alpha * (B x - (mu . x)) + beta * y - (csub ? *csub : 0) * z
 // Per-feature table in shared memory.  FP32 form: (P, Q) = (inv*x, clip*x); the
@@ -605,9 +619,12 @@ struct AccOf<double> {
 // clip)*x).  FP64 form: (1/std, clip, x); a * (1/std) is within one ulp of the
 // reference's a/std (FP64 division is slow on this part).
 // Every block builds the table and mu.x itself from x (a separate one-block
-// kernel preparing the table for all blocks measured no faster).
+// kernel preparing the table for all blocks measured no faster); with few rows
+// that is half of the time, so blocks are large.  2,000 cells, FP64: 19.5 -> 16.6 us
+// (256 threads a block, which all did both; FP64 comparisons).
+constexpr int CSR_THREADS = 512;
 template <typename ValT, typename IdxT>
-__global__ void __launch_bounds__(256) k_spmv_csr(
+__global__ void __launch_bounds__(CSR_THREADS) k_spmv_csr(
     const int64_t* __restrict__ rowptr, const IdxT* __restrict__ hcol, const ValT* __restrict__ hval,
     int64_t n_rows, int64_t nf, const double* __restrict__ x, const float* __restrict__ inv_f,
     const float* __restrict__ clip_f, const double* __restrict__ inv_d,
@@ -618,26 +635,53 @@ __global__ void __launch_bounds__(256) k_spmv_csr(
   __shared__ double red[32];
   double mux = 0;
   {
-    for (int64_t f = threadIdx.x; f < nf; f += blockDim.x) {
-      double xf = x[f];
-      if constexpr (sizeof(AccT) == 4) {
-        float xs = (float)xf;
-        float P = inv_f[f] * xs;
-        float Q = xs == 0.f ? 0.f : clip_f[f] * xs;
-        ((float2*)smem_raw)[f] = make_float2(P, Q);
-      } else {
-        double* tab = (double*)smem_raw;
-        tab[3 * f] = inv_d[f];
-        tab[3 * f + 1] = clip_d[f];
-        tab[3 * f + 2] = xf;
+    // half of the threads build the table, the other half mu.x (in the order of
+    // CSR_THREADS / 2 threads), four features per thread in flight
+    constexpr int half = CSR_THREADS / 2;
+    const int t = threadIdx.x % half;
+    const bool sums = threadIdx.x < half;
+    for (int64_t f0 = t; f0 < nf; f0 += 4 * half) {
+      double xs[4], ms[4];
+      AccT iv[4], cl[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int64_t f = f0 + u * half;
+        if (f >= nf) break;
+        xs[u] = x[f];
+        if (sums) {
+          ms[u] = mu[f];
+        } else if constexpr (sizeof(AccT) == 4) {
+          iv[u] = inv_f[f];
+          cl[u] = clip_f[f];
+        } else {
+          iv[u] = inv_d[f];
+          cl[u] = clip_d[f];
+        }
       }
-      mux += mu[f] * xf;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int64_t f = f0 + u * half;
+        if (f >= nf) break;
+        if (sums) {
+          mux += ms[u] * xs[u];
+        } else if constexpr (sizeof(AccT) == 4) {
+          const float x1 = (float)xs[u];
+          const float P = iv[u] * x1;
+          const float Q = x1 == 0.f ? 0.f : cl[u] * x1;
+          ((float2*)smem_raw)[f] = make_float2(P, Q);
+        } else {
+          double* tab = (double*)smem_raw;
+          tab[3 * f] = iv[u];
+          tab[3 * f + 1] = __longlong_as_double(clip_key(cl[u]));
+          tab[3 * f + 2] = xs[u];
+        }
+      }
     }
     mux = sv_warp_sum(mux);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mux;
     __syncthreads();
     if (threadIdx.x < 32) {
-      double v = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
+      double v = threadIdx.x < half / 32 ? red[threadIdx.x] : 0.0;
       v = sv_warp_sum(v);
       if (threadIdx.x == 0) red[0] = v;
     }
@@ -679,8 +723,8 @@ __global__ void __launch_bounds__(256) k_spmv_csr(
             } else {
               const double* tab = (const double*)smem_raw;
               double v = av[h][t] * tab[3 * ci[h][t]];          // scaling.jl:211 (times 1/std)
-              double c = tab[3 * ci[h][t] + 1];
-              acc += (v > c ? c : v) * tab[3 * ci[h][t] + 2];   // scaling.jl:212
+              const long long c = __double_as_longlong(tab[3 * ci[h][t] + 1]);
+              acc += clip_above(v, c) * tab[3 * ci[h][t] + 2];   // scaling.jl:212
             }
           }
         }
@@ -1507,8 +1551,14 @@ __global__ void k_u_prep(const double* __restrict__ u, int64_t n, float* __restr
   }
 }
 
+// A warp per chunk, CHUNK_FLIGHT groups of 4 entries per lane and their gathers in
+// flight: with few cells there are few chunks (2,000 of 400 entries at 2,000 cells, 13
+// warps an SM), and a chunk is a chain of round trips.  Blocks of two warps share
+// the chunks out evenly.  2,000 cells, FP64: 21.0 -> 15.0 us.
+constexpr int CHUNK_FLIGHT = 2;
+constexpr int CHUNK_THREADS = 64, CHUNK_PER_SM = 16;
 template <typename ValT>
-__global__ void __launch_bounds__(256) k_spmv_csc_chunks(
+__global__ void __launch_bounds__(CHUNK_THREADS) k_spmv_csc_chunks(
     const int32_t* __restrict__ rowidx, const ValT* __restrict__ val,
     const int32_t* __restrict__ chunk_feat, const int64_t* __restrict__ cstart,
     const int64_t* __restrict__ cend, int64_t nchunks, const float* __restrict__ inv_f,
@@ -1516,39 +1566,54 @@ __global__ void __launch_bounds__(256) k_spmv_csc_chunks(
     const double* __restrict__ clip_d, const float* __restrict__ uf, const double* __restrict__ ud,
     double* __restrict__ partial) {
   typedef typename AccOf<ValT>::type AccT;
-  int lane = threadIdx.x & 31;
-  int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t c = warp; c < nchunks; c += nwarps) {
-    int32_t f = chunk_feat[c];
-    int64_t s = cstart[c], e = cend[c];
-    int64_t a0 = s & ~3ll;
-    AccT acc = 0;
+    const int32_t f = chunk_feat[c];
+    const int64_t s = cstart[c], e = cend[c], a0 = s & ~3ll;
+    const int32_t* src = rowidx + a0;
+    const ValT* vs = val + a0;
+    const int head = (int)(s - a0), len = (int)(e - a0);
+    AccT inv, clip;
+    const AccT* u;
     if constexpr (sizeof(AccT) == 4) {
-      float inv = inv_f[f], clip = clip_f[f];
-      for (int64_t g = a0 + 4 * lane; g < e; g += 128) {
-        int ri[4];
-        float av[4];
-        ld4(rowidx, g, ri);
-        ld4v(val, g, av);
-#pragma unroll
-        for (int t = 0; t < 4; ++t)
-          if (g + t >= s && g + t < e) acc += fminf(av[t] * inv, clip) * __ldg(uf + ri[t]);
-      }
+      inv = inv_f[f];
+      clip = clip_f[f];
+      u = uf;
     } else {
-      double sd = std_d[f], clip = clip_d[f];
-      for (int64_t g = a0 + 4 * lane; g < e; g += 128) {
-        int ri[4];
-        double av[4];
-        ld4(rowidx, g, ri);
-        ld4v(val, g, av);
+      inv = std_d[f];          // 1/std
+      clip = clip_d[f];
+      u = ud;
+    }
+    const long long key = clip_key((double)clip);
+    AccT acc = 0;
+    for (int g0 = 4 * lane; g0 < len; g0 += 128 * CHUNK_FLIGHT) {
+      int ri[CHUNK_FLIGHT][4];
+      AccT av[CHUNK_FLIGHT][4], x[CHUNK_FLIGHT][4];
 #pragma unroll
-        for (int t = 0; t < 4; ++t)
-          if (g + t >= s && g + t < e) {
-            double v = av[t] * sd;   // sd holds 1/std
-            acc += (v > clip ? clip : v) * __ldg(ud + ri[t]);
+      for (int h = 0; h < CHUNK_FLIGHT; ++h)
+        if (g0 + 128 * h < len) {
+          ld4(src, g0 + 128 * h, ri[h]);
+          ld4v(vs, g0 + 128 * h, av[h]);
+        }
+#pragma unroll
+      for (int h = 0; h < CHUNK_FLIGHT; ++h)
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const int g = g0 + 128 * h + t;
+          x[h][t] = g >= head && g < len ? __ldg(u + ri[h][t]) : AccT(0);
+        }
+#pragma unroll
+      for (int h = 0; h < CHUNK_FLIGHT; ++h)
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const int g = g0 + 128 * h + t;
+          if (g >= head && g < len) {
+            if constexpr (sizeof(AccT) == 4) acc += fminf(av[h][t] * inv, clip) * x[h][t];
+            else acc += clip_above(av[h][t] * inv, key) * x[h][t];
           }
-      }
+        }
     }
     acc = sv_warp_sum(acc);
     if (lane == 0) partial[c] = (double)acc;
@@ -1614,12 +1679,12 @@ static void launch_rb(sv_context* ctx, const sv_centered* S, const float* uf, bo
 static void launch_chunks(sv_context* ctx, const sv_centered* S, const double* ud, const float* uf,
                           bool beside = false) {
   sv_centered* Sm = const_cast<sv_centered*>(S);
-  int grid = sv_grid_for(ctx, S->n_chunks * 32, 256, 8);
-  if (beside) grid = std::min(grid, 8 * (ctx->num_sms - 1));
+  int grid = sv_grid_for(ctx, S->n_chunks * 32, CHUNK_THREADS, CHUNK_PER_SM);
+  if (beside) grid = std::min(grid, CHUNK_PER_SM * (ctx->num_sms - 1));
   const sv_data* D = S->data;
   const int32_t* rowidx = D->counts->csc_rowidx.get();
 #define LAUNCH_CSC(VT)                                                                            \
-  sv_launch(ctx, "spmv_csc_chunks", k_spmv_csc_chunks<VT>, dim3(grid), dim3(256), 0, rowidx,      \
+  sv_launch(ctx, "spmv_csc_chunks", k_spmv_csc_chunks<VT>, dim3(grid), dim3(CHUNK_THREADS), 0, rowidx, \
             (const VT*)D->csc_val.get(), (const int32_t*)S->chunk_feat.get(),                     \
             (const int64_t*)S->chunk_start.get(), (const int64_t*)S->chunk_end.get(), S->n_chunks, \
             (const float*)S->inv_std_f.get(), (const float*)S->clip_f.get(),                      \
@@ -1656,9 +1721,9 @@ void sv_centered_apply(sv_context* ctx, const sv_centered* S, char trans, const 
   if (trans == 'N') {
     size_t smem = S->dtype == SV_F64 ? (size_t)S->nf * 24 : (size_t)S->nf * 8;
     smem = (smem + 15) & ~(size_t)15;
-    int grid = (int)std::max<int64_t>(1, std::min<int64_t>(S->grid_csr, (S->n_cells + 7) / 8));
+    int grid = (int)std::max<int64_t>(1, std::min<int64_t>(S->grid_csr, (S->n_cells * 32 + CSR_THREADS - 1) / CSR_THREADS));
 #define LAUNCH_CSR(VT, IT, COL)                                                                  \
-  sv_launch(ctx, "spmv_csr_h", k_spmv_csr<VT, IT>, dim3(grid), dim3(256), smem,                  \
+  sv_launch(ctx, "spmv_csr_h", k_spmv_csr<VT, IT>, dim3(grid), dim3(CSR_THREADS), smem,          \
             (const int64_t*)S->h_rowptr.get(), (const IT*)COL, (const VT*)S->h_val.get(),         \
             S->n_cells, S->nf, x, (const float*)S->inv_std_f.get(), (const float*)S->clip_f.get(), \
             (const double*)S->inv_std_d.get(), (const double*)S->clip_d.get(),                    \
@@ -2081,12 +2146,12 @@ static sv_centered* make_centered(sv_context* ctx, const sv_data* data, const st
         case SV_F64:
           SV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
               &b1, small16 ? (const void*)k_spmv_csr<double, uint16_t> : (const void*)k_spmv_csr<double, int32_t>,
-              256, tsm));
+              CSR_THREADS, tsm));
           break;
         case SV_F32:
           SV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
               &b1, small16 ? (const void*)k_spmv_csr<float, uint16_t> : (const void*)k_spmv_csr<float, int32_t>,
-              256, tsm));
+              CSR_THREADS, tsm));
           SV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
               &b2, small16 ? (const void*)k_spmv_csr_df<float, uint16_t> : (const void*)k_spmv_csr_df<float, int32_t>,
               256, tsm_df));
@@ -2095,7 +2160,7 @@ static sv_centered* make_centered(sv_context* ctx, const sv_data* data, const st
           SV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
               &b1, small16 ? (const void*)k_spmv_csr<__nv_bfloat16, uint16_t>
                            : (const void*)k_spmv_csr<__nv_bfloat16, int32_t>,
-              256, tsm));
+              CSR_THREADS, tsm));
           SV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
               &b2, small16 ? (const void*)k_spmv_csr_df<__nv_bfloat16, uint16_t>
                            : (const void*)k_spmv_csr_df<__nv_bfloat16, int32_t>,

@@ -1,0 +1,36 @@
+"""GPU: the FP64 products clip as a comparison of doubles does, at clips above, among and
+below the values, negative and infinite, over columns and rows around the groups of
+the two kernels and with few and many cells."""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("scale_max", [10.0, 1.0, 0.0, -0.5, -5.0, np.inf])
+@pytest.mark.parametrize("n,nf", [(3, 5), (130, 257), (700, 1030), (6000, 300)])
+def test_fp64_products_clip(sv, ctx, n, nf, scale_max):
+    rng = np.random.default_rng(n)
+    X = np.where(rng.random((n, nf)) < 0.3, rng.integers(1, 30, (n, nf)), 0)
+    X[0] = 1 + np.arange(nf) % 3                              # no constant column, no empty cell
+    X[1:, 0] = 2
+    X[2, 1:] = 0
+    D = sv.normalize_cells(sv.CountMatrix.from_csc(sp.csc_matrix(X.astype(np.int32)), ctx=ctx), scale_factor=1e4,
+                           dtype="float64")
+    S = sv.scale_features(D, scale_max=scale_max)
+    mu, mean, std = S.stats()
+    csc = sp.csc_matrix(X)
+    B = np.zeros((n, nf))
+    rows, cols = csc.indices, np.repeat(np.arange(nf), np.diff(csc.indptr))
+    v = D.values_csc() * (1.0 / std)[cols]
+    clip = scale_max + mu[cols]
+    B[rows, cols] = np.where(v > clip, clip, v)
+    A = B - mu
+    for M, x, y in ((A, rng.normal(size=nf), None), (A.T, rng.normal(size=n), None)):
+        y = S.mul(x) if M is A else S.rmul(x)
+        # sums of products in another order: (terms) 2^-53 of the sum of their sizes, with
+        # the product by mu apart
+        size = (np.abs(B) if M is A else np.abs(B).T) @ np.abs(x) + (np.abs(mu) @ np.abs(x) if M is A else
+                                                                      np.abs(mu) * np.abs(x).sum())
+        assert np.all(np.abs(y - M @ x) <= 2 * max(n, nf) * 2.0 ** -53 * size + 1e-300)
