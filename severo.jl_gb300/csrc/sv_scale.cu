@@ -1318,9 +1318,11 @@ __global__ void k_rb_count(const int64_t* __restrict__ fstart, const int64_t* __
 // included.  Entries and padding pass through a ring of RC_RING places per warp in
 // shared memory; whenever it holds 256, each lane codes one group of 8 and writes
 // its word and values at once (a 64-bit atomic or per entry and scalar value
-// stores took 1.77 ms for 117 M FP32 entries of 100,000 cells, this 1.08 ms).
+// stores took 1.77 ms for 117 M FP32 entries of 100,000 cells, this 0.88 ms; one
+// group of entries in flight instead of RC_FLIGHT 1.08).
 constexpr int RC_RING = 512;
 constexpr int RC_WARPS = 8;
+constexpr int RC_FLIGHT = 2;   // groups of 32 entries in flight
 template <typename ValT>
 __global__ void __launch_bounds__(RC_WARPS * 32) k_rb_copy(
     const int64_t* __restrict__ src, const int64_t* __restrict__ dst, const int64_t* __restrict__ fend,
@@ -1337,7 +1339,7 @@ __global__ void __launch_bounds__(RC_WARPS * 32) k_rb_copy(
     const int64_t b = p / nf;
     const int first = (int)rb_first_row(row0, b);
     const int64_t s = src[p], d = dst[p];
-    const int64_t hi = lower_bound_rows(rowidx, s, fend[p % nf], rb_first_row(row0, b + 1));
+    const int64_t hi = p + nf < npairs ? src[p + nf] : fend[p % nf];   // the next block's first entry
     int64_t word = d / RB_GROUP;   // the next word to write
     int head = 0, cur = 0;         // ring: cur places from head
     // writes the first `words` groups of the ring
@@ -1367,13 +1369,28 @@ __global__ void __launch_bounds__(RC_WARPS * 32) k_rb_copy(
       __syncwarp();
     };
     int last = 0;                  // the row before t0
-    int64_t t0 = s;
-    int nrow = s + lane < hi ? rowidx[s + lane] : 0;     // one group ahead
-    ValT nval = s + lane < hi ? val[s + lane] : ValT(0.f);
-    while (t0 < hi) {
+    int nrow[RC_FLIGHT];           // the next groups of 32 entries
+    ValT nval[RC_FLIGHT];
+#pragma unroll
+    for (int h = 0; h < RC_FLIGHT; ++h) {
+      const int64_t t = s + 32 * h + lane;
+      nrow[h] = t < hi ? rowidx[t] : 0;
+      nval[h] = t < hi ? val[t] : ValT(0.f);
+    }
+    for (int64_t t0 = s; t0 < hi; t0 += 32) {
       const bool on = t0 + lane < hi;
-      const int r = nrow - first;
-      const ValT v = nval;
+      const int r = nrow[0] - first;
+      const ValT v = nval[0];
+#pragma unroll
+      for (int h = 0; h + 1 < RC_FLIGHT; ++h) {
+        nrow[h] = nrow[h + 1];
+        nval[h] = nval[h + 1];
+      }
+      const int64_t tn = t0 + 32 * RC_FLIGHT + lane;
+      if (tn < hi) {
+        nrow[RC_FLIGHT - 1] = rowidx[tn];
+        nval[RC_FLIGHT - 1] = val[tn];
+      }
       const int up = __shfl_up_sync(0xffffffffu, r, 1);
       const int rp = lane > 0 ? up : t0 > s ? last : r;
       const int k = on ? rb_pads(r - rp) : 0;
@@ -1386,29 +1403,30 @@ __global__ void __launch_bounds__(RC_WARPS * 32) k_rb_copy(
           if (lane >= sh) incl += y;
         }
       }
-      // as many entries as 256 places take (one entry takes at most 261)
-      const unsigned fit = __ballot_sync(0xffffffffu, on && (incl <= 256 || lane == 0));
-      const int m = __popc(fit);
-      const int tot = __shfl_sync(0xffffffffu, incl, m - 1);
-      last = __shfl_sync(0xffffffffu, r, m - 1);
-      const int64_t tn = t0 + m;
-      if (cur + tot > RC_RING) flush(cur / RB_GROUP);   // fewer than 256 places: at most 31 words
-      if (tn + lane < hi) {
-        nrow = rowidx[tn + lane];
-        nval = val[tn + lane];
-      }
-      if (lane < m) {
-        int q = head + cur + incl - (k + 1);
-        for (int u = 1; u <= k; ++u, ++q) {
-          rr[q & (RC_RING - 1)] = (uint16_t)(rp + 63 * u);
-          rv[q & (RC_RING - 1)] = ValT(0.f);
+      // the group at once, or as many entries as 256 places take at a time (one entry
+      // takes at most 261)
+      unsigned todo = __ballot_sync(0xffffffffu, on);
+      last = __shfl_sync(0xffffffffu, r, 31 - __clz(todo));
+      int before = 0;                // places of the entries done
+      while (todo) {
+        const bool mine = (todo >> lane & 1) && (incl - before <= 256 || (todo & ((1u << lane) - 1)) == 0);
+        const unsigned fit = __ballot_sync(0xffffffffu, mine);
+        const int upto = __shfl_sync(0xffffffffu, incl, 31 - __clz(fit));
+        if (cur + upto - before > RC_RING) flush(cur / RB_GROUP);   // fewer than 256 places: at most 31 words
+        if (mine) {
+          int q = head + cur + incl - before - (k + 1);
+          for (int u = 1; u <= k; ++u, ++q) {
+            rr[q & (RC_RING - 1)] = (uint16_t)(rp + 63 * u);
+            rv[q & (RC_RING - 1)] = ValT(0.f);
+          }
+          rr[q & (RC_RING - 1)] = (uint16_t)r;
+          rv[q & (RC_RING - 1)] = v;
         }
-        rr[q & (RC_RING - 1)] = (uint16_t)r;
-        rv[q & (RC_RING - 1)] = v;
+        cur += upto - before;
+        before = upto;
+        todo &= ~fit;
+        if (cur >= 256) flush(32);
       }
-      cur += tot;
-      t0 = tn;
-      if (cur >= 256) flush(32);
     }
     // value-0 entries up to the group boundary, at the last row
     const int fill = (RB_GROUP - cur % RB_GROUP) % RB_GROUP;
