@@ -39,7 +39,8 @@ constexpr int64_t CHUNK = 4096;   // non-zeros per warp task in the X^T u produc
 // and each group's (hi, lo) pairs are added into FP64 sums: relative error of
 // the sums ~2^-48 per group, of M2 ~2^-47 (1 + mean^2 / var) (3.9e-14 at
 // worst on the FP32 test data, 4e-15 for BF16, against FP64 Welford).  FP64
-// and Int32 data are summed in FP64.
+// data are summed in FP64, counts in integers (in FP64 where one has 16 bits or
+// more).
 //
 // Work split: each column is cut into parts of at most MOM_PART entries, one
 // warp task each (a device-built task table: per column its range and the
