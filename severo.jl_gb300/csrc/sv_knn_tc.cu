@@ -474,9 +474,9 @@ __global__ void __launch_bounds__(THREADS, 1)
           }
         }
       }
-      if (lists || (coord && (t & 3) == 3)) {
-        // every fourth tile (every tile of a list); keys only fall, so a stale (larger) bound read by
-        // the producer is safe
+      if (nrm && ((t & 3) == 3 || (lists && t < 32))) {
+        // every fourth tile (a list's first 32 as well: its nearest tiles come first);
+        // keys only fall, so a stale (larger) bound read by the producer is safe
         float v = q < qend ? best[KH - 1] + qn : -FLT_MAX;
         if (v != v) v = __int_as_float(0x7f800000);   // no bound from a NaN
 #pragma unroll
