@@ -60,6 +60,21 @@ void SvPool::account(int64_t delta) {
 
 void* SvPool::alloc(size_t bytes) {
   void* p = nullptr;
+  if (direct(bytes)) {
+    cudaError_t e = cudaMalloc(&p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      cudaStreamSynchronize(stream);
+      cudaMemPoolTrimTo(pool, 0);
+      e = cudaMalloc(&p, bytes);
+    }
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      sv_throw(e == cudaErrorMemoryAllocation ? SV_ERR_OOM : SV_ERR_CUDA,
+               "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
+    }
+    return p;
+  }
   {
     std::lock_guard<std::mutex> lk(mu);
     account((int64_t)bytes);
@@ -86,7 +101,10 @@ void* SvPool::alloc(size_t bytes) {
 void SvPool::free(void* p, size_t bytes) {
   std::lock_guard<std::mutex> lk(mu);
   cudaSetDevice(device);
-  if (alive) {
+  if (direct(bytes)) {
+    if (alive) cudaStreamSynchronize(stream);   // what still uses the block
+    cudaFree(p);
+  } else if (alive) {
     account(-(int64_t)bytes);
     cudaFreeAsync(p, stream);
   } else {

@@ -77,7 +77,10 @@ struct SvTimedLaunch {
 // SV_POOL_KEEP of the device's memory between calls, gives all of it back when
 // the context is destroyed or an allocation fails, and is shared by the
 // context and its live blocks: a block that outlives its context is freed with
-// cudaFree.
+// cudaFree.  Blocks above a quarter of what it keeps go to cudaMalloc and cudaFree:
+// they would mostly be given back anyway, and the pool maps and unmaps them more
+// slowly (counts of 4.9 G entries, 79 GB: upload 634 ms through the pool, 500
+// so; freeing everything 110 against 50).
 constexpr size_t SV_POOL_KEEP = 16;   // one part in 16 of the device's memory
 struct SvPool {
   int device = 0;
@@ -88,6 +91,7 @@ struct SvPool {
   size_t live = 0;      // bytes of blocks in use
   size_t keep = 0;      // most bytes kept besides
   size_t threshold = 0;
+  bool direct(size_t bytes) const { return bytes > keep / 4; }
   void account(int64_t delta);
   void* alloc(size_t bytes);
   void free(void* p, size_t bytes);
