@@ -2,8 +2,8 @@
 //
 // Distances in the GEMM form key(q, p) = |p|^2 - 2 q.p over BF16-rounded
 // coordinates (K padded to 64 = one 128-byte swizzle row), FP32 accumulation in
-// tensor memory.  One CTA per block of 128 queries streams every point tile of
-// 256 points:
+// tensor memory.  One CTA per block of 128 queries streams the point tiles of 256
+// points that are within its reach:
 //   warp 0      TMA producer (one thread): the query tile once, point tiles into
 //               a 4-stage ring (cp.async.bulk.tensor, 128B swizzle, mbarriers);
 //   warp 1      MMA issuer (one thread): 4 x tcgen05.mma.kind::f16 (K = 16 each)
@@ -528,8 +528,8 @@ __global__ void k_pack_bf16(const float* __restrict__ X, int64_t n, int dp, int6
 // columns d..d+2, points carry |p|^2 split into three BF16 parts (hi, mid, lo,
 // summing to the FP32 norm of the rounded row to ~2^-24), so that the MMA yields
 // D = q.p - |p|^2/2 and the key |p|^2 - 2 q.p is -2 D.
-// With coord: also the sort coordinate (column dim) and |p|^2 of the BF16
-// operand row, and the largest |p|^2 (float bits; all values >= 0).
+// With coord: also the sort coordinate (column dim) of the BF16 operand row; with
+// nrm: its |p|^2, and the largest |p|^2 (float bits; all values >= 0).
 // Eight threads per row, eight columns each (16-byte stores; one thread per row took
 // 0.35 ms for 300,000 rows, this 0.07); the norm is thread 0's, in column order.
 __global__ void k_pack_fold(const float* __restrict__ X, int64_t n, int dp, int d,
