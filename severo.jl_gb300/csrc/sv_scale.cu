@@ -1278,10 +1278,11 @@ __device__ __forceinline__ int64_t rb_first_row(const int64_t* row0, int64_t b) 
 // 64-bit word per group: bits 0-15 the row (within the block) of the group's
 // first entry, bits 16 + 6 (t - 1) .. the 6-bit step from entry t - 1 to entry
 // t (t = 1..7).  A step longer than 63 between consecutive entries is bridged
-// by padding entries (rows r + 63, r + 126, ... and value 0), and every segment
-// is padded with value-0 entries to a whole number of groups, so segments
-// start on group boundaries.  Padding adds exactly 0 to the product:
-// min(0 * (1/sigma), clip) = 0 with clip > 0.
+// by padding entries (rows r + 63, r + 126, ... and value -0), and every segment
+// is padded with value -0 entries to a whole number of groups, so segments
+// start on group boundaries.  Padding adds exactly 0 to the product: where clip
+// >= 0 as min(-0 * (1/sigma), clip), and below that, where a stored 0 is clipped
+// as well, its sign tells it apart.
 constexpr int RB_GROUP = 8;
 __device__ __forceinline__ int rb_pads(int64_t step) { return step > 63 ? (int)((step - 1) / 63) : 0; }
 
@@ -1418,7 +1419,7 @@ __global__ void __launch_bounds__(RC_WARPS * 32) k_rb_copy(
           int q = head + cur + incl - before - (k + 1);
           for (int u = 1; u <= k; ++u, ++q) {
             rr[q & (RC_RING - 1)] = (uint16_t)(rp + 63 * u);
-            rv[q & (RC_RING - 1)] = ValT(0.f);
+            rv[q & (RC_RING - 1)] = ValT(-0.f);
           }
           rr[q & (RC_RING - 1)] = (uint16_t)r;
           rv[q & (RC_RING - 1)] = v;
@@ -1429,11 +1430,11 @@ __global__ void __launch_bounds__(RC_WARPS * 32) k_rb_copy(
         if (cur >= 256) flush(32);
       }
     }
-    // value-0 entries up to the group boundary, at the last row
+    // padding up to the group boundary, at the last row
     const int fill = (RB_GROUP - cur % RB_GROUP) % RB_GROUP;
     if (lane < fill) {
       rr[(head + cur + lane) & (RC_RING - 1)] = (uint16_t)last;
-      rv[(head + cur + lane) & (RC_RING - 1)] = ValT(0.f);
+      rv[(head + cur + lane) & (RC_RING - 1)] = ValT(-0.f);
     }
     cur += fill;
     if (cur >= 256) flush(32);
@@ -1451,6 +1452,7 @@ struct RbGroup {
     v[0] = __ldg((const uint4*)pv);
     if constexpr (sizeof(ValT) == 4) v[1] = __ldg((const uint4*)pv + 1);
   }
+  template <bool BELOW = false>   // BELOW: clip < 0
   __device__ __forceinline__ void add(float& acc, float inv, float clip, const float* us) const {
     // byte offsets into us: a field is shifted to bit 2 and masked
     const unsigned lo = (unsigned)c, hi = (unsigned)(c >> 32);
@@ -1468,6 +1470,7 @@ struct RbGroup {
       } else {
         a = __uint_as_float((&v[t >> 2].x)[t & 3]);
       }
+      if (BELOW && __float_as_uint(a) == 0x80000000u) continue;   // padding
       acc += fminf(a * inv, clip) * *(const float*)((const char*)us + r);
     }
   }
@@ -1480,13 +1483,21 @@ __device__ __forceinline__ float rb_seg_dot(const unsigned long long* __restrict
                                            const ValT* __restrict__ pv, int n,
                                            float inv, float clip, const float* us, int lane) {
   constexpr int D = sizeof(ValT) == 2 ? RB_DEPTH2 : RB_DEPTH4;
+  float acc = 0.f;
+  if (clip < 0.f) {   // scale_max below -mu: rare, one group at a time
+    for (int g = lane; g < n; g += 32) {
+      RbGroup<ValT> one;
+      one.load(code + g, pv + RB_GROUP * g);
+      one.template add<true>(acc, inv, clip, us);
+    }
+    return acc;
+  }
   RbGroup<ValT> buf[D];
 #pragma unroll
   for (int h = 0; h < D; ++h) {
     const int g = lane + 32 * h;
     if (g < n) buf[h].load(code + g, pv + RB_GROUP * g);
   }
-  float acc = 0.f;
   for (int g0 = lane; g0 < n; g0 += 32 * D) {
 #pragma unroll
     for (int h = 0; h < D; ++h) {

@@ -34,3 +34,35 @@ def test_fp64_products_clip(sv, ctx, n, nf, scale_max):
         size = (np.abs(B) if M is A else np.abs(B).T) @ np.abs(x) + (np.abs(mu) @ np.abs(x) if M is A else
                                                                       np.abs(mu) * np.abs(x).sum())
         assert np.all(np.abs(y - M @ x) <= 2 * max(n, nf) * 2.0 ** -53 * size + 1e-300)
+
+
+def _clipped(sv, ctx, n, nf, scale_max, dtype, seed):
+    """A scaled matrix over rows with gaps of more than 63 in most columns (bridged in the
+    row-blocked copy), and B - mu of it in FP64 from the parameters that FP32 products use."""
+    rng = np.random.default_rng(seed)
+    X = np.where(rng.random((n, nf)) < rng.choice([0.004, 0.1, 0.5], nf), rng.integers(1, 30, (n, nf)), 0)
+    X[0] = 1 + np.arange(nf) % 3                              # no constant column, no empty cell
+    X[1:, 0] = 2
+    X[n - 1, 1:] = 5
+    D = sv.normalize_cells(sv.CountMatrix.from_csc(sp.csc_matrix(X.astype(np.int32)), ctx=ctx), scale_factor=1e4,
+                           dtype=dtype)
+    S = sv.scale_features(D, scale_max=scale_max)
+    mu, _, std = S.stats()
+    csc = sp.csc_matrix(X)
+    B = np.zeros((n, nf))
+    rows, cols = csc.indices, np.repeat(np.arange(nf), np.diff(csc.indptr))
+    inv, clip = (1.0 / std).astype(np.float32)[cols], (scale_max + mu).astype(np.float32)[cols]
+    B[rows, cols] = np.minimum((D.values_csc().astype(np.float32) * inv).astype(np.float64), clip)
+    return D, S, B, mu
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("scale_max", [10.0, 0.0, -0.5, -5.0])
+@pytest.mark.parametrize("n,nf", [(130, 257), (3000, 90), (20000, 40)])
+def test_row_blocked_product_clips(sv, ctx, n, nf, scale_max, dtype):
+    """X^T u over the padded row-blocked copy: padding adds nothing, below any clip either."""
+    _, S, B, mu = _clipped(sv, ctx, n, nf, scale_max, dtype, n)
+    u = np.random.default_rng(1).normal(size=n).astype(np.float32).astype(np.float64)
+    # FP32 sums of at most n products, each rounded; sum(u) and mu in FP64
+    size = np.abs(B).T @ np.abs(u)
+    assert np.all(np.abs(S.rmul(u) - (B - mu).T @ u) <= (n + 4) * 2.0 ** -24 * size + 1e-12 * np.abs(mu) * np.abs(u).sum())
