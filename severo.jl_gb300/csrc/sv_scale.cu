@@ -922,7 +922,7 @@ __device__ __forceinline__ void dfx_fma(float& sh, float& sl, float ah, float al
 
 // Prologue shared by the double-float X v kernels: with stacked samples (blk
 // non-null) selects block b's row range and sample s = blk[b].seg (false: the
-// sample is frozen, nothing to do); builds the per-feature (inv*x, clip*x)
+// sample is frozen, nothing to do); builds the per-feature (inv*x, clip*|x|)
 // table in shared memory and returns mu.x and -csub as double-float pairs.
 struct XvDf {
   int64_t rb0, rb1;
@@ -972,7 +972,7 @@ __device__ __forceinline__ bool xv_df_prologue(
       if (f >= nf) break;
       const float xs = in[u][0];
       const float P = in[u][2] * xs;
-      const float Q = xs == 0.f ? 0.f : in[u][3] * xs;
+      const float Q = xs == 0.f ? 0.f : in[u][3] * fabsf(xs);   // of clip's sign
       ((float2*)smem_raw)[f] = make_float2(P, Q);
       dfx_fma(mh, ml, in[u][4], in[u][5], xs, in[u][1]);
     }
@@ -1063,12 +1063,12 @@ struct XvGroup {
   __device__ __forceinline__ unsigned index(int t) const {
     return sizeof(IdxT) == 2 ? ((t & 1) ? i[t >> 1] >> 16 : i[t >> 1] & 0xffffu) : i[t];
   }
-  // min(a P, Q) for P >= 0, max(a P, Q) for P < 0, as the sign of P on min(a |P|, |Q|)
-  // (P and Q have one sign): one minimum and no comparison
+  // min(a/std, clip) x with (P, Q) = (x/std, clip |x|): the sign of x, which is P's,
+  // on min(a |P|, Q) -- one minimum and no comparison, and clip may be negative
   __device__ __forceinline__ float term(int t, float2 x) const {
     const float a = __uint_as_float(
         sizeof(ValT) == 2 ? ((t & 1) ? v[t >> 1] & 0xffff0000u : v[t >> 1] << 16) : v[t]);
-    const float m = fminf(a * fabsf(x.x), fabsf(x.y));
+    const float m = fminf(a * fabsf(x.x), x.y);
     return __uint_as_float(__float_as_uint(m) ^ (__float_as_uint(x.x) & 0x80000000u));
   }
 };

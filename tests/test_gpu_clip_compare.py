@@ -66,3 +66,39 @@ def test_row_blocked_product_clips(sv, ctx, n, nf, scale_max, dtype):
     # FP32 sums of at most n products, each rounded; sum(u) and mu in FP64
     size = np.abs(B).T @ np.abs(u)
     assert np.all(np.abs(S.rmul(u) - (B - mu).T @ u) <= (n + 4) * 2.0 ** -24 * size + 1e-12 * np.abs(mu) * np.abs(u).sum())
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("scale_max", [10.0, 1.0, 0.0, -0.5, -5.0])
+@pytest.mark.parametrize("n,nf", [(130, 257), (3000, 1100)])
+def test_irlba_products_clip(sv, ctx, n, nf, scale_max, dtype):
+    """Both streamed products of the PCA are those of one matrix, the clipped one: A V = U s
+    row by row, and the singular values are A's."""
+    _, S, B, mu = _clipped(sv, ctx, n, nf, scale_max, dtype, nf)
+    A = B - mu
+    U, s, V = sv.irlba(S, 3, tol=1e-8, seed=1)
+    # FP32 sums of at most nf products, each rounded; mu.x in double-float; what the
+    # iteration leaves (1e-8 s)
+    size = ((nf + 4) * 2.0 ** -24 * np.abs(B) + 2.0 ** -40 * np.abs(mu)) @ np.abs(V) + 1e-7 * s[0]
+    assert np.all(np.abs(A @ V - U * s) <= size)
+    assert np.max(np.abs(s - np.linalg.svd(A, compute_uv=False)[:3])) <= 1e-5 * s[0]
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("scale_max", [1.0, -0.5])
+def test_batch_products_clip(sv, ctx, scale_max, dtype):
+    n, nf, off = 700, 300, np.array([0, 250, 700])
+    D, _, _, _ = _clipped(sv, ctx, n, nf, scale_max, dtype, 3)
+    v = sp.csr_matrix(D.to_csc())
+    ok = np.ones(nf, bool)
+    for a, b in zip(off, off[1:]):                            # features that vary in every sample
+        ok &= v[a:b].toarray().std(axis=0) > 0
+    features = np.flatnonzero(ok) + 1
+    batch = sv.Batch.create(D, off, features=features, scale_max=scale_max)
+    em = sv.batch_pca(batch, 3, tol=1e-8, seed=1)
+    mu, _, std = batch.stats()
+    for g, (a, b) in enumerate(zip(off, off[1:])):
+        M = v[a:b, features - 1].toarray().astype(np.float64)
+        B = np.where(M != 0, np.minimum(M / std[g], scale_max + mu[g]), 0.0)
+        s = np.linalg.svd(B - mu[g], compute_uv=False)[:3]
+        assert np.max(np.abs(em.stdev[g] * np.sqrt(b - a - 1) - s)) <= 1e-5 * s[0]
