@@ -27,7 +27,7 @@ namespace {
 
 constexpr int KNN_THREADS = 256;
 constexpr int KNN_TILE = 64;       // points per tile and queries per block
-constexpr int KNN_LIST = 64;       // most candidates of a query
+constexpr int KNN_LIST = 64;       // most candidates of a query (the length of its sorted list)
 constexpr int64_t KNN_ORDER_MIN = 2048;
 
 // X (n x d, column-major, leading dim ld, FP32 or FP64) -> row-major FP32 [n][dp]
@@ -114,7 +114,8 @@ __device__ __forceinline__ void w64_step(unsigned long long (&v)[2], int stride,
   }
 }
 
-// The K2 smallest keys |p|^2 - 2 q.p of every query, equal keys by index.  Block of
+// The `keep` smallest keys |p|^2 - 2 q.p of every query, equal keys by index, in K2
+// places (-1 after them).  Block of
 // 64 queries; per tile of 64 points a thread forms a 4 x 4 patch of keys (two
 // 16-byte shared loads per 16 FMAs; each key one chain over the dimensions), and
 // keys that pass their query's threshold are appended to the query's buffer in
@@ -130,7 +131,7 @@ __device__ __forceinline__ void w64_step(unsigned long long (&v)[2], int stride,
 template <int DP>
 __global__ void __launch_bounds__(KNN_THREADS, 2) k_knn_fp32(
     const float* __restrict__ Xt, const float* __restrict__ sqt, const int* __restrict__ orig, int64_t n,
-    int K2, int32_t* __restrict__ cand, const unsigned long long* __restrict__ lists,
+    int keep, int K2, int32_t* __restrict__ cand, const unsigned long long* __restrict__ lists,
     const unsigned* __restrict__ pmax) {
   extern __shared__ __align__(16) unsigned char knn_dyn[];
   float* Q = (float*)knn_dyn;                       // [DP][64], times -2
@@ -193,8 +194,8 @@ __global__ void __launch_bounds__(KNN_THREADS, 2) k_knn_fp32(
     for (int s = 32; s > 0; s >>= 1) w64_step(a, s, 64);
     L[lane] = a[0];
     L[lane + 32] = a[1];
-    const unsigned long long last = K2 > 32 ? a[1] : a[0];
-    if (lane == ((K2 - 1) & 31)) {
+    const unsigned long long last = keep > 32 ? a[1] : a[0];
+    if (lane == ((keep - 1) & 31)) {
       if (last != ~0ull) {
         thr[q] = key_float((unsigned)(last >> 32));
         thr64[q] = last;
@@ -310,7 +311,7 @@ __global__ void __launch_bounds__(KNN_THREADS, 2) k_knn_fp32(
     __syncwarp();
     const unsigned long long* L = ent + (size_t)q * 2 * KNN_LIST;
     int32_t* o = cand + (int64_t)orig[qi] * K2;
-    for (int k = lane; k < K2; k += 32) o[k] = L[k] == ~0ull ? -1 : (int32_t)(unsigned)L[k];
+    for (int k = lane; k < K2; k += 32) o[k] = k >= keep || L[k] == ~0ull ? -1 : (int32_t)(unsigned)L[k];
   }
 }
 
@@ -396,7 +397,7 @@ __global__ void k_rerank(const float* __restrict__ X, int64_t n, const int32_t* 
 }
 
 template <int DP>
-void launch_fp32(sv_context* ctx, const float* X, const float* sq, int64_t n, int d, int K2, int32_t* cand) {
+void launch_fp32(sv_context* ctx, const float* X, const float* sq, int64_t n, int d, int keep, int K2, int32_t* cand) {
   const int64_t ntiles = (n + KNN_TILE - 1) / KNN_TILE, npad = ntiles * KNN_TILE;
   KnnOrder ord;
   const bool listed = n >= KNN_ORDER_MIN && sv_knn_order(ctx, X, n, DP, d, KNN_TILE, KNN_TILE, ord);
@@ -410,7 +411,7 @@ void launch_fp32(sv_context* ctx, const float* X, const float* sq, int64_t n, in
   const size_t smem = (size_t)2 * DP * KNN_TILE * 4 + (size_t)KNN_TILE * 2 * KNN_LIST * 8;
   SV_CUDA(cudaFuncSetAttribute(k_knn_fp32<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   sv_launch(ctx, "knn_fp32_tiles", k_knn_fp32<DP>, dim3((unsigned)ntiles), dim3(KNN_THREADS), smem,
-            (const float*)Xt.get(), (const float*)sqt.get(), (const int*)orig.get(), n, K2, cand,
+            (const float*)Xt.get(), (const float*)sqt.get(), (const int*)orig.get(), n, keep, K2, cand,
             listed ? (const unsigned long long*)ord.lists.get() : (const unsigned long long*)nullptr,
             (const unsigned*)pmax.get());
 }
@@ -452,9 +453,12 @@ __global__ void k_to_host_layout(const int32_t* __restrict__ idx, const float* _
 static void knn_core(sv_context* ctx, const float* X32, const float* sq, int64_t n, int dp, int d, int k,
                      int include_self, int cosine, int precision, sv_knn* out,
                      const std::vector<int64_t>* segs = nullptr) {
-  // candidates per query: at least 2k; a multiple of 8 from the FP32 tiles, 40 (k <=
-  // 20) or 64 from the tensor-core tiles
-  int K2 = precision == SV_KNN_BF16 ? (2 * k <= 40 ? 40 : 64) : std::max(16, (2 * k + 7) / 8 * 8);
+  // candidates per query, at least 2k: 32 (k <= 16) or 64 from the FP32 tiles, the point
+  // itself among them where it is its own neighbour; 40 (k <= 20) or 64 from the
+  // tensor-core tiles.  More than 2k because the FP32 keys cancel far from the origin:
+  // 4,000 points in 50 dimensions 500 times their spread away, k = 8: recall 0.999 with
+  // 32, 0.976 with 16
+  int K2 = precision == SV_KNN_BF16 ? (2 * k <= 40 ? 40 : 64) : (2 * k <= 32 ? 32 : 64);
   if (2 * k > 64) sv_throw(SV_ERR_UNSUPPORTED, "k = %d exceeds the supported maximum of 32", k);
   DevBuf<int32_t> cand((size_t)n * K2);
   bool done = false;
@@ -465,6 +469,7 @@ static void knn_core(sv_context* ctx, const float* X32, const float* sq, int64_t
   }
   if (!done) {
     // FP32 tiles: one launch per sample (each on its own rows)
+    const int keep = include_self ? K2 - 1 : K2;   // besides the point itself
     std::vector<int64_t> one = {0, n};
     const std::vector<int64_t>& sg = segs ? *segs : one;
     for (size_t g = 0; g + 1 < sg.size(); ++g) {
@@ -474,14 +479,14 @@ static void knn_core(sv_context* ctx, const float* X32, const float* sq, int64_t
       const float* qs = sq + o;
       int32_t* cs = cand.get() + o * K2;
       switch (dp) {
-        case 8: launch_fp32<8>(ctx, Xs, qs, ns, d, K2, cs); break;
-        case 16: launch_fp32<16>(ctx, Xs, qs, ns, d, K2, cs); break;
-        case 24: launch_fp32<24>(ctx, Xs, qs, ns, d, K2, cs); break;
-        case 32: launch_fp32<32>(ctx, Xs, qs, ns, d, K2, cs); break;
-        case 40: launch_fp32<40>(ctx, Xs, qs, ns, d, K2, cs); break;
-        case 48: launch_fp32<48>(ctx, Xs, qs, ns, d, K2, cs); break;
-        case 56: launch_fp32<56>(ctx, Xs, qs, ns, d, K2, cs); break;
-        case 64: launch_fp32<64>(ctx, Xs, qs, ns, d, K2, cs); break;
+        case 8: launch_fp32<8>(ctx, Xs, qs, ns, d, keep, K2, cs); break;
+        case 16: launch_fp32<16>(ctx, Xs, qs, ns, d, keep, K2, cs); break;
+        case 24: launch_fp32<24>(ctx, Xs, qs, ns, d, keep, K2, cs); break;
+        case 32: launch_fp32<32>(ctx, Xs, qs, ns, d, keep, K2, cs); break;
+        case 40: launch_fp32<40>(ctx, Xs, qs, ns, d, keep, K2, cs); break;
+        case 48: launch_fp32<48>(ctx, Xs, qs, ns, d, keep, K2, cs); break;
+        case 56: launch_fp32<56>(ctx, Xs, qs, ns, d, keep, K2, cs); break;
+        case 64: launch_fp32<64>(ctx, Xs, qs, ns, d, keep, K2, cs); break;
         default: sv_throw(SV_ERR_UNSUPPORTED, "padded dimension %d", dp);
       }
       if (o > 0)

@@ -167,3 +167,36 @@ def test_bounded_wait_runs_out_and_context_survives(sv, ctx, O):
     X = np.random.default_rng(9).standard_normal((2000, 16))
     idx, _ = sv.ann(X, 5, precision="bf16", ctx=ctx)
     assert _check_sets(idx, X, 5, True, "euclidean", O=O) == 0
+
+
+def _fma_keys(X):
+    """|p|^2 - 2 q.p of integer points as FP32 chains over the dimensions: products and
+    sums of integers are exact in FP64, so one rounding a step is the FMA's."""
+    X = X.astype(np.float64)
+    sq = np.zeros(len(X))
+    for c in range(X.shape[1]):
+        sq = (sq + X[:, c] ** 2).astype(np.float32).astype(np.float64)
+    K = np.repeat(sq[None, :], len(X), axis=0)
+    for c in range(X.shape[1]):
+        K = (K - 2.0 * X[:, c][:, None] * X[:, c][None, :]).astype(np.float32).astype(np.float64)
+    return K
+
+
+@pytest.mark.parametrize("include_self", [True, False])
+@pytest.mark.parametrize("offset", [300, 500, 1000])
+@pytest.mark.parametrize("n,k", [(600, 20), (2500, 8), (2500, 20)])
+def test_shortlist_far_from_the_origin(sv, ctx, n, k, offset, include_self):
+    """Far from the origin the FP32 keys cancel and the re-rank works on a shortlist that is
+    partly wrong: 32 candidates up to k = 16, 64 above, the point itself among them when it
+    is its own neighbour; ties by index."""
+    d, short = 50, 32 if k <= 16 else 64
+    X = np.round(2.0 * np.random.default_rng(offset).normal(size=(n, d))) + offset
+    K = _fma_keys(X)
+    np.fill_diagonal(K, -np.inf if include_self else np.inf)
+    near = np.argsort(K, axis=1, kind="stable")[:, :short]
+    d2 = ((X[near] - X[:, None]) ** 2).sum(axis=2)             # integers: exact in FP32 as well
+    d2[near == np.arange(n)[:, None]] = -1.0
+    order = np.lexsort((near, d2), axis=1)[:, :k]
+    ref = np.take_along_axis(near, order, axis=1)
+    idx, dist = sv.ann(X.astype(np.float32), k, include_self=include_self, precision="fp32", ctx=ctx)
+    assert np.array_equal(idx - 1, ref)
