@@ -17,6 +17,7 @@
 #include "sv_internal.cuh"
 #include "sv_knn_order.cuh"
 #include <float.h>
+#include <type_traits>
 
 int sv_knn_tc_candidates(sv_context* ctx, const float* X32, const float* sq, int64_t n, int dp, int d,
                          int K2, int include_self, int32_t* cand,
@@ -28,7 +29,12 @@ namespace {
 constexpr int KNN_THREADS = 256;
 constexpr int KNN_TILE = 64;       // points per tile and queries per block
 constexpr int KNN_LIST = 64;       // most candidates of a query (the length of its sorted list)
-constexpr int64_t KNN_ORDER_MIN = 2048;
+constexpr int KNN_MERGE = 2;       // queries merged at a time
+// Points from which the order and the tile lists pay (they take 0.2-0.3 ms up to
+// 10,000 points): in 50 dimensions, k = 8, in 60 clusters 4,000 points 0.41 ms
+// without and 0.50 with, 10,000 1.01 and 0.69, 30,000 4.8 and 1.3; without clusters
+// 1.01 and 1.26, 4.8 and 5.2.
+constexpr int64_t KNN_ORDER_MIN = 8192;
 
 // X (n x d, column-major, leading dim ld, FP32 or FP64) -> row-major FP32 [n][dp]
 // (optionally unit-normalised rows for the cosine metric) and squared norms.
@@ -93,24 +99,30 @@ __device__ __forceinline__ float key_float(unsigned b) {
   return __uint_as_float((b & 0x80000000u) ? (b & 0x7fffffffu) : ~b);
 }
 
-// 64 values over a warp, element lane + 32 r in v[r]: the compare-exchange of
-// element e with e ^ stride, ascending where (e & dir) == 0
-__device__ __forceinline__ void w64_step(unsigned long long (&v)[2], int stride, int dir) {
+// M times 64 values over a warp, element lane + 32 r in v[.][r]: the compare-exchange
+// of element e with e ^ stride, ascending where (e & dir) == 0
+template <int M>
+__device__ __forceinline__ void w64_step(unsigned long long (&v)[M][2], int stride, int dir) {
   const int lane = threadIdx.x & 31;
   if (stride == 32) {
     const bool up = (lane & dir) == 0;
-    if ((v[0] > v[1]) == up) {
-      const unsigned long long t = v[0];
-      v[0] = v[1];
-      v[1] = t;
+#pragma unroll
+    for (int i = 0; i < M; ++i) {
+      const unsigned long long x = v[i][0], y = v[i][1];
+      const bool keep = (x < y) == up;
+      v[i][0] = keep ? x : y;
+      v[i][1] = keep ? y : x;
     }
     return;
   }
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
-    const unsigned long long o = __shfl_xor_sync(0xffffffffu, v[r], stride);
-    const bool up = ((lane + 32 * r) & dir) == 0, low = (lane & stride) == 0;
-    if ((low == up) ? o < v[r] : o > v[r]) v[r] = o;
+    const bool least = (((lane + 32 * r) & dir) == 0) == ((lane & stride) == 0);
+#pragma unroll
+    for (int i = 0; i < M; ++i) {
+      const unsigned long long o = __shfl_xor_sync(0xffffffffu, v[i][r], stride);
+      v[i][r] = (o < v[i][r]) == least ? o : v[i][r];
+    }
   }
 }
 
@@ -125,8 +137,12 @@ __device__ __forceinline__ void w64_step(unsigned long long (&v)[2], int stride,
 // a list of the tiles by their lower bound (sv_knn_order) the scan ends at the
 // first tile beyond every query's threshold + |q|^2 + a margin for the keys' FP32
 // rounding (2^-15 (|q|^2 + max |p|^2), several times its bound).
-// 30,011 points in 50 dimensions, 40 candidates: 1.5 ms (2.4 ms with the boxes'
-// bound alone); a query per thread with 64 candidates in registers over every
+// A merge is a chain of 27 shuffled compare-exchanges, and with few blocks, or in
+// a scan's first tiles, where most keys pass, the warps wait for it: a warp merges
+// two queries at a time (500 points in 50 dimensions, 64 candidates: 0.36 -> 0.12
+// ms; 30,000 without a list: 8.6 -> 5.1 ms; four at a time are 3% slower).
+// 30,000 points in 60 clusters x 50 dimensions, 64 candidates, with lists: 0.9 ms
+// for the tiles; a query per thread with 64 candidates in registers over every
 // tile, 235 blocks of four warps, took 7.5 ms.
 template <int DP>
 __global__ void __launch_bounds__(KNN_THREADS, 2) k_knn_fp32(
@@ -141,6 +157,7 @@ __global__ void __launch_bounds__(KNN_THREADS, 2) k_knn_fp32(
   __shared__ unsigned long long thr64[KNN_TILE];
   __shared__ int cnt[KNN_TILE], pid[KNN_TILE];
   __shared__ float bound[KNN_TILE], wm[KNN_THREADS / 32];
+  static_assert(KNN_TILE / (KNN_THREADS / 32) == 8, "a warp's queries");
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, tx = tid & 15, ty = tid >> 4;
   const int64_t ntiles = (n + KNN_TILE - 1) / KNN_TILE;
   const int own = blockIdx.x;
@@ -171,43 +188,68 @@ __global__ void __launch_bounds__(KNN_THREADS, 2) k_knn_fp32(
   unsigned long long e0 = list ? list[0] : 0;
   int64_t t = list ? knn_list_tile(e0, own) : 0;
   if (t != own) fetch(t);
-  // merges a query's buffer into its list (a warp)
-  auto merge = [&](int q) {
-    unsigned long long* L = ent + (size_t)q * 2 * KNN_LIST;
-    const int m = min(cnt[q], KNN_LIST);
-    unsigned long long b[2], a[2];
+  // merges the buffers of M queries into their lists (a warp)
+  auto merge = [&](auto m_tag, unsigned& need) {
+    constexpr int M = decltype(m_tag)::value;
+    unsigned long long a[M][2], b[M][2];
+    int q[M];
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      a[r] = L[lane + 32 * r];
-      b[r] = lane + 32 * r < m ? L[KNN_LIST + lane + 32 * r] : ~0ull;
+    for (int i = 0; i < M; ++i) {
+      q[i] = w + 8 * (__ffs(need) - 1);             // the last one again when there are fewer
+      if (need & (need - 1)) need &= need - 1;
+      else if (i == M - 1) need = 0;
+      const unsigned long long* L = ent + (size_t)q[i] * 2 * KNN_LIST;
+      const int m = min(cnt[q[i]], KNN_LIST);
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        a[i][r] = L[lane + 32 * r];
+        b[i][r] = lane + 32 * r < m ? L[KNN_LIST + lane + 32 * r] : ~0ull;
+      }
     }
 #pragma unroll
     for (int k = 2; k <= 64; k <<= 1)
 #pragma unroll
       for (int s = k >> 1; s > 0; s >>= 1) w64_step(b, s, k);
     // the 64 smallest of two ascending sequences: min(a[e], b[63 - e]), bitonic
-    const unsigned long long r0 = __shfl_sync(0xffffffffu, b[1], 31 - lane);
-    const unsigned long long r1 = __shfl_sync(0xffffffffu, b[0], 31 - lane);
-    a[0] = a[0] < r0 ? a[0] : r0;
-    a[1] = a[1] < r1 ? a[1] : r1;
+#pragma unroll
+    for (int i = 0; i < M; ++i) {
+      const unsigned long long r0 = __shfl_sync(0xffffffffu, b[i][1], 31 - lane);
+      const unsigned long long r1 = __shfl_sync(0xffffffffu, b[i][0], 31 - lane);
+      a[i][0] = a[i][0] < r0 ? a[i][0] : r0;
+      a[i][1] = a[i][1] < r1 ? a[i][1] : r1;
+    }
 #pragma unroll
     for (int s = 32; s > 0; s >>= 1) w64_step(a, s, 64);
-    L[lane] = a[0];
-    L[lane + 32] = a[1];
-    const unsigned long long last = keep > 32 ? a[1] : a[0];
-    if (lane == ((keep - 1) & 31)) {
-      if (last != ~0ull) {
-        thr[q] = key_float((unsigned)(last >> 32));
-        thr64[q] = last;
-      }
-      cnt[q] = 0;
-      const int64_t qi = own * (int64_t)KNN_TILE + q;
-      if (last != ~0ull && qi < n) {
-        const float v = thr[q] + sqt[qi] + 0x1p-15f * (sqt[qi] + __uint_as_float(*pmax));
-        bound[q] = v != v ? __int_as_float(0x7f800000) : v;   // no bound from a NaN
+#pragma unroll
+    for (int i = 0; i < M; ++i) {
+      unsigned long long* L = ent + (size_t)q[i] * 2 * KNN_LIST;
+      L[lane] = a[i][0];
+      L[lane + 32] = a[i][1];
+      const unsigned long long last = keep > 32 ? a[i][1] : a[i][0];
+      if (lane == ((keep - 1) & 31)) {
+        if (last != ~0ull) {
+          thr[q[i]] = key_float((unsigned)(last >> 32));
+          thr64[q[i]] = last;
+        }
+        cnt[q[i]] = 0;
+        const int64_t qi = own * (int64_t)KNN_TILE + q[i];
+        if (last != ~0ull && qi < n) {
+          const float v = thr[q[i]] + sqt[qi] + 0x1p-15f * (sqt[qi] + __uint_as_float(*pmax));
+          bound[q[i]] = v != v ? __int_as_float(0x7f800000) : v;   // no bound from a NaN
+        }
       }
     }
     __syncwarp();
+  };
+  // merges the buffers with more than `above` entries; true when there were any
+  auto settle = [&](int above) {
+    unsigned need = __ballot_sync(0xffffffffu, lane < 8 && cnt[w + 8 * (lane & 7)] > above);
+    if (!need) return false;
+    while (need) {
+      if (need & (need - 1)) merge(std::integral_constant<int, KNN_MERGE>(), need);
+      else merge(std::integral_constant<int, 1>(), need);
+    }
+    return true;
   };
   for (int64_t it = 0; it < ntiles; ++it) {
     __syncthreads();                                // the previous tile is done with Pt
@@ -287,13 +329,7 @@ __global__ void __launch_bounds__(KNN_THREADS, 2) k_knn_fp32(
         }
       }
       const int again = __syncthreads_or(todo != 0);
-      bool did = false;
-      for (int q = w; q < KNN_TILE; q += KNN_THREADS / 32)
-        if (cnt[q] > KNN_LIST / 2) {
-          merge(q);
-          did = true;
-        }
-      if (did) {
+      if (settle(KNN_LIST / 2)) {
         float v = lane < KNN_TILE / (KNN_THREADS / 32) ? bound[w + lane * (KNN_THREADS / 32)] : -FLT_MAX;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -304,11 +340,10 @@ __global__ void __launch_bounds__(KNN_THREADS, 2) k_knn_fp32(
     }
   }
   __syncthreads();
+  settle(0);
   for (int q = w; q < KNN_TILE; q += KNN_THREADS / 32) {
     const int64_t qi = own * (int64_t)KNN_TILE + q;
     if (qi >= n) break;
-    if (cnt[q] > 0) merge(q);
-    __syncwarp();
     const unsigned long long* L = ent + (size_t)q * 2 * KNN_LIST;
     int32_t* o = cand + (int64_t)orig[qi] * K2;
     for (int k = lane; k < K2; k += 32) o[k] = k >= keep || L[k] == ~0ull ? -1 : (int32_t)(unsigned)L[k];

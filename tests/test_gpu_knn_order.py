@@ -67,3 +67,26 @@ def test_non_finite_points_do_not_hide_others(sv, ctx):
     _, dist = sv.ann(X, 8, precision="fp32", ctx=ctx)
     ref = _brute(X[ok], 8, "euclidean", True)
     assert not np.any(np.abs(dist[ok] - ref) > 1e-3)
+
+
+@pytest.mark.parametrize("n,d,k,shape,metric,inc", [
+    (8191, 50, 16, "clusters", "euclidean", True), (8192, 50, 17, "clusters", "euclidean", False),
+    (8193, 9, 32, "one", "cosine", True), (9025, 61, 20, "clusters", "cosine", False),
+    (12001, 64, 8, "clusters", "euclidean", True), (12031, 33, 30, "equal", "euclidean", True)])
+def test_lists_where_they_begin(sv, ctx, n, d, k, shape, metric, inc):
+    """Both sides of the line (8,192 points) from which the FP32 search orders its points."""
+    X = _points(n, d, shape, np.random.default_rng(n + d))
+    idx, dist = sv.ann(X, k, metric=metric, include_self=inc, precision="fp32", ctx=ctx)
+    rows = np.unique(np.r_[0:130, np.random.default_rng(1).integers(0, n, 600), n - 130:n])
+    Y = X.astype(np.float64)
+    if metric == "cosine":
+        Y = Y / np.linalg.norm(Y, axis=1, keepdims=True)
+    d2 = (Y[rows] ** 2).sum(1)[:, None] + (Y * Y).sum(1) - 2 * Y[rows] @ Y.T
+    d2[np.arange(len(rows)), rows] = -1.0 if inc else np.inf
+    d2 = np.maximum(np.sort(np.partition(d2, k, axis=1)[:, :k], axis=1), 0)
+    ref = d2 / 2 if metric == "cosine" else np.sqrt(d2)
+    # FP32 sums of at most 64 squared differences of coordinates up to ~30
+    tol = 2e-5 * max(1.0, np.abs(X).max()) if metric == "euclidean" else 2e-6
+    assert not np.any(np.abs(dist[rows] - ref) > tol + 1e-5 * ref)
+    own = np.arange(1, n + 1)
+    assert np.array_equal(idx[:, 0], own) if inc else not np.any(idx == own[:, None])
