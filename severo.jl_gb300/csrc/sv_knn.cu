@@ -435,7 +435,8 @@ template <int DP>
 void launch_fp32(sv_context* ctx, const float* X, const float* sq, int64_t n, int d, int keep, int K2, int32_t* cand) {
   const int64_t ntiles = (n + KNN_TILE - 1) / KNN_TILE, npad = ntiles * KNN_TILE;
   KnnOrder ord;
-  const bool listed = n >= KNN_ORDER_MIN && sv_knn_order(ctx, X, n, DP, d, KNN_TILE, KNN_TILE, ord);
+  const bool listed = n >= KNN_ORDER_MIN && sv_knn_order(ctx, X, n, DP, d, KNN_TILE, KNN_TILE,
+                                                         sv_knn_spread(ctx, X, n, DP, d), ord);
   DevBuf<float> Xt((size_t)npad * DP), sqt(npad);
   DevBuf<int> orig(npad);
   DevBuf<unsigned> pmax(1);

@@ -30,6 +30,14 @@ namespace {
 constexpr int PV_MAX = 1024;       // most pivots
 constexpr int PV_TILE = 64;        // pivots staged at a time
 constexpr int PV_THREADS = 128;
+constexpr int PV_SAMPLE = 2048;    // points whose nearest pivot's distance is looked at
+// The tensor-core search takes the lists while the squared distance to the nearest
+// pivot is, on average, below this part of that between two points.  List against
+// widest dimension, kernels of the whole search, 300,000 points, k = 20: 0.035 (60
+// far clusters) 7.0 and 11.1 ms; 0.094 (30 near ones, 20 dimensions) 10.1 and 13.8;
+// 0.138 (uniform, 8 dimensions) 17.5 and 17.5; 0.21 (normal, 10) 22.9 and 22.9; 0.38
+// (normal, falling scales, 50) 25.4 and 20.7; 0.55 (normal, 50) 30.9 and 27.5.
+constexpr double PV_NEAR = 0.125;
 
 // Per-dimension sums and sums of squares (FP64, atomics: only the choice of the
 // widest dimension depends on them).
@@ -135,21 +143,23 @@ __global__ void __launch_bounds__(PV_MAX) k_pivots(const float* __restrict__ X, 
 }
 
 // Sort key of every point: its half (if any), its nearest pivot's place, then its
-// widest coordinate.
+// widest coordinate.  near (optional): instead, of every step-th point the squared
+// distance to the nearest pivot.
 template <int DP>
 __global__ void __launch_bounds__(PV_THREADS) k_pivot_assign(const float* __restrict__ X, int64_t n,
                                                              const float* __restrict__ rows,
                                                              const float* __restrict__ norms, int P, int dim,
                                                              const unsigned char* __restrict__ half,
                                                              unsigned long long* __restrict__ key,
-                                                             int* __restrict__ val) {
+                                                             int* __restrict__ val, int64_t step,
+                                                             float* __restrict__ near) {
   __shared__ __align__(16) float tile[PV_TILE * DP];
   __shared__ float tn[PV_TILE];
   const int64_t i = (int64_t)blockIdx.x * PV_THREADS + threadIdx.x;
   float q[DP];
 #pragma unroll
   for (int c = 0; c < DP; c += 4) {
-    const float4 v = i < n ? *(const float4*)(X + i * DP + c) : make_float4(0, 0, 0, 0);
+    const float4 v = i < n ? *(const float4*)(X + i * step * DP + c) : make_float4(0, 0, 0, 0);
     q[c] = -2.f * v.x;
     q[c + 1] = -2.f * v.y;
     q[c + 2] = -2.f * v.z;
@@ -188,7 +198,12 @@ __global__ void __launch_bounds__(PV_THREADS) k_pivot_assign(const float* __rest
         }
     }
   }
-  if (i < n) {
+  if (i < n && near) {
+    float s = 0.f;
+#pragma unroll
+    for (int c = 0; c < DP; ++c) s = fmaf(0.25f * q[c], q[c], s);
+    near[i] = fmaxf(bd + s, 0.f);
+  } else if (i < n) {
     const unsigned place = (unsigned)best | (half && half[i] ? 0x80000000u : 0u);
     key[i] = ((unsigned long long)place << 32) | ordered_bits(X[i * DP + dim]);
     val[i] = (int)i;
@@ -427,40 +442,64 @@ __global__ void k_tile_lists(const float* __restrict__ qlo, const float* __restr
 
 }  // namespace
 
-int sv_knn_widest_dim(sv_context* ctx, const float* X32, int64_t n, int dp, int d) {
+KnnSpread sv_knn_spread(sv_context* ctx, const float* X32, int64_t n, int dp, int d) {
   DevBuf<double> mom(2 * dp);
   sv_memset(ctx, mom.get(), 0, 2 * dp * 8);
   sv_launch(ctx, "knn_order", k_dim_moments, dim3(sv_grid_for(ctx, n, 256, 2)), dim3(256 / dp * dp), 0, X32, n, dp,
             mom.get());
   std::vector<double> hm(2 * dp);
   sv_d2h(ctx, hm.data(), mom.get(), 2 * dp * 8);
-  int dim = 0;
+  KnnSpread s;
   double best = -1;
   for (int c = 0; c < d; ++c) {
     double mean = hm[c] / (double)n, var = hm[dp + c] / (double)n - mean * mean;
+    s.sum += var;
     if (var > best) {
       best = var;
-      dim = c;
+      s.dim = c;
     }
   }
-  return dim;
+  return s;
 }
 
-bool sv_knn_order(sv_context* ctx, const float* X32, int64_t n, int dp, int d, int bq, int bp, KnnOrder& o,
-                  const int* halves_of) {
+bool sv_knn_order(sv_context* ctx, const float* X32, int64_t n, int dp, int d, int bq, int bp,
+                  const KnnSpread& spread, KnnOrder& o, const int* halves_of) {
   const bool bf16 = halves_of != nullptr;
   const int64_t nq = (n + bq - 1) / bq, np = (n + bp - 1) / bp;
   // worth it from a few tiles up; the lists have to fit (sorted in shared memory,
   // kept in 1/4 of what the pool keeps: 4 GB, 4 M points)
   if (np < 4 || np > KNN_MAX_TILES || (size_t)(nq * np) * 8 > ctx->pool->keep / 4) return false;
   const int64_t npad = (np + 63) / 64 * 64;
-  const int dim = sv_knn_widest_dim(ctx, X32, n, dp, d);
   // a cell of about two tiles of 64 points while that takes few pivots (a cluster
   // without one is split among its neighbours' cells), more than 512 only where a
   // cell would hold 2,000 points or more
   const int P = (int)std::max<int64_t>(8, std::min<int64_t>(n >= 1 << 20 ? PV_MAX : PV_MAX / 2, n / 128));
   DevBuf<float> rows((size_t)P * dp), norms(P);
   sv_launch(ctx, "knn_pivots", k_pivots, dim3(1), dim3(PV_MAX), 0, X32, n, dp, P, rows.get(), norms.get());
+  auto assign = [&](int64_t m, int64_t step, const unsigned char* half, unsigned long long* key, int* val,
+                    float* near) {
+    const dim3 g((unsigned)((m + PV_THREADS - 1) / PV_THREADS));
+#define PV_CASE(D)                                                                                             \
+  case D:                                                                                                      \
+    sv_launch(ctx, "knn_assign", k_pivot_assign<D>, g, dim3(PV_THREADS), 0, X32, m, (const float*)rows.get(),   \
+              (const float*)norms.get(), P, spread.dim, half, key, val, step, near);                            \
+    break;
+    switch (dp) {
+      PV_CASE(8) PV_CASE(16) PV_CASE(24) PV_CASE(32) PV_CASE(40) PV_CASE(48) PV_CASE(56) PV_CASE(64)
+      default: sv_throw(SV_ERR_UNSUPPORTED, "padded dimension %d", dp);
+    }
+#undef PV_CASE
+  };
+  if (halves_of) {
+    const int64_t m = std::min<int64_t>(n, PV_SAMPLE);
+    DevBuf<float> near(m);
+    assign(m, n / m, nullptr, nullptr, nullptr, near.get());
+    std::vector<float> hn(m);
+    sv_d2h(ctx, hn.data(), near.get(), m * 4);
+    double sum = 0;
+    for (float v : hn) sum += v;
+    if (!(sum / (double)m < PV_NEAR * 2 * spread.sum)) return false;
+  }
   int64_t n2 = 2048;
   while (n2 < n) n2 <<= 1;
   DevBuf<unsigned long long> key(n2);
@@ -470,17 +509,7 @@ bool sv_knn_order(sv_context* ctx, const float* X32, int64_t n, int dp, int d, i
     sv_launch(ctx, "knn_halves", k_halves, dim3(sv_grid_for(ctx, n, 256)), dim3(256), 0, halves_of, n, bp, half.get());
   }
   o.perm.alloc(n2);
-  const dim3 ga((unsigned)((n + PV_THREADS - 1) / PV_THREADS));
-#define PV_CASE(D)                                                                                       \
-  case D:                                                                                                \
-    sv_launch(ctx, "knn_assign", k_pivot_assign<D>, ga, dim3(PV_THREADS), 0, X32, n, (const float*)rows.get(), \
-              (const float*)norms.get(), P, dim, (const unsigned char*)half.get(), key.get(), o.perm.get());                              \
-    break;
-  switch (dp) {
-    PV_CASE(8) PV_CASE(16) PV_CASE(24) PV_CASE(32) PV_CASE(40) PV_CASE(48) PV_CASE(56) PV_CASE(64)
-    default: sv_throw(SV_ERR_UNSUPPORTED, "padded dimension %d", dp);
-  }
-#undef PV_CASE
+  assign(n, 1, half.get(), key.get(), o.perm.get(), nullptr);
   sv_sort_pairs(ctx, key.get(), o.perm.get(), n, n2);
   if (halves_of) {
     DevBuf<int> joined(n);

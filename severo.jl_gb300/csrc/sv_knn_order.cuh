@@ -19,11 +19,16 @@ __device__ __forceinline__ int knn_list_tile(unsigned long long e, int own) {
   return (place & 1u) ? own - (int)(place >> 1) : own + (int)(place >> 1);
 }
 
+// The dimension of largest variance, and the sum of all dimensions' variances.
+struct KnnSpread {
+  int dim = 0;
+  double sum = 0;
+};
+KnnSpread sv_knn_spread(sv_context* ctx, const float* X32, int64_t n, int dp, int d);
 // Orders the points and lists the tiles (bp points) of every block of bq queries;
 // false when the input is too small or too large for it.  halves_of: an order (place
 // -> point) whose tiles' halves are kept, for BF16 operands: bounds of the rounded
-// coordinates; bp is even.
-bool sv_knn_order(sv_context* ctx, const float* X32, int64_t n, int dp, int d, int bq, int bp, KnnOrder& o,
-                  const int* halves_of = nullptr);
-// the dimension of largest variance
-int sv_knn_widest_dim(sv_context* ctx, const float* X32, int64_t n, int dp, int d);
+// coordinates; bp is even; false as well when the points have too little structure
+// for the lists to leave out more than the order along the widest dimension does.
+bool sv_knn_order(sv_context* ctx, const float* X32, int64_t n, int dp, int d, int bq, int bp,
+                  const KnnSpread& spread, KnnOrder& o, const int* halves_of = nullptr);

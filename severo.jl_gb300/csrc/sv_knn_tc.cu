@@ -32,6 +32,10 @@ constexpr int BK = 64;             // padded dimension (BF16 elements, 128 bytes
 constexpr int STAGES = 4;
 constexpr int EPI_WARPS = 8;
 constexpr int THREADS = (2 + EPI_WARPS) * 32;
+// Points from which the order by cells of pivots and its lists can pay: in 60 clusters
+// x 50 dimensions 100,000 points take 2.5 ms with them and 2.2 without (kernels of the
+// whole search), 200,000 4.7 and 6.5.
+constexpr int64_t LIST_MIN = 150000;
 constexpr int KH_MAX = 32;         // most candidates kept per (query, column half)
 constexpr long long TIMEOUT = 4000000000ll;   // cycles (~2 s) per wait
 constexpr int RING = 16;           // tile-sequence slots (> STAGES + 2 tiles in flight)
@@ -644,10 +648,10 @@ int sv_knn_tc_candidates(sv_context* ctx, const float* X32, const float* sq_unus
     // tiles beyond every query's reach are skipped (locality order, folded norms)
     const bool prune = around && fold && !getenv("SV_KNN_NOPRUNE");
     DevBuf<int> perm;
-    int dim = 0;
+    KnnSpread spread;
     if (around) {
       int nseg = segs ? (int)segs->size() - 1 : 1;
-      dim = sv_knn_widest_dim(ctx, X32, n, dp, d);
+      spread = sv_knn_spread(ctx, X32, n, dp, d);
       int64_t n2 = 2048;
       while (n2 < n) n2 <<= 1;
       DevBuf<unsigned long long> key(n2);
@@ -658,16 +662,16 @@ int sv_knn_tc_candidates(sv_context* ctx, const float* X32, const float* sq_unus
         sv_h2d(ctx, doff.get(), segs->data(), segs->size() * 8);
       }
       dim3 kg((unsigned)sv_grid_for(ctx, segs ? n / nseg + 1 : n, 256, 4), (unsigned)nseg);
-      sv_launch(ctx, "knn_order", k_locality_keys, kg, dim3(256), 0, X32, dp, dim,
+      sv_launch(ctx, "knn_order", k_locality_keys, kg, dim3(256), 0, X32, dp, spread.dim,
                 segs ? (const int64_t*)doff.get() : (const int64_t*)nullptr, nseg, n, key.get(), perm.get());
       sv_sort_pairs(ctx, key.get(), perm.get(), n, n2);
     }
-    // one set of points: each half of the tiles by cells of pivots, and tile lists
-    // (300,000 clustered points in 50 dimensions: tiles 14.5 -> 5.3 ms, the order
-    // and the lists 2.3 ms; 10,000 points: 1.12 -> 0.87 ms in all); stacked samples
-    // (a CTA sees its own sample's tiles only): as they are
+    // one set of many points with structure: each half of the tiles by cells of
+    // pivots, and tile lists; stacked samples (a CTA sees its own sample's tiles
+    // only): as they are
     KnnOrder ord;
-    const bool listed = prune && !segs && sv_knn_order(ctx, X32, n, dp, d, BM, BN, ord, perm.get());
+    const bool listed = prune && !segs && n >= LIST_MIN &&
+                        sv_knn_order(ctx, X32, n, dp, d, BM, BN, spread, ord, perm.get());
     if (listed) perm = std::move(ord.perm);
     const int* pm = around ? (const int*)perm.get() : (const int*)nullptr;
     DevBuf<__nv_bfloat16> Xq((size_t)n * BK), Xp;
@@ -683,7 +687,7 @@ int sv_knn_tc_candidates(sv_context* ctx, const float* X32, const float* sq_unus
     if (fold) {
       Xp.alloc((size_t)n * BK);
       sv_launch(ctx, "knn_pack_fold", k_pack_fold, dim3(sv_grid_for(ctx, n * 8, 256, 8)), dim3(256), 0, X32,
-                n, dp, d, Xq.get(), Xp.get(), pm, dim, coord.get(), nrm.get(), pmax.get());
+                n, dp, d, Xq.get(), Xp.get(), pm, spread.dim, coord.get(), nrm.get(), pmax.get());
     } else {
       sv_launch(ctx, "knn_pack_bf16", k_pack_bf16, dim3(sv_grid_for(ctx, npad, 256, 8)), dim3(256), 0,
                 X32, n, dp, npad, Xq.get(), sq.get(), pm);
