@@ -101,6 +101,9 @@ int  sv_device_memory(sv_context* ctx, size_t* free_bytes, size_t* total_bytes);
  * the context's status word, the context staying usable (no reference
  * counterpart: it exercises this library's failure path without a fault). */
 int  sv_selftest_wait_timeout(sv_context* ctx, long long cycles);
+/* Test hook: frees both count matrices on another thread while the context's
+ * stream is being captured; *nodes = the operations that the graph holds (1). */
+int  sv_selftest_free_in_capture(sv_context* ctx, sv_counts* a, sv_counts* b, int64_t* nodes);
 
 /* ---- count matrix ------------------------------------------------------------
  * sv_counts_upload_csc replaces holding the CountMatrix of src/Severo.jl:26-27

@@ -87,6 +87,7 @@ SIGNATURES = {
     "sv_loess_vertices": (i64, [vp, i64, C.c_double, vp, i64]),
     "sv_normalize_cells": (i32, [vp, vp, i32, dbl, i32, P(vp)]),
     "sv_selftest_wait_timeout": (i32, [vp, C.c_longlong]),
+    "sv_selftest_free_in_capture": (i32, [vp, vp, vp, P(i64)]),
     "sv_centered_gram": (i32, [vp, vp, vp, dbl, dbl, vp]),
     "sv_sparse_mul_spvec": (i32, [vp, i64, i64, vp, vp, vp, i64, vp, vp, i32, dbl, dbl, vp]),
     "sv_sparse_mul_sparse": (i32, [vp, i64, i64, i64, vp, vp, vp, i32, vp, vp, vp, i32, dbl, dbl, vp]),

@@ -101,12 +101,35 @@ void* SvPool::alloc(size_t bytes) {
 void SvPool::free(void* p, size_t bytes) {
   std::lock_guard<std::mutex> lk(mu);
   cudaSetDevice(device);
+  if (held) {
+    try {
+      waiting.emplace_back(p, bytes);
+    } catch (...) {   // no host memory for the note: the pool's end gives the block back
+    }
+    return;
+  }
+  give_back(p, bytes);
+}
+
+void SvPool::hold() {
+  std::lock_guard<std::mutex> lk(mu);
+  held = true;
+}
+
+void SvPool::let_go() {
+  std::lock_guard<std::mutex> lk(mu);
+  held = false;
+  for (auto& w : waiting) give_back(w.first, w.second);
+  waiting.clear();
+}
+
+void SvPool::give_back(void* p, size_t bytes) {
   if (direct(bytes)) {
     if (alive) cudaStreamSynchronize(stream);   // what still uses the block
     cudaFree(p);
   } else if (alive) {
-    account(-(int64_t)bytes);
-    cudaFreeAsync(p, stream);
+    if (cudaFreeAsync(p, stream) == cudaSuccess) account(-(int64_t)bytes);
+    else cudaGetLastError();
   } else {
     cudaFree(p);
     cudaMemPoolTrimTo(pool, 0);
@@ -123,6 +146,34 @@ void SvPool::close() {
 
 SvPool::~SvPool() {
   if (pool) cudaMemPoolDestroy(pool);
+}
+
+SvCapture::SvCapture(sv_context* c) : ctx(c), stream(c->stream) {
+  ctx->pool->hold();
+  cudaError_t e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
+  if (e != cudaSuccess) {
+    ctx->pool->let_go();
+    SV_CUDA(e);
+  }
+  open = true;
+}
+
+cudaGraph_t SvCapture::end() {
+  cudaGraph_t graph = nullptr;
+  open = false;
+  cudaError_t e = cudaStreamEndCapture(stream, &graph);
+  ctx->pool->let_go();
+  SV_CUDA(e);
+  return graph;
+}
+
+SvCapture::~SvCapture() {
+  if (!open) return;
+  cudaGraph_t graph = nullptr;
+  cudaStreamEndCapture(stream, &graph);
+  if (graph) cudaGraphDestroy(graph);
+  cudaGetLastError();
+  ctx->pool->let_go();
 }
 
 cudaEvent_t sv_ctx_event(sv_context* ctx) {
@@ -395,6 +446,37 @@ SV_API int sv_context_destroy(sv_context* ctx) {
   if (sv_pool == ctx->pool) sv_pool.reset();
   delete ctx;
   return SV_OK;
+}
+
+// Captures one operation while another thread frees a and b (both are gone
+// afterwards), and runs it: *nodes = what the graph holds.
+SV_API int sv_selftest_free_in_capture(sv_context* ctx, sv_counts* a, sv_counts* b, int64_t* nodes) {
+  SV_TRY
+  sv_ctx_check(ctx);
+  SV_REQUIRE(nodes, "nodes is null");
+  size_t n = 0;
+  cudaGraph_t graph = nullptr;
+  {
+    SvCapture capture(ctx);
+    SV_CUDA(cudaMemsetAsync(ctx->d_status, 0, 256, ctx->stream));
+    std::thread other([=] {
+      sv_counts_free(a);
+      sv_counts_free(b);
+    });
+    other.join();
+    graph = capture.end();
+  }
+  cudaGraphExec_t exec = nullptr;
+  cudaError_t e = cudaGraphGetNodes(graph, nullptr, &n);
+  if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
+  cudaGraphDestroy(graph);
+  SV_CUDA(e);
+  e = cudaGraphLaunch(exec, ctx->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  cudaGraphExecDestroy(exec);
+  SV_CUDA(e);
+  *nodes = (int64_t)n;
+  SV_CATCH
 }
 
 SV_API int sv_synchronize(sv_context* ctx) {

@@ -95,8 +95,15 @@ struct SvPool {
   void account(int64_t delta);
   void* alloc(size_t bytes);
   void free(void* p, size_t bytes);
+  void hold();          // frees wait until let_go: the stream is being captured
+  void let_go();
   void close();         // the context goes away
   ~SvPool();
+
+ private:
+  bool held = false;
+  std::vector<std::pair<void*, size_t>> waiting;
+  void give_back(void* p, size_t bytes);
 };
 // the pool of the context whose call this thread is in (sv_ctx_check)
 extern thread_local std::shared_ptr<SvPool> sv_pool;
@@ -128,6 +135,24 @@ struct sv_context {
   void* h_run = nullptr;
   size_t h_run_bytes = 0;
   std::shared_ptr<SvPool> pool;
+};
+
+// Captures the context's stream from construction to end().  Handles that other
+// threads drop meanwhile keep their blocks until it is over: a free on a capturing
+// stream would become part of the graph, and waiting for the stream would end the
+// capture.
+class SvCapture {
+ public:
+  explicit SvCapture(sv_context* c);
+  cudaGraph_t end();    // what was captured, the caller's
+  ~SvCapture();         // without end(): discards it
+  SvCapture(const SvCapture&) = delete;
+  SvCapture& operator=(const SvCapture&) = delete;
+
+ private:
+  sv_context* ctx;
+  cudaStream_t stream;
+  bool open = false;
 };
 
 void sv_ctx_check(sv_context* ctx);

@@ -2747,8 +2747,7 @@ struct Lanczos {
       // capturing runs the host side of the cycle (basis sets flip) but
       // launches nothing: the launch count is charged per replay instead
       int64_t l0 = ctx->launches;
-      cudaGraph_t graph = nullptr;
-      SV_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+      SvCapture capture(ctx);
       try {
         capturing = ctx->side != nullptr;
         g.matvecs = cycle(restart, k, seed);
@@ -2756,15 +2755,12 @@ struct Lanczos {
       } catch (...) {
         if (capturing && main_stream) ctx->stream = main_stream;
         capturing = false;
-        cudaStreamEndCapture(ctx->stream, &graph);
-        if (graph) cudaGraphDestroy(graph);
-        cudaGetLastError();
         ctx->launches = l0;
         throw;
       }
-      SV_CUDA(cudaStreamEndCapture(ctx->stream, &graph));
       g.launches = ctx->launches - l0;
       ctx->launches = l0;
+      cudaGraph_t graph = capture.end();
       cudaError_t e = cudaGraphInstantiate(&g.exec, graph, 0);
       cudaGraphDestroy(graph);
       if (e != cudaSuccess) {

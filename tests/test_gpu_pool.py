@@ -39,3 +39,30 @@ def test_handles_freed_on_another_thread(sv, O):
         t.join()
         assert np.array_equal(got, ref)
     c.close()
+
+
+@pytest.mark.parametrize("genes,mu", [(200, 1.0), (8000, 20.0)])      # blocks of the pool, and larger ones
+def test_handles_freed_while_the_stream_is_captured(sv, genes, mu):
+    """Blocks that another thread frees during a capture wait for its end: the graph holds
+    what was captured and nothing else, and the memory is given back afterwards."""
+    import ctypes as C
+    c = sv.Context(0)
+    cells = 200000
+    free0, total = c.memory()
+    pair = [sv.CountMatrix.generate(cells, genes, np.full(genes, mu), np.ones(cells), seed=s, ctx=c) for s in (1, 2)]
+    assert (4 * pair[0].nnz > total // 64) == (genes == 8000)
+    h = [p.h for p in pair]
+    for p in pair:
+        p.h = None
+    nodes = C.c_int64()
+    sv._lib.check(c.lib.sv_selftest_free_in_capture(c.h, h[0], h[1], C.byref(nodes)))
+    assert nodes.value == 1
+    assert free0 - c.memory()[0] <= total // 16 + (256 << 20)
+    X = sv.CountMatrix.generate(3000, 2000, np.ones(2000), np.ones(3000), seed=3, ctx=c)   # the context goes on
+    D = sv.normalize_cells(X, scale_factor=1e4, dtype="float32")
+    em = sv.pca(sv.scale_features(D, scale_max=10.0), 5)
+    assert np.all(np.isfinite(em.coordinates))
+    c.close()
+    d = sv.Context(0)
+    assert free0 - d.memory()[0] <= 256 << 20
+    d.close()
