@@ -213,15 +213,25 @@ void* sv_ctx_stage(sv_context* ctx, size_t bytes) {
   return ctx->h_stage;
 }
 
-void* sv_ctx_run_stage(sv_context* ctx, size_t bytes) {
-  if (bytes > ctx->h_run_bytes) {
-    if (ctx->h_run) cudaFreeHost(ctx->h_run);
-    ctx->h_run = nullptr;
-    ctx->h_run_bytes = 0;
-    SV_CUDA(cudaMallocHost(&ctx->h_run, bytes));
-    ctx->h_run_bytes = bytes;
+void* SvRunStage::alloc(sv_context* c, size_t bytes) {
+  if (c->h_run_used.exchange(true)) {
+    SV_CUDA(cudaMallocHost(&own, bytes));
+    return own;
   }
-  return ctx->h_run;
+  kept = c;
+  if (bytes > c->h_run_bytes) {
+    if (c->h_run) cudaFreeHost(c->h_run);
+    c->h_run = nullptr;
+    c->h_run_bytes = 0;
+    SV_CUDA(cudaMallocHost(&c->h_run, bytes));
+    c->h_run_bytes = bytes;
+  }
+  return c->h_run;
+}
+
+SvRunStage::~SvRunStage() {
+  if (own) cudaFreeHost(own);
+  if (kept) kept->h_run_used = false;
 }
 
 void sv_sync(sv_context* ctx) { SV_CUDA(cudaStreamSynchronize(ctx->stream)); }

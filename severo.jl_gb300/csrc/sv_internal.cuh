@@ -14,6 +14,7 @@
 #include <mutex>
 #include <tuple>
 #include <algorithm>
+#include <atomic>
 
 #include "../../include/severo_gpu.h"
 
@@ -131,9 +132,10 @@ struct sv_context {
   // a second stream that captured work forks to and joins from
   cudaStream_t side = nullptr;
   cudaEvent_t fork_ev[2] = {nullptr, nullptr};
-  // pinned read-back area of a Lanczos run (sv_ctx_run_stage)
+  // pinned read-back area of a Lanczos run (SvRunStage)
   void* h_run = nullptr;
   size_t h_run_bytes = 0;
+  std::atomic<bool> h_run_used{false};
   std::shared_ptr<SvPool> pool;
 };
 
@@ -159,9 +161,22 @@ void sv_ctx_check(sv_context* ctx);
 cudaEvent_t sv_ctx_event(sv_context* ctx);
 void sv_ctx_harvest(sv_context* ctx);
 void* sv_ctx_stage(sv_context* ctx, size_t bytes);
-// pinned memory that one Lanczos run at a time uses, kept between runs (apart
-// from the scalar staging buffer, which other reads use meanwhile)
-void* sv_ctx_run_stage(sv_context* ctx, size_t bytes);
+// Pinned memory of one Lanczos run (apart from the scalar staging buffer, which
+// other reads use meanwhile): the context's, kept between runs, or memory of its
+// own while another run has that -- one whose operator calls back to the host may
+// start others from there, and other threads may.
+class SvRunStage {
+ public:
+  void* alloc(sv_context* c, size_t bytes);
+  SvRunStage() = default;
+  ~SvRunStage();
+  SvRunStage(const SvRunStage&) = delete;
+  SvRunStage& operator=(const SvRunStage&) = delete;
+
+ private:
+  sv_context* kept = nullptr;   // whose area it is
+  void* own = nullptr;
+};
 void sv_check_device_status(sv_context* ctx, const char* where);
 
 // Launch a kernel on the context stream; counts launches and, when profiling

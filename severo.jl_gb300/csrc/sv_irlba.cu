@@ -2245,6 +2245,7 @@ struct Lanczos {
   DevBuf<int> active, finsel;
   DevBuf<float> uf;             // the current cell-side vector in FP32 (X^T u's input)
   DevBuf<double> upart;         // and its partial sums
+  SvRunStage stage;
   double* hsum = nullptr;       // pinned copy of the cycle summaries
   int* hflags = nullptr;        // pinned staging of the active / finish masks
   double eps_b = 0;
@@ -2336,7 +2337,7 @@ struct Lanczos {
     Vfin.alloc(n * nu);
     sv_memset(ctx, counter.get(), 0, (4 + nseg) * 4);
     sv_memset(ctx, B.get(), 0, (size_t)nseg * work * work * 8);
-    hsum = (double*)sv_ctx_run_stage(ctx, (size_t)nseg * (2 * work + 2) * 8 + (size_t)nseg * 4);
+    hsum = (double*)stage.alloc(ctx, (size_t)nseg * (2 * work + 2) * 8 + (size_t)nseg * 4);
     hflags = (int*)(hsum + (size_t)nseg * (2 * work + 2));
     op->bind_active(active.get());
     for (auto kern : {k_jacobi_svd<1>, k_jacobi_svd<2>, k_jacobi_svd<3>})

@@ -208,3 +208,50 @@ def test_caller_provided_outputs(sv, ctx, O):
     assert np.array_equal(oi, idx) and np.array_equal(od, dist)
     with pytest.raises(ValueError):
         sv.pca(S, 12, tol=1e-8, init=init, out=np.zeros((2500, 12)))   # row-major
+
+
+def _low_rank(m, n, seed):
+    rng = np.random.default_rng(seed)
+    X = rng.normal(size=(m, n))
+    return X, np.linalg.svd(X, compute_uv=False)
+
+
+def test_irlba_callback_may_run_another(sv):
+    """An operator whose callbacks run irlba themselves, with a larger basis: each run has
+    its own read-back memory."""
+    X, s_out = _low_rank(60, 40, 1)
+    Y, s_in = _low_rank(300, 200, 2)
+    seen = []
+
+    def matvec(x):
+        if len(seen) < 6:
+            seen.append(sv.irlba_callback(lambda v: Y @ v, lambda v: Y.T @ v, 300, 200, 3 + len(seen), tol=1e-9,
+                                          work=20 + 8 * len(seen))[1])
+        return X @ x
+
+    _, s, _ = sv.irlba_callback(matvec, lambda y: X.T @ y, 60, 40, 3, tol=1e-9)
+    assert np.max(np.abs(s - s_out[:3])) < 1e-7 * s_out[0]
+    assert len(seen) == 6
+    for i, t in enumerate(seen):
+        assert np.max(np.abs(t - s_in[:3 + i])) < 1e-7 * s_in[0]
+
+
+def test_irlba_callbacks_in_threads(sv):
+    import threading
+    out, errors = {}, []
+
+    def work(i):
+        try:
+            X, s = _low_rank(80 + 10 * i, 50, i)
+            for _ in range(10):
+                t = sv.irlba_callback(lambda v: X @ v, lambda v: X.T @ v, len(X), 50, 2 + i, tol=1e-9)[1]
+                assert np.max(np.abs(t - s[:2 + i])) < 1e-7 * s[0]
+        except Exception as e:
+            errors.append(repr(e))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors[0]
