@@ -630,7 +630,9 @@ void sv_transpose_counts(sv_context* ctx, int64_t n_major, int64_t n_minor, int6
   const int H = wide ? 8 : 4;
   auto kern = wide ? k_tr_write<8> : k_tr_write<4>;
   const size_t smem = (size_t)TR_WARPS * T * (8 + 4 * H);
-  SV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // what the largest tiles take: the setting is the process's, and other threads'
+  // launches may have larger ones
+  SV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TR_WARPS * TR_MAXT * (8 + 4 * H)));
   sv_launch(ctx, "counts_transpose_write", kern, gt, bt, smem, ptr, idx, cnt, n_major, n_minor, tshift,
             n_tiles, (const int32_t*)toff.get(), per_part, (const int32_t*)part_cnt.get(),
             (const int64_t*)optr.get(), oidx.get(), ocnt.get());

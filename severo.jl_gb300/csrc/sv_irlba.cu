@@ -2282,7 +2282,9 @@ struct Lanczos {
     lag_tma = work <= 64 && !getenv("SV_NO_LAG_TMA");
     if (lag_tma) {
       const size_t dyn = lag_smem(work - 1);
-      SV_CUDA(cudaFuncSetAttribute(k_cgs_lag_tma<LR_STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+      // for any width: the setting is the process's, other threads' runs included
+      SV_CUDA(cudaFuncSetAttribute(k_cgs_lag_tma<LR_STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)lag_smem(63)));
       SV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&lag_per_sm, k_cgs_lag_tma<LR_STAGES>,
                                                             32 * (LR_WARPS + 1), dyn));
     } else if (work <= 64) {

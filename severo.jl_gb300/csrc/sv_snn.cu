@@ -29,6 +29,7 @@ namespace {
 constexpr int CAP_WARP = 1024;
 constexpr int CAP_BLOCK = 16384;
 constexpr int SNN_BLOCK = 256;
+constexpr int SNN_MAX_K = 1024;                  // most neighbours of a list
 constexpr int SLOTS_WARP = 3 * CAP_WARP / 2;     // hash slots per warp (load <= 2/3)
 constexpr int SLOTS_BLOCK = 3 * CAP_BLOCK / 2;   // hash slots per block
 
@@ -588,13 +589,16 @@ void snn_run(sv_context* ctx, const int32_t* nn, int64_t n, int k, int64_t kpara
   const int32_t* rl = rlist.get();
   const int kp = (int)kparam;
   if (hash) {
-    const size_t ws = (size_t)(SNN_BLOCK / 32) * SLOTS_WARP * 4 + wtab, bs = (size_t)SLOTS_BLOCK * 4 + wtab;
-    SV_CUDA(cudaFuncSetAttribute(k_snn_hash_warp<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ws));
-    SV_CUDA(cudaFuncSetAttribute(k_snn_hash_block<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bs));
+    const size_t ws = (size_t)(SNN_BLOCK / 32) * SLOTS_WARP * 4, bs = (size_t)SLOTS_BLOCK * 4;
+    // the most that any call asks for: the setting is the process's, other threads'
+    // launches with other k included
+    const size_t most = (size_t)(SNN_MAX_K + 1) * (sizeof(T) + 1);
+    SV_CUDA(cudaFuncSetAttribute(k_snn_hash_warp<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(ws + most)));
+    SV_CUDA(cudaFuncSetAttribute(k_snn_hash_block<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(bs + most)));
     sv_memset(ctx, used.get(), 0, 8);
-    sv_launch(ctx, "snn_hash_warp", k_snn_hash_warp<T>, dim3(nl[0] ? gw : 0), dim3(SNN_BLOCK), ws, L0, nl[0],
+    sv_launch(ctx, "snn_hash_warp", k_snn_hash_warp<T>, dim3(nl[0] ? gw : 0), dim3(SNN_BLOCK), ws + wtab, L0, nl[0],
               Gp, gc, rp, rl, k, kp, prune, cb, used.get(), arena.get(), kept.get(), at.get(), ctx->d_status);
-    sv_launch(ctx, "snn_hash_block", k_snn_hash_block<T>, dim3(nl[1] ? gb : 0), dim3(1024), bs, L1, nl[1], Gp,
+    sv_launch(ctx, "snn_hash_block", k_snn_hash_block<T>, dim3(nl[1] ? gb : 0), dim3(1024), bs + wtab, L1, nl[1], Gp,
               gc, rp, rl, k, kp, prune, cb, used.get(), arena.get(), kept.get(), at.get(), ctx->d_status);
   }
   const size_t warp_smem = (size_t)(SNN_BLOCK / 32) * CAP_WARP * 4, block_smem = (size_t)CAP_BLOCK * 4;
@@ -749,7 +753,7 @@ SV_API int sv_snn_host(sv_context* ctx, const int32_t* nn_index, int64_t n, int6
   SV_TRY
   sv_ctx_check(ctx);
   SV_REQUIRE(out && nn_index, "null argument");
-  SV_REQUIRE(n >= 1 && n < (1ll << 31) && k >= 1 && k <= 1024, "bad sizes");
+  SV_REQUIRE(n >= 1 && n < (1ll << 31) && k >= 1 && k <= SNN_MAX_K, "bad sizes");
   SV_REQUIRE(dtype == SV_F32 || dtype == SV_F64, "dtype must be F32 or F64");
   DevBuf<int32_t> raw((size_t)n * k), nn((size_t)n * k);
   sv_h2d(ctx, raw.get(), nn_index, (size_t)n * k * 4);

@@ -23,3 +23,30 @@ def test_snn_hash_edges(sv, ctx, O, n, k, hub, dtype, kparam):
     R = O.jaccard_index(O.knn_graph(idx + 1, n), kp, 1 / 15, dtype)
     assert np.array_equal(W.indptr, R.indptr) and np.array_equal(W.indices, R.indices)
     assert np.array_equal(W.data, R.data) and W.data.dtype == R.data.dtype
+
+
+def test_threads_with_other_list_lengths(sv):
+    """Two contexts in two threads, long lists in one and short ones in the other: what a
+    launch asks for in shared memory does not depend on what the other thread set."""
+    import threading
+    lists = {k: np.asfortranarray(np.random.default_rng(k).integers(1, 65, (64, k)).astype(np.int32))
+             for k in (2, 1024)}
+    errors = []
+
+    def work(k):
+        try:
+            c = sv.Context(0)
+            first = sv.jaccard_index(lists[k], k, ctx=c)
+            for _ in range(400):
+                G = sv.jaccard_index(lists[k], k, ctx=c)
+                assert np.array_equal(G.indptr, first.indptr) and np.array_equal(G.data, first.data)
+            c.close()
+        except Exception as e:
+            errors.append(repr(e))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in (2, 1024, 2, 1024)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors[:2]
