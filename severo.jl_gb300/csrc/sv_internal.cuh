@@ -315,6 +315,7 @@ struct sv_centered {
   DevBuf<double> mean, std_, mu;      // nf (FP64)
   DevBuf<float> mu_h, mu_l;           // nf: mu as double-float (the FP64-free products)
   int grid_csr = 1, grid_csr_df = 1;  // resident blocks of the X v kernels (one wave)
+  DevBuf<int64_t> xv_cut;             // grid_csr_df + 1 first rows of the blocks of the streamed X v
   DevBuf<float> inv_std_f, clip_f;    // nf (FP32 form of the scale / clip)
   DevBuf<double> inv_std_d, clip_d;   // nf (FP64 form, for FP64 data)
   // chunk table of the CSC (X^T u) product

@@ -43,3 +43,22 @@ def test_transposed_product_with_few_features(sv, ctx, nf):
     S = sv.CenteredMatrix.from_sparse(X, np.zeros(nf), dtype="float32", ctx=ctx)
     w = rng.integers(-4, 5, n).astype(np.float64)
     assert np.array_equal(S.rmul(w), X.T @ w)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_rows_of_very_different_depth(sv, ctx, dtype):
+    """Empty cells, then shallow ones, then a few with most of the entries: the ranges of rows
+    that the blocks take hold as many entries each."""
+    rng = np.random.default_rng(3)
+    n, nf = 9001, 1500
+    depth = np.r_[np.zeros(3000), np.full(5500, 0.01), np.linspace(0.02, 0.9, 501)]
+    X = np.where(rng.random((n, nf)) < depth[:, None], rng.integers(1, 9, (n, nf)), 0).astype(np.int32)
+    D = sv.normalize_cells(sv.CountMatrix.from_csc(sp.csc_matrix(X), ctx=ctx), scale_factor=1e3, dtype=dtype)
+    S = sv.scale_features(D, scale_max=np.inf)
+    U, s, V = sv.irlba(S, 3, tol=1e-8, seed=1)
+    mu, _, std = S.stats()
+    B = D.to_csc().toarray().astype(np.float64) / std
+    A = B - mu
+    # as in test_rows_of_every_length
+    size = (1.5e-4 * B + 2.0 ** -40 * np.abs(mu)) @ np.abs(V) + 1e-6 * s[0] / np.sqrt(n)
+    assert np.all(np.abs(A @ V - U * s) <= size.max(axis=1)[:, None] + 1e-7 * s[0])
