@@ -767,12 +767,14 @@ __device__ __forceinline__ double clip_above(double v, long long key) {
 // clip)*x).  FP64 form: (1/std, clip, x); a * (1/std) is within one ulp of the
 // reference's a/std (FP64 division is slow on this part).
 // Every block builds the table and mu.x itself from x (a separate one-block
-// kernel preparing the table for all blocks measured no faster); with few rows
-// that is half of the time, so blocks are large.  2,000 cells, FP64: 19.5 -> 16.6 us
-// (256 threads a block, which all did both; FP64 comparisons).
-constexpr int CSR_THREADS = 512;
-template <typename ValT, typename IdxT>
-__global__ void __launch_bounds__(CSR_THREADS) k_spmv_csr(
+// kernel preparing the table for all blocks measured no faster).  Blocks have 256
+// threads but for FP64 values where 512 make it one block per SM and 256 two on some
+// (2,000 features, 256 and 512 threads: 1,000 cells 12.2 and 14.8 us, 1,500 16.6 and
+// 14.7, 2,000 16.3 and 15.1, 3,000 20.7 and 23.0, 20,000 64.6 and 64.8; FP32, 3,000
+// features, 100,000 cells: 98 and 111).
+constexpr int CSR_SUMS = 256;    // threads that sum mu.x: its order
+template <typename ValT, typename IdxT, int THREADS>
+__global__ void __launch_bounds__(THREADS) k_spmv_csr(
     const int64_t* __restrict__ rowptr, const IdxT* __restrict__ hcol, const ValT* __restrict__ hval,
     int64_t n_rows, int64_t nf, const double* __restrict__ x, const float* __restrict__ inv_f,
     const float* __restrict__ clip_f, const double* __restrict__ inv_d,
@@ -783,11 +785,11 @@ __global__ void __launch_bounds__(CSR_THREADS) k_spmv_csr(
   __shared__ double red[32];
   double mux = 0;
   {
-    // half of the threads build the table, the other half mu.x (in the order of
-    // CSR_THREADS / 2 threads), four features per thread in flight
-    constexpr int half = CSR_THREADS / 2;
+    // with 512 threads half of them build the table, the other half mu.x; four
+    // features per thread in flight
+    constexpr int half = CSR_SUMS;
     const int t = threadIdx.x % half;
-    const bool sums = threadIdx.x < half;
+    const bool sums = threadIdx.x < half, builds = THREADS == half || !sums;
     for (int64_t f0 = t; f0 < nf; f0 += 4 * half) {
       double xs[4], ms[4];
       AccT iv[4], cl[4];
@@ -796,23 +798,24 @@ __global__ void __launch_bounds__(CSR_THREADS) k_spmv_csr(
         const int64_t f = f0 + u * half;
         if (f >= nf) break;
         xs[u] = x[f];
-        if (sums) {
-          ms[u] = mu[f];
-        } else if constexpr (sizeof(AccT) == 4) {
-          iv[u] = inv_f[f];
-          cl[u] = clip_f[f];
-        } else {
-          iv[u] = inv_d[f];
-          cl[u] = clip_d[f];
+        if (sums) ms[u] = mu[f];
+        if (builds) {
+          if constexpr (sizeof(AccT) == 4) {
+            iv[u] = inv_f[f];
+            cl[u] = clip_f[f];
+          } else {
+            iv[u] = inv_d[f];
+            cl[u] = clip_d[f];
+          }
         }
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int64_t f = f0 + u * half;
         if (f >= nf) break;
-        if (sums) {
-          mux += ms[u] * xs[u];
-        } else if constexpr (sizeof(AccT) == 4) {
+        if (sums) mux += ms[u] * xs[u];
+        if (!builds) continue;
+        if constexpr (sizeof(AccT) == 4) {
           const float x1 = (float)xs[u];
           const float P = iv[u] * x1;
           const float Q = x1 == 0.f ? 0.f : cl[u] * x1;
@@ -886,6 +889,18 @@ __global__ void __launch_bounds__(CSR_THREADS) k_spmv_csr(
       y[r] = out;
     }
   }
+}
+
+static int csr_threads(sv_context* ctx, int dtype, int64_t n_rows) {
+  const int64_t per_sm = (n_rows + ctx->num_sms - 1) / ctx->num_sms;   // a warp per row
+  return dtype == SV_F64 && per_sm > 8 && per_sm <= 16 ? 512 : 256;
+}
+template <typename ValT, typename IdxT>
+static auto csr_kernel(int threads) {
+  if constexpr (sizeof(ValT) == 8) {
+    if (threads == 512) return k_spmv_csr<ValT, IdxT, 512>;
+  }
+  return k_spmv_csr<ValT, IdxT, 256>;
 }
 
 // ---- X v for the Lanczos W side, double-float in and out (FP32 storage) -------
@@ -1921,9 +1936,10 @@ void sv_centered_apply(sv_context* ctx, const sv_centered* S, char trans, const 
   if (trans == 'N') {
     size_t smem = S->dtype == SV_F64 ? (size_t)S->nf * 24 : (size_t)S->nf * 8;
     smem = (smem + 15) & ~(size_t)15;
-    int grid = (int)std::max<int64_t>(1, std::min<int64_t>(S->grid_csr, (S->n_cells * 32 + CSR_THREADS - 1) / CSR_THREADS));
+    const int threads = csr_threads(ctx, S->dtype, S->n_cells);
+    int grid = (int)std::max<int64_t>(1, std::min<int64_t>(S->grid_csr, (S->n_cells * 32 + threads - 1) / threads));
 #define LAUNCH_CSR(VT, IT, COL)                                                                  \
-  sv_launch(ctx, "spmv_csr_h", k_spmv_csr<VT, IT>, dim3(grid), dim3(CSR_THREADS), smem,          \
+  sv_launch(ctx, "spmv_csr_h", csr_kernel<VT, IT>(threads), dim3(grid), dim3(threads), smem,     \
             (const int64_t*)S->h_rowptr.get(), (const IT*)COL, (const VT*)S->h_val.get(),         \
             S->n_cells, S->nf, x, (const float*)S->inv_std_f.get(), (const float*)S->clip_f.get(), \
             (const double*)S->inv_std_d.get(), (const double*)S->clip_d.get(),                    \
@@ -2328,8 +2344,8 @@ static sv_centered* make_centered(sv_context* ctx, const sv_data* data, const st
       S->red_partial.alloc(std::max<int64_t>(UPREP_BLOCKS, S->t_blocks));
     }
 #define SET_SMEM(VT, IT)                                                                         \
-  SV_CUDA(cudaFuncSetAttribute(k_spmv_csr<VT, IT>, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
-                               200 * 1024))
+  for (int th : {256, 512})                                                                       \
+    SV_CUDA(cudaFuncSetAttribute(csr_kernel<VT, IT>(th), cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024))
     SET_SMEM(double, uint16_t);
     SET_SMEM(double, int32_t);
     SET_SMEM(float, uint16_t);
@@ -2348,25 +2364,26 @@ static sv_centered* make_centered(sv_context* ctx, const sv_data* data, const st
       size_t tsm_df = ((size_t)nf * 8 + 15) & ~(size_t)15;
       int b1 = 0, b2 = 0;
       bool small16 = nf <= 65536;
+      const int th = csr_threads(ctx, data->dtype, C->n_cells);
       switch (data->dtype) {
         case SV_F64:
           SV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-              &b1, small16 ? (const void*)k_spmv_csr<double, uint16_t> : (const void*)k_spmv_csr<double, int32_t>,
-              CSR_THREADS, tsm));
+              &b1, small16 ? (const void*)csr_kernel<double, uint16_t>(th) : (const void*)csr_kernel<double, int32_t>(th),
+              th, tsm));
           break;
         case SV_F32:
           SV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-              &b1, small16 ? (const void*)k_spmv_csr<float, uint16_t> : (const void*)k_spmv_csr<float, int32_t>,
-              CSR_THREADS, tsm));
+              &b1, small16 ? (const void*)csr_kernel<float, uint16_t>(th) : (const void*)csr_kernel<float, int32_t>(th),
+              th, tsm));
           SV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
               &b2, small16 ? (const void*)k_spmv_csr_df<float, uint16_t> : (const void*)k_spmv_csr_df<float, int32_t>,
               256, tsm_df));
           break;
         default:
           SV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-              &b1, small16 ? (const void*)k_spmv_csr<__nv_bfloat16, uint16_t>
-                           : (const void*)k_spmv_csr<__nv_bfloat16, int32_t>,
-              CSR_THREADS, tsm));
+              &b1, small16 ? (const void*)csr_kernel<__nv_bfloat16, uint16_t>(th)
+                           : (const void*)csr_kernel<__nv_bfloat16, int32_t>(th),
+              th, tsm));
           SV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
               &b2, small16 ? (const void*)k_spmv_csr_df<__nv_bfloat16, uint16_t>
                            : (const void*)k_spmv_csr_df<__nv_bfloat16, int32_t>,
