@@ -588,6 +588,15 @@ void sv_transpose_counts(sv_context* ctx, int64_t n_major, int64_t n_minor, int6
                          const int64_t* ptr, const int32_t* idx, const int32_t* cnt,
                          DevBuf<int64_t>& optr, DevBuf<int32_t>& oidx, DevBuf<int32_t>& ocnt,
                          const char* where) {
+  SV_REQUIRE(n_minor > 0 || nnz == 0, "%s: an index is out of range", where);
+  if (n_minor == 0) {   // nothing to place: no tiles to share out
+    optr.alloc(1);
+    sv_memset(ctx, optr.get(), 0, 8);
+    oidx.alloc(0);
+    ocnt.alloc(0);
+    sv_sync(ctx);
+    return;
+  }
   // tile size: enough warps to fill the device (~8 tiles per SM slot), tile
   // offsets bounded to ~2 GB
   int tshift = 8;

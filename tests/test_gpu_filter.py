@@ -89,3 +89,14 @@ def test_select_cells_is_a_row_slice(sv, ctx, O):
     R = sp.csc_matrix(sp.csr_matrix(X)[120:455])
     _same(D.to_csc(), R)
     _same(D.to_csr().tocsc(), R)
+
+
+def test_filters_that_leave_nothing(sv, ctx):
+    """No cells, no genes, neither: matrices of that shape (a transpose without output
+    segments has no tiles to share out)."""
+    X = sp.random(300, 50, 0.3, format="csc", random_state=1, data_rvs=lambda k: np.ones(k))
+    c = sv.CountMatrix.from_csc(X.astype(np.int32), ctx=ctx)
+    for kw, shape in ((dict(min_features=1000), (0, 50)), (dict(min_cells=1000), (300, 0)),
+                      (dict(min_features=1000, min_cells=1000), (0, 0))):
+        Y = sv.filter_counts(c, **kw)[0]
+        assert Y.shape == shape and Y.nnz == 0
