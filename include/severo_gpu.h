@@ -76,6 +76,10 @@ int  sv_last_error(char* buf, size_t len);               /* copies the message, 
 int  sv_context_create(int device, sv_context** out);
 int  sv_context_destroy(sv_context* ctx);
 int  sv_synchronize(sv_context* ctx);
+/* Gives the device memory that the context keeps between calls (at most 1/16 of
+ * the device's) back to it, for other users of the device: other libraries of the
+ * process, other processes.  Waits for the context's work. */
+int  sv_context_trim(sv_context* ctx);
 /* Pin (page-lock) caller memory so that uploads run at full link speed. */
 int  sv_host_register(void* ptr, size_t bytes);
 int  sv_host_unregister(void* ptr);

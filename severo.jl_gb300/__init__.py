@@ -78,6 +78,10 @@ class Context:
     def sync(self):
         L.check(self.lib.sv_synchronize(self.h))
 
+    def trim(self):
+        """Gives the device memory kept between calls back to the device."""
+        L.check(self.lib.sv_context_trim(self.h))
+
     def mark(self, slot):
         L.check(self.lib.sv_mark(self.h, slot))
 

@@ -58,6 +58,7 @@ SIGNATURES = {
     "sv_last_error": (i32, [C.c_char_p, C.c_size_t]),
     "sv_context_create": (i32, [i32, P(vp)]),
     "sv_context_destroy": (i32, [vp]),
+    "sv_context_trim": (i32, [vp]),
     "sv_synchronize": (i32, [vp]),
     "sv_host_register": (i32, [vp, C.c_size_t]),
     "sv_host_unregister": (i32, [vp]),

@@ -58,14 +58,41 @@ void SvPool::account(int64_t delta) {
   threshold = (size_t)want;
 }
 
+// The pools of the process's contexts: memory that one of them keeps is there for
+// another's allocation.  (Never destroyed: contexts may outlive static objects.)
+static std::mutex& pools_mu() {
+  static std::mutex* m = new std::mutex();
+  return *m;
+}
+static std::vector<std::shared_ptr<SvPool>>& pools() {
+  static auto* v = new std::vector<std::shared_ptr<SvPool>>();
+  return *v;
+}
+
+static void trim_pools(int device) {
+  std::vector<std::shared_ptr<SvPool>> all;
+  {
+    std::lock_guard<std::mutex> lk(pools_mu());
+    all = pools();
+  }
+  for (auto& p : all)
+    if (p->device == device) p->trim();
+}
+
+void SvPool::trim() {
+  std::lock_guard<std::mutex> lk(mu);
+  if (!alive || held) return;
+  cudaStreamSynchronize(stream);   // its frees take effect
+  cudaMemPoolTrimTo(pool, 0);
+}
+
 void* SvPool::alloc(size_t bytes) {
   void* p = nullptr;
   if (direct(bytes)) {
     cudaError_t e = cudaMalloc(&p, bytes);
     if (e == cudaErrorMemoryAllocation) {
       cudaGetLastError();
-      cudaStreamSynchronize(stream);
-      cudaMemPoolTrimTo(pool, 0);
+      trim_pools(device);
       e = cudaMalloc(&p, bytes);
     }
     if (e != cudaSuccess) {
@@ -81,11 +108,9 @@ void* SvPool::alloc(size_t bytes) {
   }
   cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, pool, stream);
   if (e == cudaErrorMemoryAllocation) {
-    // let the stream's frees take effect and give back what the pool keeps, then
-    // try once more
+    // give back what is kept, then try once more
     cudaGetLastError();
-    cudaStreamSynchronize(stream);
-    cudaMemPoolTrimTo(pool, 0);
+    trim_pools(device);
     e = cudaMallocFromPoolAsync(&p, bytes, pool, stream);
   }
   if (e != cudaSuccess) {
@@ -137,6 +162,15 @@ void SvPool::give_back(void* p, size_t bytes) {
 }
 
 void SvPool::close() {
+  {
+    std::lock_guard<std::mutex> lk(pools_mu());
+    auto& all = pools();
+    for (size_t i = 0; i < all.size(); ++i)
+      if (all[i].get() == this) {
+        all.erase(all.begin() + i);
+        break;
+      }
+  }
   std::lock_guard<std::mutex> lk(mu);
   alive = false;
   uint64_t none = 0;
@@ -422,6 +456,10 @@ SV_API int sv_context_create(int device, sv_context** out) {
     delete ctx;
     sv_throw(SV_ERR_CUDA, "memory pool: %s", cudaGetErrorString(e));
   }
+  {
+    std::lock_guard<std::mutex> lk(pools_mu());
+    pools().push_back(ctx->pool);
+  }
   for (int i = 0; i < 16; ++i) SV_CUDA(cudaEventCreate(&ctx->marks[i]));
   SV_CUDA(cudaMalloc((void**)&ctx->d_status, 256));
   SV_CUDA(cudaMemsetAsync(ctx->d_status, 0, 256, ctx->stream));
@@ -493,6 +531,13 @@ SV_API int sv_synchronize(sv_context* ctx) {
   SV_TRY
   sv_ctx_check(ctx);
   sv_sync(ctx);
+  SV_CATCH
+}
+
+SV_API int sv_context_trim(sv_context* ctx) {
+  SV_TRY
+  sv_ctx_check(ctx);
+  ctx->pool->trim();
   SV_CATCH
 }
 

@@ -76,7 +76,8 @@ struct SvTimedLaunch {
 // cudaFree took 3.7 of the 10.0 ms of normalise + scale at 100,000 x 33,538,
 // 5 of 15.7 ms of filter + vst at 30,000 cells.)  The pool keeps at most
 // SV_POOL_KEEP of the device's memory between calls, gives all of it back when
-// the context is destroyed or an allocation fails, and is shared by the
+// the context is destroyed, when an allocation of any context of the process fails
+// or when the program asks for it (sv_context_trim), and is shared by the
 // context and its live blocks: a block that outlives its context is freed with
 // cudaFree.  Blocks above a quarter of what it keeps go to cudaMalloc and cudaFree:
 // they would mostly be given back anyway, and the pool maps and unmaps them more
@@ -98,6 +99,7 @@ struct SvPool {
   void free(void* p, size_t bytes);
   void hold();          // frees wait until let_go: the stream is being captured
   void let_go();
+  void trim();          // gives back what it keeps (not while the stream is captured)
   void close();         // the context goes away
   ~SvPool();
 

@@ -66,3 +66,36 @@ def test_handles_freed_while_the_stream_is_captured(sv, genes, mu):
     d = sv.Context(0)
     assert free0 - d.memory()[0] <= 256 << 20
     d.close()
+
+
+def _fill(nbytes):
+    import torch
+    return torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+
+
+def test_kept_memory_is_there_for_others(sv):
+    """What a context keeps between calls goes back to the device when it is trimmed, and
+    when another context has no memory left."""
+    import torch
+    torch.cuda.empty_cache()
+    a, b = sv.Context(0), sv.Context(0)
+    n, genes = 400000, 2000
+
+    def make(c):
+        return sv.CountMatrix.generate(n, genes, np.full(genes, 3.0), np.ones(n), seed=1, ctx=c)
+
+    free0 = a.memory()[0]
+    nbytes = 16 * make(a).nnz                       # 10 GB in blocks of the pool, dropped at once
+    kept = free0 - a.memory()[0]
+    assert kept > nbytes // 2
+    a.trim()
+    assert free0 - a.memory()[0] < 256 << 20
+    make(a)
+    fill = _fill(a.memory()[0] - nbytes // 2)       # half of it besides what a keeps
+    try:
+        assert make(b).nnz * 16 == nbytes
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+        a.close()
+        b.close()
