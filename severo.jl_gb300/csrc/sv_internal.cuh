@@ -270,6 +270,16 @@ struct DevBuf {
     pool = sv_pool;
     n = count;
   }
+  // for what only makes a call faster: false when there is no memory for it
+  bool try_alloc(size_t count) {
+    try {
+      alloc(count);
+    } catch (const SvError& e) {
+      if (e.code != SV_ERR_OOM) throw;
+      return false;
+    }
+    return true;
+  }
   static size_t bytes(size_t count) { return (count * sizeof(T) + 64 + 255) & ~size_t(255); }
   void release() {
     if (p) pool->free(p, bytes(n));
@@ -424,6 +434,18 @@ struct sv_graph {
   DevBuf<int32_t> rowidx;          // nnz, 0-based
   DevBuf<unsigned char> val;       // nnz * elem
 };
+
+// Runs f(true), whose extra memory only makes it faster, and where the device has
+// not that much f(false).
+template <typename Fn>
+inline void sv_if_memory(Fn f) {
+  try {
+    f(true);
+  } catch (const SvError& e) {
+    if (e.code != SV_ERR_OOM) throw;
+    f(false);
+  }
+}
 
 inline size_t sv_elem_size(int dtype) {
   switch (dtype) {

@@ -21,7 +21,7 @@
 
 int sv_knn_tc_candidates(sv_context* ctx, const float* X32, const float* sq, int64_t n, int dp, int d,
                          int K2, int include_self, int32_t* cand,
-                         const std::vector<int64_t>* segs);
+                         const std::vector<int64_t>* segs, bool lists);
 sv_context* sv_default_context();
 
 namespace {
@@ -432,10 +432,11 @@ __global__ void k_rerank(const float* __restrict__ X, int64_t n, const int32_t* 
 }
 
 template <int DP>
-void launch_fp32(sv_context* ctx, const float* X, const float* sq, int64_t n, int d, int keep, int K2, int32_t* cand) {
+void launch_fp32(sv_context* ctx, const float* X, const float* sq, int64_t n, int d, int keep, int K2, int32_t* cand,
+                 bool lists) {
   const int64_t ntiles = (n + KNN_TILE - 1) / KNN_TILE, npad = ntiles * KNN_TILE;
   KnnOrder ord;
-  const bool listed = n >= KNN_ORDER_MIN && sv_knn_order(ctx, X, n, DP, d, KNN_TILE, KNN_TILE,
+  const bool listed = lists && n >= KNN_ORDER_MIN && sv_knn_order(ctx, X, n, DP, d, KNN_TILE, KNN_TILE,
                                                          sv_knn_spread(ctx, X, n, DP, d), ord);
   DevBuf<float> Xt((size_t)npad * DP), sqt(npad);
   DevBuf<int> orig(npad);
@@ -497,13 +498,12 @@ static void knn_core(sv_context* ctx, const float* X32, const float* sq, int64_t
   int K2 = precision == SV_KNN_BF16 ? (2 * k <= 40 ? 40 : 64) : (2 * k <= 32 ? 32 : 64);
   if (2 * k > 64) sv_throw(SV_ERR_UNSUPPORTED, "k = %d exceeds the supported maximum of 32", k);
   DevBuf<int32_t> cand((size_t)n * K2);
-  bool done = false;
-  if (precision == SV_KNN_BF16) {
-    int st = sv_knn_tc_candidates(ctx, X32, sq, n, dp, d, K2, include_self, cand.get(), segs);
-    if (st != SV_OK) sv_throw(st, "tensor-core kNN failed");
-    done = true;
-  }
-  if (!done) {
+  sv_if_memory([&](bool lists) {
+    if (precision == SV_KNN_BF16) {
+      int st = sv_knn_tc_candidates(ctx, X32, sq, n, dp, d, K2, include_self, cand.get(), segs, lists);
+      if (st != SV_OK) sv_throw(st, "tensor-core kNN failed");
+      return;
+    }
     // FP32 tiles: one launch per sample (each on its own rows)
     const int keep = include_self ? K2 - 1 : K2;   // besides the point itself
     std::vector<int64_t> one = {0, n};
@@ -515,21 +515,21 @@ static void knn_core(sv_context* ctx, const float* X32, const float* sq, int64_t
       const float* qs = sq + o;
       int32_t* cs = cand.get() + o * K2;
       switch (dp) {
-        case 8: launch_fp32<8>(ctx, Xs, qs, ns, d, keep, K2, cs); break;
-        case 16: launch_fp32<16>(ctx, Xs, qs, ns, d, keep, K2, cs); break;
-        case 24: launch_fp32<24>(ctx, Xs, qs, ns, d, keep, K2, cs); break;
-        case 32: launch_fp32<32>(ctx, Xs, qs, ns, d, keep, K2, cs); break;
-        case 40: launch_fp32<40>(ctx, Xs, qs, ns, d, keep, K2, cs); break;
-        case 48: launch_fp32<48>(ctx, Xs, qs, ns, d, keep, K2, cs); break;
-        case 56: launch_fp32<56>(ctx, Xs, qs, ns, d, keep, K2, cs); break;
-        case 64: launch_fp32<64>(ctx, Xs, qs, ns, d, keep, K2, cs); break;
+        case 8: launch_fp32<8>(ctx, Xs, qs, ns, d, keep, K2, cs, lists); break;
+        case 16: launch_fp32<16>(ctx, Xs, qs, ns, d, keep, K2, cs, lists); break;
+        case 24: launch_fp32<24>(ctx, Xs, qs, ns, d, keep, K2, cs, lists); break;
+        case 32: launch_fp32<32>(ctx, Xs, qs, ns, d, keep, K2, cs, lists); break;
+        case 40: launch_fp32<40>(ctx, Xs, qs, ns, d, keep, K2, cs, lists); break;
+        case 48: launch_fp32<48>(ctx, Xs, qs, ns, d, keep, K2, cs, lists); break;
+        case 56: launch_fp32<56>(ctx, Xs, qs, ns, d, keep, K2, cs, lists); break;
+        case 64: launch_fp32<64>(ctx, Xs, qs, ns, d, keep, K2, cs, lists); break;
         default: sv_throw(SV_ERR_UNSUPPORTED, "padded dimension %d", dp);
       }
       if (o > 0)
         sv_launch(ctx, "knn_offset", k_add_offset, dim3(sv_grid_for(ctx, ns * K2, 256, 4)), dim3(256), 0,
                   cs, ns * K2, (int32_t)o);
     }
-  }
+  });
   out->n = n;
   out->k = k;
   out->idx.alloc((size_t)n * k);

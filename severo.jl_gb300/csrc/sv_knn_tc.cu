@@ -630,7 +630,7 @@ __global__ void k_cand_unperm(const int32_t* __restrict__ cs, const int* __restr
 }  // namespace
 
 int sv_knn_tc_candidates(sv_context* ctx, const float* X32, const float* sq_unused, int64_t n, int dp,
-                         int d, int K2, int include_self, int32_t* cand, const std::vector<int64_t>* segs) {
+                         int d, int K2, int include_self, int32_t* cand, const std::vector<int64_t>* segs, bool lists) {
   (void)sq_unused;
   (void)include_self;   // the re-rank places or removes the point itself
   try {
@@ -670,7 +670,7 @@ int sv_knn_tc_candidates(sv_context* ctx, const float* X32, const float* sq_unus
     // pivots, and tile lists; stacked samples (a CTA sees its own sample's tiles
     // only): as they are
     KnnOrder ord;
-    const bool listed = prune && !segs && n >= LIST_MIN &&
+    const bool listed = lists && prune && !segs && n >= LIST_MIN &&
                         sv_knn_order(ctx, X32, n, dp, d, BM, BN, spread, ord, perm.get());
     if (listed) perm = std::move(ord.perm);
     const int* pm = around ? (const int*)perm.get() : (const int*)nullptr;

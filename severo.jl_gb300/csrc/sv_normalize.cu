@@ -215,9 +215,8 @@ void run_normalize(sv_context* ctx, const sv_counts* c, sv_data* d, NormArgs p) 
   // The table has NORM_TABLE values a cell, written a sector each: with a few
   // entries a cell that costs more than the entries do (from twice as many
   // entries as table values on, the table is at most a fifth of the writes).
-  const bool tabled = nnz >= 2 * NORM_TABLE * c->n_cells;
   DevBuf<OutT> table;
-  if (tabled) table.alloc(NORM_TABLE * c->n_cells);
+  const bool tabled = nnz >= 2 * NORM_TABLE * c->n_cells && table.try_alloc(NORM_TABLE * c->n_cells);
   sv_launch(ctx, "normalize_csr", k_norm_csr<OutT>, dim3(sv_grid_for(ctx, c->n_cells * 32, 256, 8)),
             dim3(256), 0, (const int64_t*)c->csr_rowptr.get(), (const int32_t*)c->csr_count.get(),
             c->n_cells, p, (OutT*)d->csr_val.get(), d->totals.get(), tabled ? table.get() : (OutT*)nullptr);

@@ -18,7 +18,7 @@
 // only those by row and leave them as packed words in an arena; once the kept
 // counts are scanned, a second kernel writes rows and weights from there.  The
 // hub form (and rows or k too large for the packing, or an arena above 1/16 of
-// the device's memory) sorts all candidates, reads the counts as run lengths and
+// the device's memory or of more than it has left) sorts all candidates, reads the counts as run lengths and
 // runs twice: count the kept entries, scan, write.  All integer work; a weight
 // is one IEEE-correctly rounded division, made once per possible count.
 #include "sv_internal.cuh"
@@ -526,7 +526,7 @@ __global__ void __launch_bounds__(1024) k_snn_block(
 
 template <typename T>
 void snn_run(sv_context* ctx, const int32_t* nn, int64_t n, int k, int64_t kparam, double prune_d,
-             sv_graph* out) {
+             sv_graph* out, bool arena_fits) {
   T prune = (T)prune_d;   // convert(T, prune)
   DevBuf<int32_t> G((size_t)n * k), gcnt(n);
   DevBuf<unsigned long long> rc(n + 1);
@@ -573,7 +573,7 @@ void snn_run(sv_context* ctx, const int32_t* nn, int64_t n, int k, int64_t kpara
     while (cmin < k && !((T)cmin / ((T)(int)kparam + ((T)(int)kparam - (T)cmin)) > prune)) ++cmin;
   size_t arena_words = (size_t)(cands / cmin) + 1;
   if (arena_words * 4 > ctx->pool->keep) cb = 0;
-  const bool hash = cb > 0;
+  const bool hash = cb > 0 && arena_fits;
   DevBuf<uint32_t> arena(hash ? arena_words : 1);
   DevBuf<int64_t> at(hash ? n : 1);
   DevBuf<unsigned long long> used(1);
@@ -670,8 +670,10 @@ void snn_dispatch(sv_context* ctx, const int32_t* nn, int64_t n, int k, int64_t 
   g->ctx = ctx;
   g->n = n;
   g->dtype = dtype;
-  if (dtype == SV_F64) snn_run<double>(ctx, nn, n, k, kparam, prune, g);
-  else snn_run<float>(ctx, nn, n, k, kparam, prune, g);
+  sv_if_memory([&](bool arena) {
+    if (dtype == SV_F64) snn_run<double>(ctx, nn, n, k, kparam, prune, g, arena);
+    else snn_run<float>(ctx, nn, n, k, kparam, prune, g, arena);
+  });
 }
 
 
