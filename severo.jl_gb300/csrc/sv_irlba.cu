@@ -2247,7 +2247,8 @@ struct Lanczos {
   DevBuf<double> upart;         // and its partial sums
   SvRunStage stage;
   double* hsum = nullptr;       // pinned copy of the cycle summaries
-  int* hflags = nullptr;        // pinned staging of the active / finish masks
+  int* hflags = nullptr;        // pinned staging of the active mask, and of the finish
+  int* hsel = nullptr;          // mask: the copy of one may not be over when the other is set
   double eps_b = 0;
   int cgs_blocks = RED_BLOCKS;  // resident blocks of the CGS kernels (one wave)
   bool vside_multi = false;     // feature side through the multi-block kernels
@@ -2339,8 +2340,9 @@ struct Lanczos {
     Vfin.alloc(n * nu);
     sv_memset(ctx, counter.get(), 0, (4 + nseg) * 4);
     sv_memset(ctx, B.get(), 0, (size_t)nseg * work * work * 8);
-    hsum = (double*)stage.alloc(ctx, (size_t)nseg * (2 * work + 2) * 8 + (size_t)nseg * 4);
+    hsum = (double*)stage.alloc(ctx, (size_t)nseg * (2 * work + 2) * 8 + (size_t)nseg * 8);
     hflags = (int*)(hsum + (size_t)nseg * (2 * work + 2));
+    hsel = hflags + nseg;
     op->bind_active(active.get());
     for (auto kern : {k_jacobi_svd<1>, k_jacobi_svd<2>, k_jacobi_svd<3>})
       SV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2779,9 +2781,9 @@ struct Lanczos {
     return g.matvecs;
   }
 
-  // U_s = W_s P_s[:, :nu], V_s = V_s Q_s[:, :nu] (FP64) for the samples in hflags
+  // U_s = W_s P_s[:, :nu], V_s = V_s Q_s[:, :nu] (FP64) for the samples in hsel
   void finish_selected() {
-    sv_h2d(ctx, finsel.get(), hflags, (size_t)nseg * 4);
+    sv_h2d(ctx, finsel.get(), hsel, (size_t)nseg * 4);
     rotate(Ws, P.get(), nu, Ufin.get(), finsel.get());
     rotate(Vs, Q.get(), nu, Vfin.get(), finsel.get());
   }
@@ -2819,7 +2821,7 @@ struct Lanczos {
       sv_sync(ctx);
       bool any = false;
       for (int s = 0; s < nseg; ++s) {
-        hflags[s] = 0;
+        hsel[s] = 0;
         if (!act[s]) continue;
         const double* hs = hsum + (size_t)s * (2 * work + 2);
         double rf = hs[2 * work];
@@ -2831,7 +2833,7 @@ struct Lanczos {
           res.info[s] = 0;
           res.iters[s] = it + 1;
           act[s] = 0;
-          hflags[s] = 1;
+          hsel[s] = 1;
           --nact;
           any = true;
         }
@@ -2845,7 +2847,7 @@ struct Lanczos {
       }
     }
     if (nact > 0) {
-      for (int s = 0; s < nseg; ++s) hflags[s] = act[s];
+      for (int s = 0; s < nseg; ++s) hsel[s] = act[s];
       finish_selected();
       sv_sync(ctx);
     }
