@@ -508,12 +508,12 @@ void sv_rotate_tc(sv_context* ctx, const float* inh, const float* inl, int64_t l
 // staged through the context's pinned buffers with several host threads.
 void sv_h2d(sv_context* ctx, void* dst, const void* src, size_t bytes);
 void sv_d2h(sv_context* ctx, void* dst, const void* src, size_t bytes);
-// the context's two pinned staging buffers (SV_IO_CHUNK bytes each) and the
-// events of their last transfers (wait on them before refilling)
 // blocks and threads of the pass that sums u for X^T u (its partial sums are
 // grid-stride sums of this shape)
 constexpr int SV_UPREP_BLOCKS = 304;
 constexpr int SV_UPREP_THREADS = 256;
+// the context's two pinned staging buffers (SV_IO_CHUNK bytes each) and the
+// events of their last transfers (wait on them before refilling)
 constexpr size_t SV_IO_CHUNK = (size_t)64 << 20;
 void sv_ctx_io(sv_context* ctx, void* buf[2], cudaEvent_t ev[2]);
 // memcpy split over up to 8 host threads

@@ -141,7 +141,7 @@ __device__ __forceinline__ void w64_step(unsigned long long (&v)[M][2], int stri
 // a scan's first tiles, where most keys pass, the warps wait for it: a warp merges
 // two queries at a time (500 points in 50 dimensions, 64 candidates: 0.36 -> 0.12
 // ms; 30,000 without a list: 8.6 -> 5.1 ms; four at a time are 3% slower).
-// 30,000 points in 60 clusters x 50 dimensions, 64 candidates, with lists: 0.9 ms
+// 30,000 points in 60 clusters x 50 dimensions, 64 candidates, with lists: 0.8 ms
 // for the tiles; a query per thread with 64 candidates in registers over every
 // tile, 235 blocks of four warps, took 7.5 ms.
 template <int DP>

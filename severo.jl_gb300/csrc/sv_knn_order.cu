@@ -466,8 +466,11 @@ bool sv_knn_order(sv_context* ctx, const float* X32, int64_t n, int dp, int d, i
                   const KnnSpread& spread, KnnOrder& o, const int* halves_of) {
   const bool bf16 = halves_of != nullptr;
   const int64_t nq = (n + bq - 1) / bq, np = (n + bp - 1) / bp;
-  // worth it from a few tiles up; the lists have to fit (sorted in shared memory,
-  // kept in 1/4 of what the pool keeps: 4 GB, 4 M points)
+  // worth it from a few tiles up; a list has to fit the shared memory that it is
+  // sorted in (16,384 tiles: 1,048,576 points of the FP32 search's 64, 4 M of the
+  // tensor-core search's 256), and all of them 1/64 of the device's memory (4.4 GB of
+  // 284: 4.3 M points of the tensor-core search); beyond that the order stays the
+  // caller's
   if (np < 4 || np > KNN_MAX_TILES || (size_t)(nq * np) * 8 > ctx->pool->keep / 4) return false;
   const int64_t npad = (np + 63) / 64 * 64;
   // a cell of about two tiles of 64 points while that takes few pivots (a cluster

@@ -419,8 +419,8 @@ __global__ void k_hsub_write(const int64_t* __restrict__ rowptr, const int32_t* 
 // Entries of class c fill the c-slots in order of appearance; the surplus of
 // over-full classes fills the slots left empty, in slot order.  The segment's
 // sum is then taken in another order (a different, equally valid rounding).
-// Applied to the CSR_h rows (X v: 1.61 -> 1.52 ms per product at the atlas
-// size, for ~16 ms once per scale_features); for the row-blocked runs (NC = 32)
+// Applied to the CSR_h rows (X v: 1.61 -> 1.52 ms per product when it was added, at
+// the atlas size; once per scale_features, 2.4 ms for 525 M entries); for the row-blocked runs (NC = 32)
 // the product gained 1% and the reordering cost more than it saved.
 constexpr int BO_EMPTY = 1024;   // most empty slots a segment may have to be reordered
 constexpr int BO_WARPS = 4;

@@ -1,5 +1,5 @@
-"""GPU: the FP32 neighbour search over tile lists against FP64 brute force, where
-the lists begin (2,048 points), at ragged last tiles and blocks, for
+"""GPU: the FP32 neighbour search, without and over tile lists, against FP64 brute
+force, where the lists begin (8,192 points), at ragged last tiles and blocks, for
 clustered, unclustered, sorted, repeated and non-finite points, every padded
 dimension's edges, and both metrics."""
 import numpy as np
